@@ -368,6 +368,12 @@ static gbfs_params effective_params(gbfs_graph *g)
         if (csr_build_transpose(g->csr, g->stream, err) != GBFS_OK) cudaGetLastError();
     }
     if (!g->symmetric && !g->csr.trow) p.direction = GBFS_DIR_TOPDOWN;
+    // the label-correcting kernel's adjacency (it walks the rows themselves
+    // where that does not fit in memory)
+    if (!g->csr.quad && bfs_wants_quads(g->csr, p)) {
+        std::string err;
+        if (csr_build_quads(g->csr, g->stream, err) != GBFS_OK) cudaGetLastError();
+    }
     return p;
 }
 

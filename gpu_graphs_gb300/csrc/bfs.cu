@@ -1232,6 +1232,8 @@ BfsArgs make_args(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const in
     a.qb64[0] = reinterpret_cast<longlong2 *>(w.qb0);  // the workspace of a wide graph has 16-byte bounds
     a.qb64[1] = reinterpret_cast<longlong2 *>(w.qb1);
     a.bigl = w.big;
+    a.quad = g.quad;
+    a.over = g.over;
     a.ctrl = w.ctrl;
     a.out = slot;
     a.roots = d_roots;
@@ -1338,6 +1340,16 @@ cudaError_t add_bfs_node(cudaGraph_t g, const cudaGraphNode_t *dep, size_t ndep,
 bool bfs_relax_tail(const DeviceCsr &g, const gbfs_params &p)
 {
     return !p.per_level_launch && p.direction != GBFS_DIR_BOTTOMUP && g.max_degree <= RELAX_MAX_DEGREE;
+}
+
+bool bfs_wants_quads(const DeviceCsr &g, const gbfs_params &p)
+{
+    // Up to one row in 16 longer than four (grids, road networks).  A linked
+    // row costs its hop another round trip.  2000 x 2000 grid with a growing
+    // share of such rows, quads against the CSR kernel: 0.1 % 3.95 and 7.99 ms,
+    // 4 % 4.62 and 5.60, 7.6 % 5.43 and 5.34, 12 % 6.27 and 5.12, all (a
+    // triangular mesh) 16.0 and 4.65.
+    return bfs_relax_tail(g, p) && g.max_degree <= QUAD_MAX_DEGREE && (int64_t)g.nover4 * 16 <= g.n;
 }
 
 int bfs_launches_per_search(const DeviceCsr &g, const gbfs_params &p) { return bfs_relax_tail(g, p) ? 2 : 1; }

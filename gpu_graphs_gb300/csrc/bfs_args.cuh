@@ -28,6 +28,8 @@ struct BfsArgs {
     int2 *qb[2];             // row bounds beside q0 and q1
     longlong2 *qb64[2];      // the same for wide graphs
     int *bigl;
+    const int4 *quad;        // fixed-width adjacency (DeviceCsr::quad / over), or null
+    const int *over;
     BfsCtrl *ctrl;
     BfsOut *out;
     const int *roots;

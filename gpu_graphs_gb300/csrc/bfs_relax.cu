@@ -64,6 +64,91 @@ constexpr int RX_ILP_BIG = 4;
 constexpr int RX_HOPS = 64;
 constexpr int RX_BPS = 2;  // CTAs per SM (one: 7000^2 grid 19.6 ms, thin-start expander +30 %)
 
+// round stamps start at 0: round j marks the vertices it queues with j + 1
+__device__ __forceinline__ void rx_clear_stamps(int *stamp, int n, long long gtid, long long gthreads)
+{
+    if (((uintptr_t)stamp & 15) == 0) {
+        int4 *s4 = reinterpret_cast<int4 *>(stamp);
+        const long long n4 = n >> 2;
+        for (long long i = gtid; i < n4; i += gthreads) s4[i] = make_int4(0, 0, 0, 0);
+        for (long long i = (n4 << 2) + gtid; i < n; i += gthreads) stamp[i] = 0;
+    } else {
+        for (long long i = gtid; i < n; i += gthreads) stamp[i] = 0;
+    }
+}
+
+// Ends a search: the largest level, and the totals of first relaxations.
+// tl: trace rows written.  All threads call it.
+template <int BLOCK>
+__device__ __forceinline__ void rx_close(const BfsArgs &a, const BfsResume &rs, unsigned long long cd0,
+                                         unsigned long long my_reached, unsigned long long my_edges, int tl,
+                                         unsigned &epoch, int *s_max, unsigned long long (*s_red)[BLOCK / 32])
+{
+    BfsCtrl *ctrl = a.ctrl;
+    const int n = a.n;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long gtid = (long long)blockIdx.x * BLOCK + threadIdx.x;
+    const long long gthreads = (long long)gridDim.x * BLOCK;
+    int mx = -1;
+    if (((uintptr_t)a.level & 15) == 0) {
+        const int4 *l4 = reinterpret_cast<const int4 *>(a.level);
+        const long long n4 = n >> 2;
+        for (long long i = gtid; i < n4; i += gthreads) {
+            const int4 x = __ldcg(l4 + i);
+            mx = max(mx, max(max(x.x, x.y), max(x.z, x.w)));
+        }
+        for (long long i = (n4 << 2) + gtid; i < n; i += gthreads) mx = max(mx, __ldcg(a.level + i));
+    } else {
+        for (long long i = gtid; i < n; i += gthreads) mx = max(mx, __ldcg(a.level + i));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, o));
+    const unsigned long long rsum = warp_sum(my_reached), esum = warp_sum(my_edges);
+    if (lane == 0) {
+        s_max[warp] = mx;
+        s_red[0][warp] = rsum;
+        s_red[1][warp] = esum;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int m2 = lane < BLOCK / 32 ? s_max[lane] : -1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m2 = max(m2, __shfl_xor_sync(FULL, m2, o));
+        const unsigned long long r2 = warp_sum(lane < BLOCK / 32 ? s_red[0][lane] : 0ull);
+        const unsigned long long e2 = warp_sum(lane < BLOCK / 32 ? s_red[1][lane] : 0ull);
+        if (lane == 0) {
+            atomicMax(&ctrl->rx_max, m2);
+            atomicAdd(&ctrl->rx_reached, r2);
+            atomicAdd(&ctrl->rx_edges, e2);
+        }
+    }
+    if (!grid_sync(&ctrl->bar, &ctrl->status, a.timeout_ns, epoch)) return;
+    if (gtid == 0) {
+        const int levels = ctrl->rx_max + 1;
+        BfsOut o;
+        o.levels = levels;
+        o.td_levels = levels - rs.bu_levels;
+        o.bu_levels = rs.bu_levels;
+        o.roots = (int)rs.roots;
+        o.reached = rs.reached + cd_count(cd0) + ctrl->rx_reached;
+        o.edges_c = rs.edges_c + cd_degree(cd0) + ctrl->rx_edges;
+        *a.out = o;
+        ctrl->t_end = globaltimer_ns();
+        ctrl->trace_len = tl < TRACE_CAP ? tl : TRACE_CAP;
+        ctrl->rx_max = 0;
+        ctrl->rx_reached = 0;
+        ctrl->rx_edges = 0;
+        for (int i = 0; i < 3; i++) {
+            ctrl->cd[i] = 0;
+            ctrl->big[i] = 0;
+        }
+        ctrl->fill = 0;
+        ctrl->rs.done = 1;
+        ctrl->rs.mode = RESUME_LEVEL;
+    }
+    grid_exit(&ctrl->bar, &ctrl->t_exit);
+}
+
 template <typename RT>
 __global__ void __launch_bounds__(RX_BLOCK, 2) k_bfs_relax(BfsArgs a)
 {
@@ -90,15 +175,7 @@ __global__ void __launch_bounds__(RX_BLOCK, 2) k_bfs_relax(BfsArgs a)
     unsigned *const lvl = reinterpret_cast<unsigned *>(a.level);  // -1 (unreached) is the largest unsigned
     int *const stamp = a.bigl;  // round stamps (rows are never deferred on graphs of small degree)
 
-    // round stamps start at 0: round j marks the vertices it queues with j + 1
-    if (((uintptr_t)stamp & 15) == 0) {
-        int4 *s4 = reinterpret_cast<int4 *>(stamp);
-        const long long n4 = n >> 2;
-        for (long long i = gtid; i < n4; i += gthreads) s4[i] = make_int4(0, 0, 0, 0);
-        for (long long i = (n4 << 2) + gtid; i < n; i += gthreads) stamp[i] = 0;
-    } else {
-        for (long long i = gtid; i < n; i += gthreads) stamp[i] = 0;
-    }
+    rx_clear_stamps(stamp, n, gtid, gthreads);
     if (!grid_sync(&ctrl->bar, &ctrl->status, a.timeout_ns, epoch)) return;
 
     const int L0 = rs.L;
@@ -337,66 +414,249 @@ __global__ void __launch_bounds__(RX_BLOCK, 2) k_bfs_relax(BfsArgs a)
         }
     }
 
-    // complete: the largest level, and the totals of first relaxations
-    int mx = -1;
-    if (((uintptr_t)a.level & 15) == 0) {
-        const int4 *l4 = reinterpret_cast<const int4 *>(a.level);
-        const long long n4 = n >> 2;
-        for (long long i = gtid; i < n4; i += gthreads) {
-            const int4 x = __ldcg(l4 + i);
-            mx = max(mx, max(max(x.x, x.y), max(x.z, x.w)));
-        }
-        for (long long i = (n4 << 2) + gtid; i < n; i += gthreads) mx = max(mx, __ldcg(a.level + i));
-    } else {
-        for (long long i = gtid; i < n; i += gthreads) mx = max(mx, __ldcg(a.level + i));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, o));
-    const unsigned long long rsum = warp_sum(my_reached), esum = warp_sum(my_edges);
-    if (lane == 0) {
-        s_max[warp] = mx;
-        s_red[0][warp] = rsum;
-        s_red[1][warp] = esum;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        int m2 = lane < RX_NW ? s_max[lane] : -1;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m2 = max(m2, __shfl_xor_sync(FULL, m2, o));
-        const unsigned long long r2 = warp_sum(lane < RX_NW ? s_red[0][lane] : 0ull);
-        const unsigned long long e2 = warp_sum(lane < RX_NW ? s_red[1][lane] : 0ull);
-        if (lane == 0) {
-            atomicMax(&ctrl->rx_max, m2);
-            atomicAdd(&ctrl->rx_reached, r2);
-            atomicAdd(&ctrl->rx_edges, e2);
-        }
-    }
+    rx_close<RX_BLOCK>(a, rs, cd0, my_reached, my_edges, L0 + rounds, epoch, s_max, s_red);
+}
+
+// The same search on a graph whose rows are nearly all of four entries or
+// fewer, over its fixed-width adjacency (BfsArgs::quad).  A local frontier
+// entry carries its vertex's four neighbours and level, so slot t of the
+// frontier is thread t's edge (no degree scan, no search for the edge's row)
+// and a hop is ONE dependent memory round trip: the atomicMin on the
+// neighbour's level and the load of the neighbour's own quad are issued
+// together, where the CSR kernel above needs two (column entry and level[u],
+// then atomicMin and row bounds).  The few linked rows are walked by their
+// warp after the hop's other edges, one lane per further entry.
+//
+// An entry relaxes with the level it was queued with.  If that has fallen
+// since, whoever lowered it has queued the vertex again, so the rounds still
+// end only when every level is exact.
+// 256 threads: a CTA's piece is a few dozen entries, and a larger CTA's idle
+// warps slow its barrier (7000 x 7000 grid: 14.1 ms with 512 threads, 13.9 with
+// 256; 1000 x 1000: 1.51 and 1.35; 128 threads are too few on the large grid)
+constexpr int RXQ_BLOCK = 256;
+constexpr size_t RXQ_SMEM = 2 * RX_CAP * (sizeof(int4) + sizeof(unsigned) + sizeof(int));
+
+__global__ void __launch_bounds__(RXQ_BLOCK, 2) k_bfs_relax_quads(BfsArgs a)
+{
+    extern __shared__ __align__(16) unsigned char rx_smem[];
+    __shared__ unsigned s_cnt[3];
+    __shared__ unsigned long long s_cd;
+    __shared__ unsigned long long s_red[2][RXQ_BLOCK / 32];
+    __shared__ int s_max[RXQ_BLOCK / 32];
+
+    BfsCtrl *ctrl = a.ctrl;
+    // run only when the grid kernel parked its loop for this kernel
+    const BfsResume rs = ctrl->rs;
+    if (rs.done || rs.mode != RESUME_RELAX || ctrl->status != DEV_OK) return;
+
+    const int n = a.n;
+    const unsigned t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    // two local frontiers of RX_CAP entries: neighbours, 2 x level + (first
+    // reached by this entry: it is counted as it is expanded), ids
+    int4 *const s_q = reinterpret_cast<int4 *>(rx_smem);
+    unsigned *const s_l = reinterpret_cast<unsigned *>(s_q + 2 * RX_CAP);
+    int *const s_v = reinterpret_cast<int *>(s_l + 2 * RX_CAP);
+    const long long gtid = (long long)blockIdx.x * RXQ_BLOCK + t;
+    const long long gthreads = (long long)gridDim.x * RXQ_BLOCK;
+    unsigned epoch = 0;
+    unsigned *const lvl = reinterpret_cast<unsigned *>(a.level);  // -1 (unreached) is the largest unsigned
+    int *const stamp = a.bigl;
+    const int4 *const quad = a.quad;
+    const int *const over = a.over;
+
+    rx_clear_stamps(stamp, n, gtid, gthreads);
     if (!grid_sync(&ctrl->bar, &ctrl->status, a.timeout_ns, epoch)) return;
-    if (gtid == 0) {
-        const int levels = ctrl->rx_max + 1;
-        BfsOut o;
-        o.levels = levels;
-        o.td_levels = levels - rs.bu_levels;
-        o.bu_levels = rs.bu_levels;
-        o.roots = (int)rs.roots;
-        o.reached = rs.reached + cd_count(cd0) + ctrl->rx_reached;
-        o.edges_c = rs.edges_c + cd_degree(cd0) + ctrl->rx_edges;
-        *a.out = o;
-        ctrl->t_end = globaltimer_ns();
-        const int tl = L0 + rounds;
-        ctrl->trace_len = tl < TRACE_CAP ? tl : TRACE_CAP;
-        ctrl->rx_max = 0;
-        ctrl->rx_reached = 0;
-        ctrl->rx_edges = 0;
-        for (int i = 0; i < 3; i++) {
-            ctrl->cd[i] = 0;
-            ctrl->big[i] = 0;
+
+    const int L0 = rs.L;
+    const unsigned long long cd0 = ld_relaxed_u64(&ctrl->cd[L0 % 3]);
+    unsigned long long my_reached = 0, my_edges = 0;
+    int rounds = 0;
+
+    for (int j = 0;; ++j) {
+        const int Lj = L0 + j;
+        if (t == 0) s_cd = ld_relaxed_u64(&ctrl->cd[Lj % 3]);
+        __syncthreads();
+        const unsigned long long F = cd_count(s_cd);
+        if (F == 0) {
+            rounds = j;
+            break;
         }
-        ctrl->fill = 0;
-        ctrl->rs.done = 1;
-        ctrl->rs.mode = RESUME_LEVEL;
+        // the count two rounds back (read by every CTA before the last barrier)
+        if (gtid == 0) ctrl->cd[(Lj + 2) % 3] = 0;
+        const int *qin = (Lj & 1) ? a.q1 : a.q0;
+        int *qout = (Lj & 1) ? a.q0 : a.q1;
+        unsigned long long *cnt_out = &ctrl->cd[(Lj + 1) % 3];
+        const int mark = j + 1;
+        unsigned reached = 0, edges = 0;  // first relaxations of this round
+
+        // global push of v by the lanes with `go`, at most once per vertex and
+        // round; an entry not yet counted (first) is counted here
+        auto push_global = [&](bool go, int v, bool first, int4 vq) {
+            if (go && first) {
+                ++reached;
+                edges += vq.w < -1 ? __ldg(over + 16 * (size_t)(-2 - vq.w) + 15)
+                                   : (vq.x >= 0) + (vq.y >= 0) + (vq.z >= 0) + (vq.w >= 0);
+            }
+            if (go) go = atomicMax(stamp + v, mark) < mark;
+            const unsigned m = __ballot_sync(FULL, go);
+            if (!m) return;
+            const int leader = __ffs(m) - 1;
+            unsigned long long base = 0;
+            if ((int)lane == leader) base = cd_count(atomicAdd(cnt_out, (unsigned long long)__popc(m)));
+            base = __shfl_sync(FULL, base, leader) + __popc(m & lanemask_lt());
+            if (go) qout[base] = v;
+        };
+
+        // offer level nd[q] to w[q] (w[q] < 0: none); improvements join local
+        // frontier `nb` (its counter cnt_nb), or the global queue if `last` or
+        // that frontier is full
+        auto relax = [&](auto ilp, const int *w, const unsigned *nd, bool last, int nb, unsigned *cnt_nb) {
+            constexpr int Q = decltype(ilp)::value;
+            unsigned old[Q];
+            int4 wq[Q];
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                old[q] = 0;
+                wq[q] = make_int4(-1, -1, -1, -1);
+                if (w[q] >= 0) {
+                    old[q] = atomicMin(lvl + w[q], nd[q]);
+                    wq[q] = __ldg(quad + w[q]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                const bool imp = nd[q] < old[q];
+                const unsigned m = __ballot_sync(FULL, imp);
+                if (!m) continue;
+                const unsigned first = old[q] == 0xffffffffu;
+                if (last) {
+                    push_global(imp, w[q], first, wq[q]);
+                    continue;
+                }
+                const int leader = __ffs(m) - 1;
+                unsigned pos = 0;
+                if ((int)lane == leader) pos = atomicAdd(cnt_nb, (unsigned)__popc(m));
+                pos = __shfl_sync(FULL, pos, leader);
+                // past RX_CAP: the hop overflowed
+                if (pos + __popc(m) > (unsigned)RX_CAP)
+                    push_global(imp && pos + __popc(m & lanemask_lt()) >= (unsigned)RX_CAP, w[q], first, wq[q]);
+                pos += __popc(m & lanemask_lt());
+                if (imp && pos < (unsigned)RX_CAP) {
+                    s_q[nb * RX_CAP + pos] = wq[q];
+                    s_l[nb * RX_CAP + pos] = 2 * nd[q] + first;
+                    s_v[nb * RX_CAP + pos] = w[q];
+                }
+            }
+        };
+
+        // expand local frontier `cur` (nc entries) one level, Q edges per
+        // thread in flight
+        auto expand = [&](auto ilp, int cur, int nc, bool last, unsigned *cnt_nb) {
+            constexpr int Q = decltype(ilp)::value;
+            const int *slots = reinterpret_cast<const int *>(s_q + cur * RX_CAP);
+            const int S = 4 * nc;
+            for (int b = 0; b < S; b += RXQ_BLOCK * Q) {
+                if (b + (int)(warp * 32) >= S) break;  // no edge left for this warp
+                int w[Q];
+                unsigned nd[Q], lf[Q];
+#pragma unroll
+                for (int q = 0; q < Q; q++) {
+                    const int s = b + q * RXQ_BLOCK + (int)t;
+                    w[q] = -1;
+                    lf[q] = 0;
+                    if (s < S) {
+                        w[q] = slots[s];
+                        lf[q] = s_l[cur * RX_CAP + (s >> 2)];
+                    }
+                    nd[q] = (lf[q] >> 1) + 1u;
+                }
+                bool linked = false;
+#pragma unroll
+                for (int q = 0; q < Q; q++) {
+                    linked |= w[q] < -1;
+                    edges += (lf[q] & 1u) & (unsigned)(w[q] >= 0);
+                    reached += (lf[q] & 1u) & (unsigned)((lane & 3u) == 0);
+                }
+                relax(ilp, w, nd, last, cur ^ 1, cnt_nb);
+                if (!__any_sync(FULL, linked)) continue;
+                // linked rows: the warp takes the node's entries, one per lane
+#pragma unroll
+                for (int q = 0; q < Q; q++) {
+                    unsigned links = __ballot_sync(FULL, w[q] < -1);
+                    while (links) {
+                        const int src = __ffs(links) - 1;
+                        links &= links - 1u;
+                        const int k = -2 - __shfl_sync(FULL, w[q], src);
+                        const unsigned llf = __shfl_sync(FULL, lf[q], src);
+                        const int lw = lane < 15 ? __ldg(over + 16 * (size_t)k + lane) : -1;
+                        const unsigned lnd = (llf >> 1) + 1u;
+                        edges += (llf & 1u) & (unsigned)(lw >= 0);
+                        relax(std::integral_constant<int, 1>{}, &lw, &lnd, last, cur ^ 1, cnt_nb);
+                    }
+                }
+            }
+        };
+
+        const unsigned long long lo = F * blockIdx.x / gridDim.x, hi = F * (blockIdx.x + 1) / gridDim.x;
+        const bool hops = hi - lo <= (unsigned long long)RX_CAP;
+        for (unsigned long long s0 = lo; s0 < hi; s0 += RX_CAP) {
+            const int ns = (int)min((unsigned long long)RX_CAP, hi - s0);
+            for (int i = (int)t; i < ns; i += RXQ_BLOCK) {
+                const int v = __ldcg(qin + s0 + i);
+                s_v[i] = v;
+                s_l[i] = 2 * __ldcg(lvl + v);
+                s_q[i] = __ldg(quad + v);
+            }
+            // hop h expands local frontier h & 1, counted by s_cnt[h % 3], into
+            // frontier (h + 1) & 1, counted by s_cnt[(h + 1) % 3]; s_cnt[(h + 2) % 3]
+            // (hop h - 1's, read before the barrier that ended it) is zeroed
+            // during hop h, so a hop needs one CTA barrier
+            if (t == 0) {
+                s_cnt[0] = (unsigned)ns;
+                s_cnt[1] = 0;
+                s_cnt[2] = 0;
+            }
+            __syncthreads();
+            int nc = ns;
+            for (int h = 0;; ++h) {
+                const bool last = !hops || h == RX_HOPS - 1;
+                if (t == 0 && h > 0) s_cnt[(h + 2) % 3] = 0;
+                unsigned *cnt_nb = &s_cnt[(h + 1) % 3];
+                if (4 * nc <= RXQ_BLOCK) expand(std::integral_constant<int, 1>{}, h & 1, nc, last, cnt_nb);
+                else expand(std::integral_constant<int, RX_ILP_BIG>{}, h & 1, nc, last, cnt_nb);
+                __syncthreads();
+                if (last) break;
+                const unsigned raw = *cnt_nb;
+                const unsigned nn = min(raw, (unsigned)RX_CAP);
+                if (raw > (unsigned)RX_CAP || nn == 0) {
+                    // the hop overflowed the local frontier (or found nothing):
+                    // what it holds joins the global queue
+                    for (unsigned k0 = 0; k0 < nn; k0 += RXQ_BLOCK) {
+                        const bool in = k0 + t < nn;
+                        const unsigned o = ((h + 1) & 1) * RX_CAP + (in ? k0 + t : 0u);
+                        push_global(in, s_v[o], s_l[o] & 1u, s_q[o]);
+                    }
+                    break;
+                }
+                nc = (int)nn;
+            }
+            __syncthreads();  // before the next piece overwrites the local frontiers
+        }
+        my_reached += reached;
+        my_edges += edges;
+        if (!grid_sync(&ctrl->bar, &ctrl->status, a.timeout_ns, epoch)) return;
+        if (gtid == 0) {
+            LevelTrace tr;
+            tr.level = Lj;
+            tr.dir = 4;
+            tr.frontier = F;
+            tr.edges = 0;
+            tr.t_ns = globaltimer_ns();
+            ctrl->trace[Lj < TRACE_CAP - 1 ? Lj : TRACE_CAP - 1] = tr;
+        }
     }
-    grid_exit(&ctrl->bar, &ctrl->t_exit);
+
+    rx_close<RXQ_BLOCK>(a, rs, cd0, my_reached, my_edges, L0 + rounds, epoch, s_max, s_red);
 }
 
 }  // namespace
@@ -408,6 +668,12 @@ cudaError_t bfs_relax_launch(const BfsArgs &args, cudaStream_t st, int max_ctas)
     cudaError_t e = setup.get(sms, occ, [](int dev, int &s_out, int &o_out) {
         cudaError_t r = cudaDeviceGetAttribute(&s_out, cudaDevAttrMultiProcessorCount, dev);
         if (r == cudaSuccess) r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o_out, k_bfs_relax<int>, RX_BLOCK, 0);
+        int oq = 0;
+        if (r == cudaSuccess)
+            r = cudaFuncSetAttribute(k_bfs_relax_quads, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RXQ_SMEM);
+        if (r == cudaSuccess)
+            r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&oq, k_bfs_relax_quads, RXQ_BLOCK, RXQ_SMEM);
+        o_out = std::min(o_out, oq);
         return r;
     });
     if (e != cudaSuccess) return e;
@@ -416,6 +682,9 @@ cudaError_t bfs_relax_launch(const BfsArgs &args, cudaStream_t st, int max_ctas)
     if (max_ctas > 0) grid = std::max(1, std::min(grid, max_ctas));
     BfsArgs a = args;
     void *kargs[] = {&a};
+    if (a.quad)
+        return cudaLaunchCooperativeKernel((const void *)k_bfs_relax_quads, dim3(grid), dim3(RXQ_BLOCK), kargs,
+                                           RXQ_SMEM, st);
     // the wide kernel holds twice the row-bound bytes in shared memory; its
     // CTAs still fit two per SM
     const void *fn = a.wide ? (const void *)k_bfs_relax<long long> : (const void *)k_bfs_relax<int>;

@@ -505,11 +505,12 @@ __global__ void k_compact_long(const RT *__restrict__ row, const RT *__restrict_
 
 template <typename RT>
 __global__ void k_finalize(const RT *__restrict__ row, int n, unsigned *zmask, int *maxdeg,
-                           unsigned long long *nonisolated)
+                           unsigned long long *nonisolated, unsigned *nover4)
 {
     __shared__ unsigned long long s_red[32];
     __shared__ int s_max[32];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    // non-isolated rows, and rows of more than four entries in the high half
     unsigned long long mine = 0;
     int mx = 0;
     const int W = (n + 31) >> 5;
@@ -519,11 +520,14 @@ __global__ void k_finalize(const RT *__restrict__ row, int n, unsigned *zmask, i
         int d = v < n ? (int)(row[v + 1] - row[v]) : 0;
         unsigned z = __ballot_sync(FULL, d == 0);  // out-of-range bits count as zero-degree
         if (lane_id() == 0) zmask[v >> 5] = z;
-        mine += d > 0;
+        mine += (d > 0 ? 1ull : 0ull) + (d > 4 ? 1ull << 32 : 0ull);
         mx = max(mx, d);
     }
     unsigned long long t = block_sum(mine, s_red);
-    if (threadIdx.x == 0 && t) atomicAdd(nonisolated, t);
+    if (threadIdx.x == 0 && t) {
+        atomicAdd(nonisolated, t & 0xffffffffull);
+        if (t >> 32) atomicAdd(nover4, (unsigned)(t >> 32));
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, o));
     __syncthreads();
@@ -756,19 +760,20 @@ template <typename RT>
 int finalize_t(DeviceCsr &out, const RT *row, cudaStream_t st, std::string &err)
 {
     int rc = GBFS_OK;
-    struct Res { unsigned long long nonisolated; int maxdeg; unsigned nheavy; } h{};
+    struct Res { unsigned long long nonisolated; int maxdeg; unsigned nheavy, nover4, pad; } h{};
     Res *d_res = nullptr;
     const int W = (out.n + 31) / 32;
     CK(cudaMalloc(&out.zmask, sizeof(unsigned) * (size_t)W));
     CK(cudaMalloc(&d_res, sizeof(Res)));
     CK(cudaMemsetAsync(d_res, 0, sizeof(Res), st));
     k_finalize<<<grid_for((int64_t)W * 32, 256), 256, 0, st>>>(row, out.n, out.zmask, &d_res->maxdeg,
-                                                                &d_res->nonisolated);
+                                                                &d_res->nonisolated, &d_res->nover4);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(&h, d_res, sizeof(Res), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     out.max_degree = h.maxdeg;
     out.nonisolated = (int64_t)h.nonisolated;
+    out.nover4 = (int32_t)h.nover4;
     {
         // heavy-row list (sized by a first count pass folded into k_heavy_list's atomic)
         CK(cudaMalloc(&out.heavy, sizeof(int) * (size_t)std::max<int64_t>(1, out.n)));
@@ -1052,6 +1057,64 @@ done:
     return rc;
 }
 
+namespace {
+
+template <typename RT>
+__global__ void k_quads(const RT *__restrict__ row, const int *__restrict__ col, int n, int4 *quad, int *over,
+                        unsigned *nover)
+{
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        const RT b = row[v];
+        const int d = (int)(row[v + 1] - b);
+        int4 q = make_int4(-1, -1, -1, -1);
+        if (d > 0) q.x = col[b];
+        if (d > 1) q.y = col[b + 1];
+        if (d > 2) q.z = col[b + 2];
+        if (d == 4) q.w = col[b + 3];
+        if (d > 4) {
+            const unsigned k = atomicAdd(nover, 1u);
+            q.w = -2 - (int)k;
+            int *o = over + 16 * (size_t)k;
+            for (int i = 0; i < 15; i++) o[i] = 3 + i < d ? col[b + 3 + i] : -1;
+            o[15] = d;
+        }
+        quad[v] = q;
+    }
+}
+
+}  // namespace
+
+int64_t csr_quad_bytes(const DeviceCsr &c)
+{
+    return (int64_t)sizeof(int4) * c.n + 16 * (int64_t)sizeof(int) * c.nover4;
+}
+
+int csr_build_quads(DeviceCsr &c, cudaStream_t st, std::string &err)
+{
+    if (c.quad) return GBFS_OK;
+    int rc = GBFS_OK;
+    int4 *quad = nullptr;
+    int *over = nullptr;
+    unsigned *cnt = nullptr;
+    CK(cudaMalloc(&quad, sizeof(int4) * (size_t)std::max(1, c.n)));
+    CK(cudaMalloc(&over, 16 * sizeof(int) * (size_t)std::max(1, c.nover4)));
+    CK(cudaMalloc(&cnt, sizeof(unsigned)));
+    CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned), st));
+    if (c.wide) k_quads<<<grid_for(c.n, 256), 256, 0, st>>>((const long long *)c.row64, c.col, c.n, quad, over, cnt);
+    else k_quads<<<grid_for(c.n, 256), 256, 0, st>>>((const int *)c.row, c.col, c.n, quad, over, cnt);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(st));
+    c.quad = quad;
+    c.over = over;
+    quad = nullptr;
+    over = nullptr;
+done:
+    if (quad) cudaFree(quad);
+    if (over) cudaFree(over);
+    if (cnt) cudaFree(cnt);
+    return rc;
+}
+
 int64_t csr_device_bytes(const DeviceCsr &c)
 {
     const int64_t n = c.n, m = c.m;
@@ -1062,6 +1125,7 @@ int64_t csr_device_bytes(const DeviceCsr &c)
     if (c.trow) b += 4 * (n + 1 + m) + 4 * n;                    // trow, tcol, theavy
     if (c.tfirst) b += 4 * n;
     if (c.tpieces) b += 8 * (int64_t)c.ntpieces;
+    if (c.quad) b += csr_quad_bytes(c);
     return b;
 }
 
@@ -1074,6 +1138,8 @@ void csr_free(DeviceCsr &c)
     if (c.first) cudaFree(c.first);
     if (c.second) cudaFree(c.second);
     if (c.tpieces) cudaFree(c.tpieces);
+    if (c.quad) cudaFree(c.quad);
+    if (c.over) cudaFree(c.over);
     if (c.heavy) cudaFree(c.heavy);
     if (c.pieces) cudaFree(c.pieces);
     if (c.row) cudaFree(c.row);

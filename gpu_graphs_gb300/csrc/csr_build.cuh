@@ -28,6 +28,14 @@ struct DeviceCsr {
     int *first = nullptr;      // n
     int *second = nullptr;     // n; not allocated for hub-first rows (probed at the first entry alone)
     bool hub_rows = false;     // rows are hub-first (csr_hub_first ran)
+    // fixed-width adjacency of a small-degree graph, built on demand by
+    // csr_build_quads for the label-correcting kernel: quad[v] holds row v's
+    // entries, -1 past its end; a row of more than four keeps its first three
+    // there and a link -2 - k in the fourth place to its node, over[16 k ..]:
+    // the entries from the fourth on (-1 past the end) and, last, its degree
+    int32_t nover4 = 0;        // rows of more than four entries
+    int4 *quad = nullptr;      // n
+    int *over = nullptr;       // 16 per row of more than four entries
     // multi-source pull pieces (built on demand by ms_prepare): every row of
     // degree > 2 * MS_PIECE contributes {vertex, j} for its j-th MS_PIECE edges
     int2 *pieces = nullptr;
@@ -77,6 +85,13 @@ int csr_build_transpose(DeviceCsr &c, cudaStream_t st, std::string &err);
 
 // (Re)compute c.first / c.second from the rows as they are now.  Synchronises st.
 int csr_build_first(DeviceCsr &c, cudaStream_t st, std::string &err);
+
+// Build c.quad / c.over; a no-op once built.  Only for graphs of out-degree at
+// most QUAD_MAX_DEGREE.  Synchronises st.
+constexpr int QUAD_MAX_DEGREE = 16;
+int csr_build_quads(DeviceCsr &c, cudaStream_t st, std::string &err);
+// Bytes csr_build_quads allocates.
+int64_t csr_quad_bytes(const DeviceCsr &c);
 
 // Device bytes held by the CSR and everything built on it.
 int64_t csr_device_bytes(const DeviceCsr &c);

@@ -517,9 +517,18 @@ extern "C" int gbfs_server_add_graph(gbfs_server *s, gbfs_graph *g, int32_t *gra
     const bool has_t = want_t || g->csr.trow != nullptr;
     const int64_t tbytes =  // trow, tcol, theavy, tfirst still to build
         want_t && !g->csr.trow ? (int64_t)sizeof(int) * (3 * (int64_t)g->csr.n + 1 + g->csr.m) : 0;
-    const int64_t gbytes = csr_device_bytes(g->csr) + tbytes + ms_prepare_bytes(g->csr, has_t);
+    const int64_t qbytes = csr_quad_bytes(g->csr);
+    int64_t gbytes = csr_device_bytes(g->csr) - (g->csr.quad ? qbytes : 0) + tbytes + ms_prepare_bytes(g->csr, has_t);
     const int64_t new_cap = std::max<int64_t>(s->n_cap, g->csr.n);
-    const int64_t need = s->resident + gbytes + s->slots_total(new_cap);
+    int64_t need = s->resident + gbytes + s->slots_total(new_cap);
+    // the label-correcting kernel's adjacency, where the budget has room for
+    // it (else this server's searches of the graph walk its rows)
+    const bool want_q =
+        bfs_wants_quads(g->csr, graph_params(g)) && need + qbytes <= s->cfg.mem_budget_bytes;
+    if (want_q) {
+        gbytes += qbytes;
+        need += qbytes;
+    }
     if (need > s->cfg.mem_budget_bytes) {
         ++s->rejected;
         return fail(GBFS_ERR_BUDGET, "graph plus slot workspaces exceed the memory budget (" + std::to_string(need) +
@@ -572,7 +581,12 @@ extern "C" int gbfs_server_add_graph(gbfs_server *s, gbfs_graph *g, int32_t *gra
         int rc = want_t ? csr_build_transpose(g->csr, g->stream, err) : GBFS_OK;
         if (!rc) rc = ms_prepare(g->csr, g->stream, err);
         if (rc) return fail(rc, err);
+        if (want_q && csr_build_quads(g->csr, g->stream, err) != GBFS_OK) cudaGetLastError();
         csr_snapshot = g->csr;
+        if (!want_q) {
+            csr_snapshot.quad = nullptr;
+            csr_snapshot.over = nullptr;
+        }
     }
     const int32_t gid = s->next_gid++;
     SrvGraph sg;
