@@ -885,7 +885,7 @@ done:
 
 }  // namespace
 
-int csr_check_symmetric(const DeviceCsr &c, cudaStream_t st, bool &sym, std::string &err)
+int csr_check_symmetric(DeviceCsr &c, cudaStream_t st, bool &sym, std::string &err)
 {
     int rc = GBFS_OK;
     int *flags = nullptr, *copy = nullptr;
@@ -914,6 +914,7 @@ int csr_check_symmetric(const DeviceCsr &c, cudaStream_t st, bool &sym, std::str
         CK(cudaMemcpyAsync(h, flags, 8, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         sym = h[1] == 0;
+        c.sorted_rows = h[0] == 0;
     }
 done:
     if (flags) cudaFree(flags);
@@ -928,6 +929,7 @@ int csr_hub_first(DeviceCsr &c, cudaStream_t st, std::string &err)
                 : hub_first_rows((const int *)c.row, c.n, c.m, c.col, st, err);
     if (rc) goto done;
     c.hub_rows = true;
+    c.sorted_rows = false;
 done:
     return rc;
 }
@@ -1121,10 +1123,9 @@ int64_t csr_device_bytes(const DeviceCsr &c)
     int64_t b = (c.wide ? 8 : 4) * (n + 1) + 4 * m + 4 * ((n + 31) / 32) + 4 * n;  // row, col, zmask, heavy list
     if (c.first) b += 4 * n;
     if (c.second) b += 4 * n;
-    if (c.pieces) b += 8 * (int64_t)c.npieces;
+    b += c.pieces_bytes;
     if (c.trow) b += 4 * (n + 1 + m) + 4 * n;                    // trow, tcol, theavy
     if (c.tfirst) b += 4 * n;
-    if (c.tpieces) b += 8 * (int64_t)c.ntpieces;
     if (c.quad) b += csr_quad_bytes(c);
     return b;
 }
@@ -1308,6 +1309,7 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
         rc = build_rows<int>(n, m, (int64_t)h_total, d_src, d_dst, flags, deg, ss, lcnt, st, out.row, out.col,
                              out.m, err);
     if (rc) goto done;
+    out.sorted_rows = true;
     {
         unsigned h_scan_status[3] = {0, 0, 0};
         CK(cudaMemcpyAsync(h_scan_status, ss.ctl, 12, cudaMemcpyDeviceToHost, st));

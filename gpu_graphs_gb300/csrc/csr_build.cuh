@@ -28,6 +28,7 @@ struct DeviceCsr {
     int *first = nullptr;      // n
     int *second = nullptr;     // n; not allocated for hub-first rows (probed at the first entry alone)
     bool hub_rows = false;     // rows are hub-first (csr_hub_first ran)
+    bool sorted_rows = false;  // every row is known to be ascending
     // fixed-width adjacency of a small-degree graph, built on demand by
     // csr_build_quads for the label-correcting kernel: quad[v] holds row v's
     // entries, -1 past its end; a row of more than four keeps its first three
@@ -40,6 +41,7 @@ struct DeviceCsr {
     // degree > 2 * MS_PIECE contributes {vertex, j} for its j-th MS_PIECE edges
     int2 *pieces = nullptr;
     int32_t npieces = 0;
+    int64_t pieces_bytes = 0;  // of pieces and tpieces together
     bool pieces_built = false;
     // transpose (in-edges), built on demand for bottom-up steps on graphs
     // whose in-edges differ from their out-edges; rows unsorted
@@ -72,8 +74,9 @@ int csr_adopt(int32_t n, int64_t m, int *d_row, int *d_col, cudaStream_t st, Dev
 int csr_adopt64(int32_t n, int64_t m, long long *d_row, int *d_col, cudaStream_t st, DeviceCsr &out,
                 std::string &err);
 
-// in-edges == out-edges?  Rows need not be sorted (a sorted copy is checked).
-int csr_check_symmetric(const DeviceCsr &c, cudaStream_t st, bool &sym, std::string &err);
+// in-edges == out-edges?  Rows need not be sorted (a sorted copy is checked);
+// c.sorted_rows is set from what the check finds.
+int csr_check_symmetric(DeviceCsr &c, cudaStream_t st, bool &sym, std::string &err);
 
 // Move each row's highest-degree neighbour to the row's front.
 int csr_hub_first(DeviceCsr &c, cudaStream_t st, std::string &err);

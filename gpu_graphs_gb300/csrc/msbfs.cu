@@ -24,7 +24,6 @@
 // Levels are separated by the bounded grid barrier of common.cuh.
 #include <algorithm>
 #include <cstddef>
-#include <vector>
 
 #include "blockq.cuh"
 #include "msbfs.cuh"
@@ -629,10 +628,20 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) k_msbfs(MsArgs a)
     grid_exit(&ctrl->bar, &ctrl->t_exit);
 }
 
-__global__ void k_heavy_degrees(const int *__restrict__ row, const int *__restrict__ heavy, int nheavy, int *deg)
+// Appends {vertex, j} for the j-th MS_PIECE edges of every listed row longer
+// than MS_HUGE (in no particular order of the rows).
+template <typename RT>
+__global__ void k_pieces(const RT *__restrict__ row, const int *__restrict__ heavy, int nheavy, int2 *pieces,
+                         unsigned *cnt)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nheavy; i += gridDim.x * blockDim.x)
-        deg[i] = row[heavy[i] + 1] - row[heavy[i]];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nheavy; i += gridDim.x * blockDim.x) {
+        const int v = heavy[i];
+        const int d = (int)(row[v + 1] - row[v]);
+        if (d <= MS_HUGE) continue;
+        const unsigned np = (unsigned)((d + MS_PIECE - 1) / MS_PIECE);
+        const unsigned at = atomicAdd(cnt, np);
+        for (unsigned j = 0; j < np; j++) pieces[at + j] = make_int2(v, (int)j);
+    }
 }
 
 size_t ms_smem_bytes()
@@ -643,57 +652,52 @@ size_t ms_smem_bytes()
 
 }  // namespace
 
+namespace {
+
+// Room for the pieces of m edges: a row of degree d > 2 * MS_PIECE gives
+// ceil(d / MS_PIECE) < 1.5 d / MS_PIECE of them.
+int64_t pieces_room(int64_t m) { return 3 * m / (2 * MS_PIECE) + 1; }
+
+}  // namespace
+
 int64_t ms_prepare_bytes(const DeviceCsr &g, bool transpose)
 {
-    // rows of degree d > 2 * MS_PIECE give ceil(d / MS_PIECE) < 1.5 d / MS_PIECE pieces
-    const int64_t one = (int64_t)sizeof(int2) * (3 * g.m / (2 * MS_PIECE) + 1);
+    const int64_t one = (int64_t)sizeof(int2) * pieces_room(g.m);
     return (g.pieces_built ? 0 : one) + (transpose && !g.tpieces_built ? one : 0);
 }
 
 namespace {
 
-// The pull pieces of one adjacency (out-edge rows, or the transpose's
-// in-edge rows): {vertex, j} for the j-th MS_PIECE edges of every heavy row
-// longer than MS_HUGE.
-int build_pieces(const int *row, const int *heavy, int nheavy, cudaStream_t st, int2 *&out, int32_t &count,
-                 std::string &err)
+// The pieces of one adjacency (out-edge rows, or the transpose's in-edge
+// rows); nheavy = 0: none.
+template <typename RT>
+int build_pieces(const RT *row, const int *heavy, int nheavy, int64_t m, cudaStream_t st, int2 *&out, int32_t &count,
+                 int64_t &bytes, std::string &err)
 {
-    std::vector<int2> h_pieces;
-    if (nheavy > 0) {
-        int *deg = nullptr;
-        std::vector<int> h_heavy(nheavy), h_deg(nheavy);
-        cudaError_t e = cudaMalloc(&deg, sizeof(int) * (size_t)nheavy);
-        if (e == cudaSuccess) {
-            k_heavy_degrees<<<std::max(1, std::min(1216, (nheavy + 255) / 256)), 256, 0, st>>>(row, heavy, nheavy,
-                                                                                             deg);
-            e = cudaMemcpyAsync(h_deg.data(), deg, sizeof(int) * (size_t)nheavy, cudaMemcpyDeviceToHost, st);
-        }
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(h_heavy.data(), heavy, sizeof(int) * (size_t)nheavy, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        cudaFree(deg);
-        if (e != cudaSuccess) {
-            err = std::string("pull pieces: ") + cudaGetErrorString(e);
-            return GBFS_ERR_CUDA;
-        }
-        for (int i = 0; i < nheavy; i++)
-            if (h_deg[i] > MS_HUGE)
-                for (int j = 0; j * MS_PIECE < h_deg[i]; j++) h_pieces.push_back(make_int2(h_heavy[i], j));
-    }
+    out = nullptr;
+    count = 0;
+    if (nheavy <= 0) return GBFS_OK;
     int2 *d = nullptr;
-    if (!h_pieces.empty()) {
-        cudaError_t e = cudaMalloc(&d, sizeof(int2) * h_pieces.size());
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(d, h_pieces.data(), sizeof(int2) * h_pieces.size(), cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) {
-            cudaFree(d);
-            err = std::string("pull pieces: ") + cudaGetErrorString(e);
-            return e == cudaErrorMemoryAllocation ? GBFS_ERR_OOM : GBFS_ERR_CUDA;
-        }
+    unsigned *d_cnt = nullptr, h_cnt = 0;
+    const size_t room = sizeof(int2) * (size_t)pieces_room(m);
+    cudaError_t e = cudaMalloc(&d, room);
+    if (e == cudaSuccess) e = cudaMalloc(&d_cnt, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, sizeof(unsigned), st);
+    if (e == cudaSuccess) {
+        k_pieces<RT><<<std::max(1, std::min(1216, (nheavy + 255) / 256)), 256, 0, st>>>(row, heavy, nheavy, d, d_cnt);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h_cnt, d_cnt, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d_cnt);
+    if (e != cudaSuccess) {
+        cudaFree(d);
+        err = std::string("pull pieces: ") + cudaGetErrorString(e);
+        return e == cudaErrorMemoryAllocation ? GBFS_ERR_OOM : GBFS_ERR_CUDA;
     }
     out = d;
-    count = (int32_t)h_pieces.size();
+    count = (int32_t)h_cnt;
+    bytes += (int64_t)room;
     return GBFS_OK;
 }
 
@@ -703,12 +707,14 @@ int ms_prepare(DeviceCsr &g, cudaStream_t st, std::string &err)
 {
     if (!g.pieces_built) {
         const int nh = g.max_degree > MS_HUGE ? g.nheavy : 0;
-        const int rc = build_pieces(g.row, g.heavy, nh, st, g.pieces, g.npieces, err);
+        const int rc =
+            g.wide ? build_pieces(g.row64, g.heavy, nh, g.m, st, g.pieces, g.npieces, g.pieces_bytes, err)
+                   : build_pieces(g.row, g.heavy, nh, g.m, st, g.pieces, g.npieces, g.pieces_bytes, err);
         if (rc) return rc;
         g.pieces_built = true;
     }
     if (g.trow && !g.tpieces_built) {
-        const int rc = build_pieces(g.trow, g.theavy, g.ntheavy, st, g.tpieces, g.ntpieces, err);
+        const int rc = build_pieces(g.trow, g.theavy, g.ntheavy, g.m, st, g.tpieces, g.ntpieces, g.pieces_bytes, err);
         if (rc) return rc;
         g.tpieces_built = true;
     }

@@ -10,15 +10,23 @@
 // and -1 for the source and for unreached vertices, so one graph and source
 // give one parent array and every entry is a valid BFS-tree parent.
 //
-// Symmetric graphs pull: each reached vertex scans its own row for the
-// smallest neighbour one level closer (one thread per light row, one warp
-// per row of degree > HEAVY_DEGREE), no atomics.  Directed graphs push: every
-// reached u offers itself to the out-neighbours one level further with
-// atomicMin, after a plain-load filter (parent values only decrease).
+// A vertex of level 1 has one possible parent, the source.  The others:
+// symmetric graphs pull: each vertex looks for the smallest neighbour one
+// level closer, in ascending rows up to the first hit (one thread per row of
+// up to HEAVY_DEGREE entries, one warp per longer row, and the rows past
+// MS_HUGE in pieces of MS_PIECE over all warps with an atomicMin per piece).
+// Directed graphs push: every reached u offers itself to the out-neighbours
+// one level further with atomicMin, after a plain-load filter (parent values
+// only decrease), one warp per row or piece.
+//
+// The longest rows bounded this: RMAT-20 with its search took 1,033 us with a
+// warp to each row, walked to its end (900 of them in the heavy rows' kernel),
+// and takes 161 us now; the level gathers hit L2.
 #include <algorithm>
 #include <climits>
 
 #include "common.cuh"
+#include "msbfs.cuh"
 #include "parents.cuh"
 
 namespace gbfs {
@@ -27,20 +35,55 @@ namespace {
 
 constexpr int PT = 256;
 
+// Smallest entry u of row entries [b, e) with level[u] == want; INT_MAX if
+// none.  The whole warp walks them, 128 a step; sorted: ascending entries,
+// the first hit ends the walk.  All 32 lanes get the result.
 template <typename RT>
-__global__ void k_parents_pull_light(const RT *__restrict__ row, const int *__restrict__ col, int n,
-                                     const int *__restrict__ level, int *__restrict__ parent)
+__device__ __forceinline__ int warp_min_at(const int *__restrict__ col, RT b, RT e, const int *__restrict__ level,
+                                           int want, bool sorted, int lane)
+{
+    int best = INT_MAX;
+    for (RT i0 = b; i0 < e; i0 += 128) {
+        int u[4], l[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const RT i = i0 + t * 32 + lane;
+            u[t] = i < e ? __ldg(col + i) : -1;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++) l[t] = u[t] >= 0 ? __ldg(level + u[t]) : -2;
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+            if (l[t] == want) best = min(best, u[t]);
+        if (sorted && __any_sync(FULL, best != INT_MAX)) break;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(FULL, best, o));
+    return best;
+}
+
+template <typename RT>
+__global__ void k_parents_pull_light(const RT *__restrict__ row, const int *__restrict__ col, int n, int source,
+                                     bool sorted, const int *__restrict__ level, int *__restrict__ parent)
 {
     for (long long v = (long long)blockIdx.x * PT + threadIdx.x; v < n; v += (long long)gridDim.x * PT) {
         const int lv = level[v];
-        const RT b = row[v], e = row[v + 1];
-        if (lv > 0 && e - b > HEAVY_DEGREE) continue;  // the heavy kernel's row
-        int best = -1;
-        if (lv > 0) {
-            best = INT_MAX;
-            for (RT i = b; i < e; i++) {
-                const int u = col[i];
-                if (u < best && level[u] == lv - 1) best = u;
+        int best = lv == 1 ? source : -1;
+        if (lv > 1) {
+            best = INT_MAX;  // stays so in a long row: the heavy kernel's
+            const RT b = row[v], e = row[v + 1];
+            if (e - b <= HEAVY_DEGREE) {
+                for (RT i = b; i < e; i += 4) {
+                    int u[4], l[4];
+#pragma unroll
+                    for (int t = 0; t < 4; t++) u[t] = __ldg(col + (i + t < e ? i + t : e - 1));
+#pragma unroll
+                    for (int t = 0; t < 4; t++) l[t] = __ldg(level + u[t]);
+#pragma unroll
+                    for (int t = 0; t < 4; t++)
+                        if (l[t] == lv - 1) best = min(best, u[t]);
+                    if (sorted && best != INT_MAX) break;
+                }
             }
         }
         parent[v] = best;
@@ -49,48 +92,72 @@ __global__ void k_parents_pull_light(const RT *__restrict__ row, const int *__re
 
 template <typename RT>
 __global__ void k_parents_pull_heavy(const RT *__restrict__ row, const int *__restrict__ col,
-                                     const int *__restrict__ heavy, int nheavy, const int *__restrict__ level,
-                                     int *__restrict__ parent)
+                                     const int *__restrict__ heavy, int nheavy, const int2 *__restrict__ pieces,
+                                     int npieces, bool sorted, const int *__restrict__ level, int *parent)
 {
     const long long gw = ((long long)blockIdx.x * PT + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * PT) >> 5;
     const int lane = threadIdx.x & 31;
+    for (long long c = gw; c < npieces; c += nw) {
+        const int2 pc = __ldg(pieces + c);
+        const int lv = __ldg(level + pc.x);
+        if (lv <= 1) continue;  // written by the light kernel
+        const RT b = row[pc.x] + (RT)pc.y * MS_PIECE;
+        const RT e = min(row[pc.x + 1], b + MS_PIECE);
+        // an earlier piece of an ascending row has the answer (one read,
+        // broadcast: the branch is the warp's)
+        if (sorted && __shfl_sync(FULL, ld_relaxed_i32(parent + pc.x), 0) <= __ldg(col + b)) continue;
+        const int best = warp_min_at(col, b, e, level, lv - 1, sorted, lane);
+        if (lane == 0 && best != INT_MAX) atomicMin(parent + pc.x, best);
+    }
     for (long long h = gw; h < nheavy; h += nw) {
-        const int v = heavy[h];
-        const int lv = level[v];
-        if (lv <= 0) continue;  // written by the light kernel
-        int best = INT_MAX;
-        for (RT i = row[v] + lane; i < row[v + 1]; i += 32) {
-            const int u = col[i];
-            if (u < best && level[u] == lv - 1) best = u;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(FULL, best, o));
+        const int v = __ldg(heavy + h);
+        const int lv = __ldg(level + v);
+        const RT b = row[v], e = row[v + 1];
+        if (lv <= 1 || (npieces > 0 && e - b > MS_HUGE)) continue;
+        const int best = warp_min_at(col, b, e, level, lv - 1, sorted, lane);
         if (lane == 0) parent[v] = best;
     }
 }
 
-__global__ void k_parents_init(int n, const int *__restrict__ level, int *__restrict__ parent)
+__global__ void k_parents_init(int n, int source, const int *__restrict__ level, int *__restrict__ parent)
 {
     for (long long v = (long long)blockIdx.x * PT + threadIdx.x; v < n; v += (long long)gridDim.x * PT)
-        parent[v] = level[v] > 0 ? INT_MAX : -1;
+        parent[v] = level[v] > 1 ? INT_MAX : level[v] == 1 ? source : -1;
 }
 
-// one warp per vertex u: offer u to the out-neighbours one level further
+// offer u, of level lu, to its out-neighbours [b, e) of the next level
+template <typename RT>
+__device__ __forceinline__ void warp_offer(int u, int lu, const int *__restrict__ col, RT b, RT e,
+                                           const int *__restrict__ level, int *parent, int lane)
+{
+    for (RT i = b + lane; i < e; i += 32) {
+        const int v = __ldg(col + i);
+        if (__ldg(level + v) == lu + 1 && ld_relaxed_i32(parent + v) > u) atomicMin(parent + v, u);
+    }
+}
+
 template <typename RT>
 __global__ void k_parents_push(const RT *__restrict__ row, const int *__restrict__ col, int n,
-                               const int *__restrict__ level, int *parent)
+                               const int2 *__restrict__ pieces, int npieces, const int *__restrict__ level,
+                               int *parent)
 {
     const long long gw = ((long long)blockIdx.x * PT + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * PT) >> 5;
     const int lane = threadIdx.x & 31;
+    for (long long c = gw; c < npieces; c += nw) {
+        const int2 pc = __ldg(pieces + c);
+        const int lu = __ldg(level + pc.x);
+        if (lu < 1) continue;  // unreached, or the source (its offers are in place)
+        const RT b = row[pc.x] + (RT)pc.y * MS_PIECE;
+        warp_offer(pc.x, lu, col, b, min(row[pc.x + 1], b + MS_PIECE), level, parent, lane);
+    }
     for (long long u = gw; u < n; u += nw) {
-        const int lu = level[u];
-        if (lu < 0) continue;
-        for (RT i = row[u] + lane; i < row[u + 1]; i += 32) {
-            const int v = col[i];
-            if (level[v] == lu + 1 && parent[v] > (int)u) atomicMin(parent + v, (int)u);
-        }
+        const int lu = __ldg(level + u);
+        if (lu < 1) continue;
+        const RT b = row[u], e = row[u + 1];
+        if (npieces > 0 && e - b > MS_HUGE) continue;
+        warp_offer((int)u, lu, col, b, e, level, parent, lane);
     }
 }
 
@@ -105,28 +172,32 @@ int grid_of(long long work, int cap)
 namespace {
 
 template <typename RT>
-cudaError_t parents_launch(const DeviceCsr &g, const RT *row, bool symmetric, const int *d_level, int *d_parent,
-                           cudaStream_t st)
+cudaError_t parents_launch(const DeviceCsr &g, const RT *row, bool symmetric, int source, const int *d_level,
+                           int *d_parent, cudaStream_t st)
 {
+    const int np = g.pieces ? g.npieces : 0;
     if (symmetric) {
-        k_parents_pull_light<RT><<<grid_of(g.n, 152 * 16), PT, 0, st>>>(row, g.col, g.n, d_level, d_parent);
+        k_parents_pull_light<RT><<<grid_of(g.n, 152 * 16), PT, 0, st>>>(row, g.col, g.n, source, g.sorted_rows,
+                                                                        d_level, d_parent);
         if (g.nheavy > 0)
-            k_parents_pull_heavy<RT><<<grid_of((long long)g.nheavy * 32, 152 * 16), PT, 0, st>>>(
-                row, g.col, g.heavy, g.nheavy, d_level, d_parent);
+            k_parents_pull_heavy<RT><<<grid_of(((long long)g.nheavy + np) * 32, 152 * 16), PT, 0, st>>>(
+                row, g.col, g.heavy, g.nheavy, g.pieces, np, g.sorted_rows, d_level, d_parent);
     } else {
-        k_parents_init<<<grid_of(g.n, 152 * 16), PT, 0, st>>>(g.n, d_level, d_parent);
-        k_parents_push<RT><<<grid_of((long long)g.n * 32, 152 * 16), PT, 0, st>>>(row, g.col, g.n, d_level, d_parent);
+        k_parents_init<<<grid_of(g.n, 152 * 16), PT, 0, st>>>(g.n, source, d_level, d_parent);
+        k_parents_push<RT><<<grid_of((long long)g.n * 32, 152 * 16), PT, 0, st>>>(row, g.col, g.n, g.pieces, np,
+                                                                                 d_level, d_parent);
     }
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t parents_enqueue(const DeviceCsr &g, bool symmetric, const int *d_level, int *d_parent, cudaStream_t st)
+cudaError_t parents_enqueue(const DeviceCsr &g, bool symmetric, int source, const int *d_level, int *d_parent,
+                            cudaStream_t st)
 {
     if (g.n == 0) return cudaSuccess;
-    return g.wide ? parents_launch(g, (const long long *)g.row64, symmetric, d_level, d_parent, st)
-                  : parents_launch(g, (const int *)g.row, symmetric, d_level, d_parent, st);
+    return g.wide ? parents_launch(g, (const long long *)g.row64, symmetric, source, d_level, d_parent, st)
+                  : parents_launch(g, (const int *)g.row, symmetric, source, d_level, d_parent, st);
 }
 
 }  // namespace gbfs

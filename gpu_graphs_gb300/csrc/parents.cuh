@@ -9,7 +9,9 @@ namespace gbfs {
 
 // parent[v] = smallest u with an edge u -> v and level[u] == level[v] - 1;
 // -1 for level <= 0 (the source, unreached).  d_level must be a complete BFS
-// level array of g.  Enqueued on st; no sync.
-cudaError_t parents_enqueue(const DeviceCsr &g, bool symmetric, const int *d_level, int *d_parent, cudaStream_t st);
+// level array of g from `source`.  Rows longer than MS_HUGE are split over the
+// GPU where g's pieces have been built (ms_prepare).  Enqueued on st; no sync.
+cudaError_t parents_enqueue(const DeviceCsr &g, bool symmetric, int source, const int *d_level, int *d_parent,
+                            cudaStream_t st);
 
 }  // namespace gbfs
