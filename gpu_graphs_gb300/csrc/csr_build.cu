@@ -9,11 +9,12 @@
 //                lanes with the same source so hubs take one atomic)
 //   2. scan      decoupled look-back exclusive scan -> row offsets
 //   3. k_scatter each edge to its row (aggregated atomic cursors)
-//   4. k_bin + k_sort_small / k_sort_medium / k_sort_large
-//                per-row sort: rows <= 32 in registers (warp bitonic), rows
-//                <= 4096 in shared memory (CTA bitonic), longer rows with a
-//                CTA-wide stable LSD radix sort; each row also counts (and
-//                packs to its front) its distinct values when deduplicating
+//   4. k_bin + per-row sorts by length: up to 32 entries in a warp's registers
+//                (k_sort_small), up to 512 (k_sort_warp), up to 4096 in a CTA's
+//                (k_sort_block), longer rows in sorted chunks of 4096 merged
+//                pairwise, every chunk of every row in parallel (k_merge);
+//                each row also counts (and packs to its front) its distinct
+//                values when deduplicating
 //   5. scan + k_compact   packed rows -> final col_idx (dedup only)
 //   6. k_finalize zero-degree bitmap, max degree, non-isolated count
 #include <algorithm>
@@ -30,10 +31,12 @@ namespace {
 
 constexpr int W4_MAX = 128;       // rows up to this length: warp sort, 4 values per lane
 constexpr int W16_MAX = 512;      // rows up to this length: warp sort, 16 values per lane
-constexpr int MED_MAX = 4096;     // rows up to this length sort in shared memory
-constexpr int MED_THREADS = 512;
-constexpr int LARGE_THREADS = 1024;
+constexpr int SB_E = 8;           // values per thread of a CTA sort
+constexpr int MED_MAX = 4096;     // rows up to this length: CTA sort; longer ones in chunks of it
+constexpr int MED_THREADS = MED_MAX / SB_E;
 constexpr int BIN_THREADS = 1024;
+// row classes of k_bin: warp sorts, CTA sorts of 1024, 2048 and 4096, long rows
+enum BinClass : int { BIN_W4, BIN_W16, BIN_1K, BIN_2K, BIN_4K, BIN_LONG, BIN_CLASSES };
 
 #define CK(call)                                                                 \
     do {                                                                         \
@@ -160,30 +163,68 @@ __global__ void k_scatter(const int *__restrict__ src, const int *__restrict__ d
     }
 }
 
-// Rows longer than 32 go to one of four lists by length: up to W4_MAX and
-// up to W16_MAX (warp sorts in registers), up to MED_MAX (CTA sort in shared
-// memory), longer (radix sort).  cnt[0] medium, [1] large, [2] W4, [3] W16.
+struct BinLists {
+    int *list[BIN_CLASSES];
+};
+// What k_bin counts: rows per class, and the long rows' entries, chunks of
+// MED_MAX, and longest row.
+struct BinCounts {
+    unsigned long long long_entries;
+    unsigned rows[BIN_CLASSES];
+    unsigned chunks;
+    int longest;
+};
+
+// Rows longer than 32 go to a list by length.  A CTA ranks its rows with
+// shared counters and takes its places with one global atomic per class
+// (RMAT-22: 96 us with a block scan per class, 30 us so).
 template <typename RT>
-__global__ void k_bin(const RT *__restrict__ row, int n, int *med, int *large, int *w4, int *w16, unsigned *cnt)
+__global__ void k_bin(const RT *__restrict__ row, int n, BinLists lists, BinCounts *cnt)
 {
-    __shared__ int s_warp[33];
-    __shared__ int s_base[4];
+    __shared__ unsigned s_cnt[BIN_CLASSES], s_base[BIN_CLASSES], s_chunks;
+    __shared__ unsigned long long s_entries;
+    __shared__ int s_longest;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n;
          base += (int64_t)gridDim.x * blockDim.x) {
-        int64_t r = base + threadIdx.x;
-        int d = r < n ? (int)(row[r + 1] - row[r]) : 0;
-        const int cls = d <= 32 ? -1 : d <= W4_MAX ? 2 : d <= W16_MAX ? 3 : d <= MED_MAX ? 0 : 1;
-        int tot[4], off[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) off[c] = block_excl_scan(cls == c, s_warp, &tot[c]);
-        if (threadIdx.x == 0)
-            for (int c = 0; c < 4; c++) s_base[c] = tot[c] ? (int)atomicAdd(&cnt[c], (unsigned)tot[c]) : 0;
-        __syncthreads();
-        if (cls >= 0) {
-            int *dst = cls == 0 ? med : cls == 1 ? large : cls == 2 ? w4 : w16;
-            dst[s_base[cls] + off[cls]] = (int)r;
+        if (threadIdx.x < BIN_CLASSES) s_cnt[threadIdx.x] = 0;
+        if (threadIdx.x == 0) {
+            s_chunks = 0;
+            s_entries = 0;
+            s_longest = 0;
         }
         __syncthreads();
+        const int64_t r = base + threadIdx.x;
+        const int d = r < n ? (int)(row[r + 1] - row[r]) : 0;
+        const int cls = d <= 32       ? -1
+                        : d <= W4_MAX  ? BIN_W4
+                        : d <= W16_MAX ? BIN_W16
+                        : d <= 1024    ? BIN_1K
+                        : d <= 2048    ? BIN_2K
+                        : d <= MED_MAX ? BIN_4K
+                                       : BIN_LONG;
+        unsigned off = 0;
+        if (cls >= 0) off = atomicAdd(&s_cnt[cls], 1u);
+        if (cls == BIN_LONG) {
+            atomicAdd(&s_chunks, (unsigned)((d + MED_MAX - 1) / MED_MAX));
+            atomicAdd(&s_entries, (unsigned long long)d);
+            atomicMax(&s_longest, d);
+        }
+        __syncthreads();
+        if (threadIdx.x < BIN_CLASSES)
+            s_base[threadIdx.x] = s_cnt[threadIdx.x] ? atomicAdd(&cnt->rows[threadIdx.x], s_cnt[threadIdx.x]) : 0u;
+        if (threadIdx.x == BIN_CLASSES && s_chunks) {
+            atomicAdd(&cnt->chunks, s_chunks);
+            atomicAdd(&cnt->long_entries, s_entries);
+            atomicMax(&cnt->longest, s_longest);
+        }
+        __syncthreads();
+        if (cls >= 0) {
+            int *list = lists.list[0];
+#pragma unroll
+            for (int c = 1; c < BIN_CLASSES; c++)
+                if (cls == c) list = lists.list[c];
+            list[s_base[cls] + off] = (int)r;
+        }
     }
 }
 
@@ -319,142 +360,298 @@ __global__ void k_sort_warp(const RT *__restrict__ row, const int *__restrict__ 
     }
 }
 
-// One CTA per row of length W16_MAX+1..MED_MAX: bitonic sort in shared memory.
-template <typename RT>
-__global__ void __launch_bounds__(MED_THREADS)
-k_sort_medium(const RT *__restrict__ row, const int *__restrict__ list, const unsigned *cnt,
-              int *tmp, int dedup, int *ucnt)
+// Sorts the CTA's T * SB_E values ascending: afterwards thread t holds values
+// t * SB_E .. t * SB_E + 7.  A bitonic network in which exchanges between a
+// thread's own values and between lanes of a warp stay in registers (68 of
+// the 78 steps of 4096 values) and the others go through shared memory (buf:
+// two buffers of T * SB_E values, so a step needs one barrier).  The network
+// with every step in shared memory took 3.6 ms for the rows of 513 to 4096
+// entries of RMAT-22 (50 M entries); this takes 0.6 ms.
+template <int T>
+__device__ __forceinline__ void block_bitonic_sort(int (&v)[SB_E], int *buf)
 {
-    __shared__ int s[MED_MAX];
+    const int t = (int)threadIdx.x;
+    int4 *b4 = reinterpret_cast<int4 *>(buf);
+    int flip = 0;
+#pragma unroll
+    for (int k = 2; k <= T * SB_E; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j < SB_E) {
+#pragma unroll
+                for (int e = 0; e < SB_E; e++) {
+                    const int p = e ^ j;
+                    if (p > e) {
+                        const bool up = ((t * SB_E + e) & k) == 0;
+                        const int lo = min(v[e], v[p]), hi = max(v[e], v[p]);
+                        v[e] = up ? lo : hi;
+                        v[p] = up ? hi : lo;
+                    }
+                }
+            } else {
+                const bool keep_min = (((t * SB_E) & k) == 0) == (((t * SB_E) & j) == 0);
+                int y[SB_E];
+                if (j < 32 * SB_E) {
+#pragma unroll
+                    for (int e = 0; e < SB_E; e++) y[e] = __shfl_xor_sync(FULL, v[e], j / SB_E);
+                } else {
+                    int4 *s = b4 + flip * (T * SB_E / 4);
+                    flip ^= 1;
+                    // the two halves of a thread's values apart: consecutive
+                    // threads' 16-byte accesses are then consecutive
+                    s[t] = make_int4(v[0], v[1], v[2], v[3]);
+                    s[T + t] = make_int4(v[4], v[5], v[6], v[7]);
+                    __syncthreads();
+                    const int4 a = s[t ^ (j / SB_E)], c = s[T + (t ^ (j / SB_E))];
+                    y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w;
+                    y[4] = c.x; y[5] = c.y; y[6] = c.z; y[7] = c.w;
+                }
+#pragma unroll
+                for (int e = 0; e < SB_E; e++) v[e] = keep_min ? min(v[e], y[e]) : max(v[e], y[e]);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// Packs the CTA's sorted values (thread t: values t * SB_E ..., the first d of
+// them real) into out: all of them, or (dedup) those that differ from their
+// predecessor; `before`: the value before the first (INT_MIN: none).  Returns
+// the count.  buf: T * SB_E values of shared memory.
+template <int T>
+__device__ __forceinline__ int block_pack(const int (&v)[SB_E], int d, bool dedup, int before, int *out, int *buf,
+                                          int *s_warp)
+{
+    __shared__ int s_last[T / 32];
+    const int t = (int)threadIdx.x;
+    if (lane_id() == 31) s_last[t >> 5] = v[SB_E - 1];
+    int prev = __shfl_up_sync(FULL, v[SB_E - 1], 1);
+    __syncthreads();
+    if (lane_id() == 0) prev = t == 0 ? before : s_last[(t >> 5) - 1];
+    unsigned keep = 0;
+#pragma unroll
+    for (int e = 0; e < SB_E; e++) {
+        const int p = e ? v[e - 1] : prev;
+        if (t * SB_E + e < d && (!dedup || v[e] != p)) keep |= 1u << e;
+    }
+    int total;
+    int off = block_excl_scan(__popc(keep), s_warp, &total);
+#pragma unroll
+    for (int e = 0; e < SB_E; e++)
+        if (keep >> e & 1u) buf[off++] = v[e];
+    __syncthreads();
+    if (out)
+        for (int i = t; i < total; i += T) out[i] = buf[i];
+    __syncthreads();
+    return total;
+}
+
+// One CTA of T threads per listed row of up to T * SB_E entries: sort in
+// registers, pack in place, record the count.
+template <int T, typename RT>
+__global__ void __launch_bounds__(T) k_sort_block(const RT *__restrict__ row, const int *__restrict__ list,
+                                                  const unsigned *cnt, int *tmp, int dedup, int *ucnt)
+{
+    __shared__ __align__(16) int s[2 * T * SB_E];
     __shared__ int s_warp[33];
-    const int count = (int)cnt[0];
+    const int count = (int)*cnt;
     for (int li = blockIdx.x; li < count; li += gridDim.x) {
         const int r = list[li];
         const RT b = row[r];
         const int d = (int)(row[r + 1] - b);
-        int P = 64;
-        while (P < d) P <<= 1;
-        for (int i = threadIdx.x; i < P; i += blockDim.x) s[i] = i < d ? tmp[b + i] : INT_MAX;
-        __syncthreads();
-        for (int k = 2; k <= P; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = threadIdx.x; i < P; i += blockDim.x) {
-                    int ixj = i ^ j;
-                    if (ixj > i) {
-                        int a = s[i], c = s[ixj];
-                        bool up = (i & k) == 0;
-                        if ((a > c) == up) {
-                            s[i] = c;
-                            s[ixj] = a;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
+        int v[SB_E];
+#pragma unroll
+        for (int e = 0; e < SB_E; e++) {
+            const int i = e * T + (int)threadIdx.x;  // any order will do before the sort
+            v[e] = i < d ? tmp[b + i] : INT_MAX;
         }
-        // Each thread owns a contiguous run of ceil(P/blockDim) slots.
-        const int per = (P + blockDim.x - 1) / blockDim.x;
-        const int lo = threadIdx.x * per, hi = min(lo + per, d);
-        int c = 0;
-        for (int i = lo; i < hi; i++) c += !dedup || i == 0 || s[i] != s[i - 1];
-        int total;
-        int off = block_excl_scan(c, s_warp, &total);
-        int vals[8];
-        int nv = 0;
-        for (int i = lo; i < hi; i++)
-            if (!dedup || i == 0 || s[i] != s[i - 1]) vals[nv++] = s[i];
-        __syncthreads();
-        for (int k = 0; k < nv; k++) tmp[b + off + k] = vals[k];
+        block_bitonic_sort<T>(v, s);
+        const int total = block_pack<T>(v, d, dedup, INT_MIN, tmp + b, s, s_warp);
         if (threadIdx.x == 0) ucnt[r] = total;
+    }
+}
+
+// ---- rows longer than MED_MAX ----
+// A long row is sorted in chunks of MED_MAX, all chunks of all such rows at
+// once, and its chunks are merged pairwise, one tile of MED_MAX outputs per
+// CTA.  RMAT-22 has 1,794 long rows of 25.5 M entries, the longest 320 K: a
+// radix sort by one CTA per row took 3.5 ms, with that row its tail; chunks
+// and seven merge passes take 0.8 ms.
+
+// The j-th chunk of a row, and where in tmp2 the row's entries have their
+// second place.
+struct Chunk {
+    long long base2;
+    int row, j;
+};
+struct ChunkNext {
+    unsigned long long entries;
+    unsigned chunks, pad;
+};
+
+// The chunks of every listed row; a row's are consecutive.
+template <typename RT>
+__global__ void k_chunks(const RT *__restrict__ row, const int *__restrict__ list, const unsigned *cnt, Chunk *chunks,
+                         ChunkNext *next)
+{
+    const int count = (int)*cnt;
+    for (int li = blockIdx.x * blockDim.x + threadIdx.x; li < count; li += gridDim.x * blockDim.x) {
+        const int r = list[li];
+        const int d = (int)(row[r + 1] - row[r]);
+        const int nc = (d + MED_MAX - 1) / MED_MAX;
+        const unsigned at = atomicAdd(&next->chunks, (unsigned)nc);
+        const long long base2 = (long long)atomicAdd(&next->entries, (unsigned long long)d);
+        for (int j = 0; j < nc; j++) chunks[at + j] = Chunk{base2, r, j};
+    }
+}
+
+// Merge passes a row of d entries needs.
+__host__ __device__ inline int merge_passes(int d)
+{
+    int p = 0;
+    while (((int64_t)MED_MAX << p) < d) p++;
+    return p;
+}
+
+// Sorts every chunk, into tmp2 where the row's number of merge passes is odd
+// (so that its last pass ends in tmp).
+template <typename RT>
+__global__ void __launch_bounds__(MED_THREADS)
+k_sort_chunks(const RT *__restrict__ row, const Chunk *__restrict__ chunks, int nchunks, int *tmp, int *tmp2)
+{
+    __shared__ __align__(16) int s[2 * MED_MAX];
+    __shared__ int s_warp[33];
+    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const Chunk ck = chunks[c];
+        const RT rb = row[ck.row];
+        const int len = (int)(row[ck.row + 1] - rb), at = ck.j * MED_MAX;
+        const int d = min(MED_MAX, len - at);
+        int *from = tmp + rb + at;
+        int v[SB_E];
+#pragma unroll
+        for (int e = 0; e < SB_E; e++) {
+            const int i = e * MED_THREADS + (int)threadIdx.x;
+            v[e] = i < d ? from[i] : INT_MAX;
+        }
+        block_bitonic_sort<MED_THREADS>(v, s);
+        block_pack<MED_THREADS>(v, d, false, INT_MIN, merge_passes(len) & 1 ? tmp2 + ck.base2 + at : from, s, s_warp);
+    }
+}
+
+// How many of the first o merged values of ascending A (na) and B (nb) come
+// from A (equal values: A first).
+__device__ __forceinline__ int merge_split(const int *A, int na, const int *B, int nb, int o)
+{
+    int lo = max(0, o - nb), hi = min(o, na);
+    while (lo < hi) {
+        const int i = (lo + hi) >> 1;
+        if (A[i] <= B[o - 1 - i]) lo = i + 1; else hi = i;
+    }
+    return lo;
+}
+
+// Pass p: runs of MED_MAX << p are merged in pairs.  A chunk's CTA makes the
+// outputs in its place, from one of the row's two places to the other.
+template <typename RT>
+__global__ void __launch_bounds__(MED_THREADS)
+k_merge(const RT *__restrict__ row, const Chunk *__restrict__ chunks, int nchunks, int *tmp, int *tmp2, int p)
+{
+    __shared__ int s[MED_MAX];
+    __shared__ int s_split[2];
+    const int t = (int)threadIdx.x;
+    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const Chunk ck = chunks[c];
+        const RT rb = row[ck.row];
+        const int d = (int)(row[ck.row + 1] - rb);
+        const int left = merge_passes(d) - p;  // passes from here on
+        if (left <= 0) continue;               // this row is done
+        int *one = tmp + rb, *two = tmp2 + ck.base2;
+        const int *from = left & 1 ? two : one;
+        int *to = left & 1 ? one : two;
+        const int64_t w = (int64_t)MED_MAX << p;
+        const int a0 = (ck.j >> (p + 1)) * (int)min(2 * w, (int64_t)INT_MAX);
+        const int b0 = (int)min((int64_t)d, a0 + w), b1 = (int)min((int64_t)d, a0 + 2 * w);
+        const int o0 = ck.j * MED_MAX - a0, o1 = min(o0 + MED_MAX, b1 - a0);
+        const int *A = from + a0, *B = from + b0;
+        const int na = b0 - a0, nb = b1 - b0;
+        if (t < 64 && (t & 31) == 0) s_split[t >> 5] = merge_split(A, na, B, nb, t ? o1 : o0);
+        __syncthreads();
+        const int i0 = s_split[0], i1 = s_split[1];
+        const int ta = i1 - i0, tb = (o1 - o0) - ta;
+        for (int i = t; i < ta; i += MED_THREADS) s[i] = A[i0 + i];
+        for (int i = t; i < tb; i += MED_THREADS) s[ta + i] = B[o0 - i0 + i];
+        __syncthreads();
+        int v[SB_E];
+        const int o = min(t * SB_E, ta + tb);
+        int ia = merge_split(s, ta, s + ta, tb, o), ib = o - ia;
+#pragma unroll
+        for (int e = 0; e < SB_E; e++) {
+            const bool a = ia < ta && (ib >= tb || s[ia] <= s[ta + ib]);
+            v[e] = INT_MAX;
+            if (a) v[e] = s[ia++];
+            else if (ib < tb) v[e] = s[ta + ib++];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < SB_E; e++)
+            if (o + e < ta + tb) s[o + e] = v[e];
+        __syncthreads();
+        for (int i = t; i < ta + tb; i += MED_THREADS) to[ck.j * MED_MAX + i] = s[i];
         __syncthreads();
     }
 }
 
-// One CTA per row longer than MED_MAX: stable LSD radix sort (8-bit digits)
-// ping-ponging between tmp and tmp2 over the row's own range, then packing
-// distinct values into tmp.  Stability within a 1024-element tile comes
-// from match_any ranks inside each warp and per-digit prefixes across warps
-// in warp order.
+// Distinct values of every merged chunk (a value equal to the one before the
+// chunk is not counted), added up per row in ucnt (zeroed by the caller).
 template <typename RT>
-__global__ void __launch_bounds__(LARGE_THREADS)
-k_sort_large(const RT *__restrict__ row, const int *__restrict__ list, const unsigned *cnt,
-             int *tmp, int *tmp2, int key_bits, int dedup, int *ucnt)
+__global__ void __launch_bounds__(MED_THREADS)
+k_chunk_unique(const RT *__restrict__ row, const Chunk *__restrict__ chunks, int nchunks, const int *__restrict__ tmp,
+               int *ccnt, int *ucnt)
 {
-    __shared__ int s_hist[256];
-    __shared__ int s_base[256];
-    __shared__ int s_tile[256];
-    __shared__ unsigned short s_wcnt[LARGE_THREADS / 32][256];
+    __shared__ int s_red[32];
+    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const Chunk ck = chunks[c];
+        const RT b = row[ck.row] + (RT)ck.j * MED_MAX;
+        const int d = (int)min((RT)MED_MAX, row[ck.row + 1] - b);
+        const int *from = tmp + b;
+        int mine = 0;
+        for (int i = threadIdx.x; i < d; i += MED_THREADS) mine += (i == 0 && ck.j == 0) || from[i] != from[i - 1];
+        const int total = block_sum(mine, s_red);
+        if (threadIdx.x == 0) {
+            ccnt[c] = total;
+            atomicAdd(&ucnt[ck.row], total);
+        }
+    }
+}
+
+// The distinct values of every merged chunk into its row of col.
+template <typename RT>
+__global__ void __launch_bounds__(MED_THREADS)
+k_compact_chunks(const RT *__restrict__ row, const RT *__restrict__ row2, const Chunk *__restrict__ chunks,
+                 int nchunks, const int *__restrict__ ccnt, const int *__restrict__ tmp, int *col)
+{
+    __shared__ int s[MED_MAX];
     __shared__ int s_warp[33];
-    const int count = (int)cnt[1];
-    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-    const int nwarps = blockDim.x >> 5;
-    for (int li = blockIdx.x; li < count; li += gridDim.x) {
-        const int r = list[li];
-        const RT b = row[r];
-        const int d = (int)(row[r + 1] - b);
-        int *from = tmp + b, *to = tmp2 + b;
-        for (int shift = 0; shift < key_bits; shift += 8) {
-            for (int i = threadIdx.x; i < 256; i += blockDim.x) s_hist[i] = 0;
-            __syncthreads();
-            for (int i = threadIdx.x; i < d; i += blockDim.x)
-                atomicAdd(&s_hist[((unsigned)from[i] >> shift) & 255u], 1);
-            __syncthreads();
-            if (warp == 0) {  // exclusive scan of 256 bins, 8 per lane
-                int v[8], t = 0;
-                for (int k = 0; k < 8; k++) { v[k] = s_hist[lane * 8 + k]; t += v[k]; }
-                int incl = warp_incl_scan(t);
-                int run = incl - t;
-                for (int k = 0; k < 8; k++) { s_base[lane * 8 + k] = run; run += v[k]; }
-            }
-            __syncthreads();
-            for (int t0 = 0; t0 < d; t0 += blockDim.x) {
-                const int i = t0 + threadIdx.x;
-                const bool ok = i < d;
-                const int x = ok ? from[i] : 0;
-                const int dig = ok ? (int)(((unsigned)x >> shift) & 255u) : 256;
-                for (int k = threadIdx.x; k < nwarps * 256; k += blockDim.x)
-                    s_wcnt[k >> 8][k & 255] = 0;
-                __syncthreads();
-                unsigned peers = __match_any_sync(FULL, dig);
-                int rank = __popc(peers & lanemask_lt());
-                if (ok && (int)lane == __ffs(peers) - 1) s_wcnt[warp][dig] = (unsigned short)__popc(peers);
-                __syncthreads();
-                for (int k = threadIdx.x; k < 256; k += blockDim.x) {
-                    int run = 0;
-                    for (int w = 0; w < nwarps; w++) {
-                        int c = s_wcnt[w][k];
-                        s_wcnt[w][k] = (unsigned short)run;
-                        run += c;
-                    }
-                    s_tile[k] = run;
-                }
-                __syncthreads();
-                if (ok) to[s_base[dig] + s_wcnt[warp][dig] + rank] = x;
-                __syncthreads();
-                for (int k = threadIdx.x; k < 256; k += blockDim.x) s_base[k] += s_tile[k];
-                __syncthreads();
-            }
-            int *t = from; from = to; to = t;
-        }
-        // Sorted values are in `from`; pack (distinct) values into tmp.
-        if (from == tmp + b) {
-            for (int i = threadIdx.x; i < d; i += blockDim.x) tmp2[b + i] = from[i];
-            __syncthreads();
-            from = tmp2 + b;
-        }
-        int written = 0;
-        for (int t0 = 0; t0 < d; t0 += blockDim.x) {
-            const int i = t0 + threadIdx.x;
-            const int x = i < d ? from[i] : 0;
-            const int keep = i < d && (!dedup || i == 0 || x != from[i - 1]);
-            int total;
-            int off = block_excl_scan(keep, s_warp, &total);
-            if (keep) tmp[b + written + off] = x;
-            written += total;
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) ucnt[r] = written;
+    __shared__ int s_red[32], s_rel;
+    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const Chunk ck = chunks[c];
+        int rel = 0;  // distinct values in the row's earlier chunks
+        for (int i = threadIdx.x; i < ck.j; i += MED_THREADS) rel += ccnt[c - ck.j + i];
+        rel = block_sum(rel, s_red);
+        if (threadIdx.x == 0) s_rel = rel;
+        const RT b = row[ck.row] + (RT)ck.j * MED_MAX;
+        const int d = (int)min((RT)MED_MAX, row[ck.row + 1] - b);
+        for (int i = threadIdx.x; i < d; i += MED_THREADS) s[i] = tmp[b + i];
         __syncthreads();
+        int v[SB_E];
+#pragma unroll
+        for (int e = 0; e < SB_E; e++) {
+            const int i = (int)threadIdx.x * SB_E + e;
+            v[e] = i < d ? s[i] : INT_MAX;
+        }
+        int *out = col + row2[ck.row] + s_rel;
+        __syncthreads();
+        block_pack<MED_THREADS>(v, d, true, ck.j ? tmp[b - 1] : INT_MIN, out, s, s_warp);
     }
 }
 
@@ -471,7 +668,7 @@ __global__ void k_compact(const RT *__restrict__ row, const RT *__restrict__ row
         const int64_t r = r0 + lane;
         RT b = 0, o = 0;
         int c = 0;
-        // rows longer than MED_MAX before deduplication: k_compact_long
+        // rows longer than MED_MAX before deduplication: k_compact_chunks
         if (r < n && row[r + 1] - row[r] <= MED_MAX) {
             b = row[r];
             o = row2[r];
@@ -483,23 +680,6 @@ __global__ void k_compact(const RT *__restrict__ row, const RT *__restrict__ row
             const int cj = __shfl_sync(FULL, c, j);
             for (int i = lane; i < cj; i += 32) col[oj + i] = tmp[bj + i];
         }
-    }
-}
-
-// The rows of list[0, cnt[1]) (longer than MED_MAX before deduplication),
-// one CTA per row: a long hub row copied by one warp would set the whole
-// pass's time.
-template <typename RT>
-__global__ void k_compact_long(const RT *__restrict__ row, const RT *__restrict__ row2, const int *__restrict__ list,
-                               const unsigned *cnt, const int *__restrict__ tmp, int *col)
-{
-    const int count = (int)cnt[1];
-    for (int li = blockIdx.x; li < count; li += gridDim.x) {
-        const int r = list[li];
-        const RT b = row[r], o = row2[r];
-        const int c = (int)(row2[r + 1] - o);
-#pragma unroll 4
-        for (int i = threadIdx.x; i < c; i += blockDim.x) col[o + i] = tmp[b + i];
     }
 }
 
@@ -539,19 +719,25 @@ __global__ void k_finalize(const RT *__restrict__ row, int n, unsigned *zmask, i
     }
 }
 
+// Appends the rows with more than HEAVY_DEGREE entries to heavy, with one
+// global atomic per CTA pass (one per warp, all on one counter, took 80 us on
+// RMAT-22; this takes 22).
 template <typename RT>
 __global__ void k_heavy_list(const RT *__restrict__ row, int n, int *heavy, unsigned *cnt)
 {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-        const int64_t v = base + lane_id();
+    __shared__ unsigned s_cnt, s_base;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
+        if (threadIdx.x == 0) s_cnt = 0;
+        __syncthreads();
+        const int64_t v = base + threadIdx.x;
         const bool h = v < n && row[v + 1] - row[v] > HEAVY_DEGREE;
-        const unsigned m = __ballot_sync(FULL, h);
-        if (!m) continue;
-        unsigned pos = 0;
-        if (lane_id() == 0) pos = atomicAdd(cnt, (unsigned)__popc(m));
-        pos = __shfl_sync(FULL, pos, 0);
-        if (h) heavy[pos + __popc(m & lanemask_lt())] = (int)v;
+        unsigned off = 0;
+        if (h) off = atomicAdd(&s_cnt, 1u);
+        __syncthreads();
+        if (threadIdx.x == 0 && s_cnt) s_base = atomicAdd(cnt, s_cnt);
+        __syncthreads();
+        if (h) heavy[s_base + off] = (int)v;
+        __syncthreads();
     }
 }
 
@@ -777,7 +963,7 @@ int finalize_t(DeviceCsr &out, const RT *row, cudaStream_t st, std::string &err)
     {
         // heavy-row list (sized by a first count pass folded into k_heavy_list's atomic)
         CK(cudaMalloc(&out.heavy, sizeof(int) * (size_t)std::max<int64_t>(1, out.n)));
-        k_heavy_list<<<grid_for(out.n, 256), 256, 0, st>>>(row, out.n, out.heavy, &d_res->nheavy);
+        k_heavy_list<<<grid_for(out.n, 1024, 152 * 4), 1024, 0, st>>>(row, out.n, out.heavy, &d_res->nheavy);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(&h, d_res, sizeof(Res), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -794,46 +980,129 @@ int finalize(DeviceCsr &out, cudaStream_t st, std::string &err)
                     : finalize_t(out, (const int *)out.row, st, err);
 }
 
+// The per-row sorts of one column array: lists by length, then one launch per
+// length class.  The lists and the long rows' scratch are freed with it.
+template <typename RT>
+struct RowSorter {
+    void *mem = nullptr;       // lists and counts
+    void *long_mem = nullptr;  // long rows: chunks and their counts
+    int *tmp2 = nullptr;       // long rows: the merges' second place
+    BinLists lists{};
+    BinCounts *d_cnt = nullptr;
+    BinCounts h{};
+    Chunk *chunks = nullptr;
+    int *ccnt = nullptr;
+
+    ~RowSorter()
+    {
+        drop_tmp2();
+        if (mem) cudaFree(mem);
+        if (long_mem) cudaFree(long_mem);
+    }
+
+    // The sorts are done: room for the compacted columns.
+    void drop_tmp2()
+    {
+        if (tmp2) cudaFree(tmp2);
+        tmp2 = nullptr;
+    }
+
+    // Lists by length of n rows of m entries together; enqueued on st.
+    cudaError_t bin(const RT *row, int32_t n, int64_t m, cudaStream_t st)
+    {
+        static const int over[BIN_CLASSES] = {32, W4_MAX, W16_MAX, 1024, 2048, MED_MAX};
+        int64_t cap[BIN_CLASSES], total = 0;
+        for (int c = 0; c < BIN_CLASSES; c++) {
+            cap[c] = std::min<int64_t>(n, m / (over[c] + 1)) + 1;
+            total += cap[c];
+        }
+        cudaError_t e = cudaMalloc(&mem, 256 + sizeof(int) * (size_t)total);
+        if (e != cudaSuccess) return e;
+        d_cnt = (BinCounts *)mem;
+        int *p = (int *)((char *)mem + 256);
+        for (int c = 0; c < BIN_CLASSES; c++) {
+            lists.list[c] = p;
+            p += cap[c];
+        }
+        e = cudaMemsetAsync(mem, 0, 256, st);
+        if (e != cudaSuccess) return e;
+        k_bin<RT><<<grid_for(n, BIN_THREADS, 152 * 4), BIN_THREADS, 0, st>>>(row, n, lists, d_cnt);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_cnt, sizeof(h), cudaMemcpyDeviceToHost, st);
+        return e;
+    }
+
+    // Sorts the rows of tmp (the caller has synchronised st since bin).  Rows
+    // are packed in place and counted in ucnt (n entries), distinct values only
+    // with dedup; then the long rows' are left for compact().
+    cudaError_t sort(const RT *row, int32_t n, int *tmp, int dedup, int *ucnt, cudaStream_t st)
+    {
+        const unsigned *rows = d_cnt->rows;
+        const int thr = 256;
+        cudaError_t e = cudaSuccess;
+        const int nch = (int)h.chunks;
+        if (nch) {
+            const size_t cb = sizeof(Chunk) * (size_t)nch;
+            e = cudaMalloc(&long_mem, 256 + cb + sizeof(int) * (size_t)nch);
+            if (e == cudaSuccess) e = cudaMalloc(&tmp2, sizeof(int) * (size_t)h.long_entries);
+            if (e != cudaSuccess) return e;
+            ChunkNext *next = (ChunkNext *)long_mem;
+            chunks = (Chunk *)((char *)long_mem + 256);
+            ccnt = (int *)((char *)long_mem + 256 + cb);
+            e = cudaMemsetAsync(next, 0, sizeof(ChunkNext), st);
+            if (e == cudaSuccess) e = cudaMemsetAsync(ucnt, 0, sizeof(int) * (size_t)n, st);
+            if (e != cudaSuccess) return e;
+            const int nl = (int)h.rows[BIN_LONG];
+            const int grid = std::min(nch, 152 * 32);
+            k_chunks<RT><<<grid_for(nl, 128), 128, 0, st>>>(row, lists.list[BIN_LONG], rows + BIN_LONG, chunks, next);
+            k_sort_chunks<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, tmp2);
+            const int passes = merge_passes(h.longest);
+            for (int p = 0; p < passes; p++) k_merge<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, tmp2, p);
+            if (dedup) k_chunk_unique<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, ccnt, ucnt);
+        }
+        auto ctas = [](unsigned rows_, int cap) { return std::max(1, std::min((int)rows_, cap)); };
+        if (h.rows[BIN_4K])
+            k_sort_block<512, RT><<<ctas(h.rows[BIN_4K], 152 * 16), 512, 0, st>>>(row, lists.list[BIN_4K],
+                                                                                 rows + BIN_4K, tmp, dedup, ucnt);
+        if (h.rows[BIN_2K])
+            k_sort_block<256, RT><<<ctas(h.rows[BIN_2K], 152 * 32), 256, 0, st>>>(row, lists.list[BIN_2K],
+                                                                                 rows + BIN_2K, tmp, dedup, ucnt);
+        if (h.rows[BIN_1K])
+            k_sort_block<128, RT><<<ctas(h.rows[BIN_1K], 152 * 64), 128, 0, st>>>(row, lists.list[BIN_1K],
+                                                                                 rows + BIN_1K, tmp, dedup, ucnt);
+        if (h.rows[BIN_W16])
+            k_sort_warp<16, RT><<<152 * 8, 256, 0, st>>>(row, lists.list[BIN_W16], rows + BIN_W16, tmp, dedup, ucnt);
+        if (h.rows[BIN_W4])
+            k_sort_warp<4, RT><<<152 * 8, 256, 0, st>>>(row, lists.list[BIN_W4], rows + BIN_W4, tmp, dedup, ucnt);
+        k_sort_small<RT><<<grid_for((int64_t)n * 32, thr), thr, 0, st>>>(row, n, tmp, dedup, ucnt);
+        return cudaGetLastError();
+    }
+
+    // The long rows' distinct values into col (row2: the offsets there).
+    cudaError_t compact(const RT *row, const RT *row2, const int *tmp, int *col, cudaStream_t st)
+    {
+        if (!h.chunks) return cudaSuccess;
+        k_compact_chunks<RT><<<std::min((int)h.chunks, 152 * 32), MED_THREADS, 0, st>>>(row, row2, chunks, (int)h.chunks,
+                                                                                       ccnt, tmp, col);
+        return cudaGetLastError();
+    }
+};
+
 // Sort every row of (row, col) in place (no dedup).  Scratch is allocated
 // and freed here.  Synchronises st.
 template <typename RT>
 int sort_rows_inplace(const RT *row, int *col, int32_t n, int64_t m, cudaStream_t st, std::string &err)
 {
     int rc = GBFS_OK;
-    int *ucnt = nullptr, *med = nullptr, *large = nullptr, *tmp2 = nullptr, *w4 = nullptr, *w16 = nullptr;
-    unsigned *lcnt = nullptr;
-    int key_bits = 1;
-    const int thr = 256;
+    int *ucnt = nullptr;
+    RowSorter<RT> sorter;
     CK(cudaMalloc(&ucnt, sizeof(int) * ((size_t)n + 1)));
-    CK(cudaMalloc(&med, sizeof(int) * (size_t)n));
-    CK(cudaMalloc(&large, sizeof(int) * (size_t)n));
-    CK(cudaMalloc(&w4, sizeof(int) * (size_t)n));
-    CK(cudaMalloc(&w16, sizeof(int) * (size_t)n));
-    CK(cudaMalloc(&lcnt, 16));
-    CK(cudaMalloc(&tmp2, sizeof(int) * (size_t)std::max<int64_t>(m, 1)));
-    CK(cudaMemsetAsync(lcnt, 0, 16, st));
-    k_bin<RT><<<grid_for(n, BIN_THREADS, 152 * 4), BIN_THREADS, 0, st>>>(row, n, med, large, w4, w16, lcnt);
-    CK(cudaGetLastError());
-    k_sort_small<RT><<<grid_for((int64_t)n * 32, thr), thr, 0, st>>>(row, n, col, 0, ucnt);
-    CK(cudaGetLastError());
-    k_sort_warp<4, RT><<<152 * 8, 256, 0, st>>>(row, w4, lcnt + 2, col, 0, ucnt);
-    CK(cudaGetLastError());
-    k_sort_warp<16, RT><<<152 * 8, 256, 0, st>>>(row, w16, lcnt + 3, col, 0, ucnt);
-    CK(cudaGetLastError());
-    k_sort_medium<RT><<<152 * 4, MED_THREADS, 0, st>>>(row, med, lcnt, col, 0, ucnt);
-    CK(cudaGetLastError());
-    while (key_bits < 31 && (1LL << key_bits) < (int64_t)n) key_bits++;
-    k_sort_large<RT><<<152 * 2, LARGE_THREADS, 0, st>>>(row, large, lcnt, col, tmp2, key_bits, 0, ucnt);
-    CK(cudaGetLastError());
+    CK(sorter.bin(row, n, m, st));
+    CK(cudaStreamSynchronize(st));
+    CK(sorter.sort(row, n, col, 0, ucnt, st));
     CK(cudaStreamSynchronize(st));
 done:
     if (ucnt) cudaFree(ucnt);
-    if (med) cudaFree(med);
-    if (large) cudaFree(large);
-    if (w4) cudaFree(w4);
-    if (w16) cudaFree(w16);
-    if (lcnt) cudaFree(lcnt);
-    if (tmp2) cudaFree(tmp2);
     return rc;
 }
 
@@ -1002,7 +1271,7 @@ int csr_build_transpose(DeviceCsr &c, cudaStream_t st, std::string &err)
         k_in_scatter<<<grid_for((int64_t)n * 32, 256), 256, 0, st>>>(c.row, c.col, n, cursor, tcol);
         CK(cudaGetLastError());
     }
-    k_heavy_list<<<grid_for(n, 256), 256, 0, st>>>((const int *)trow, n, theavy, d_nheavy);
+    k_heavy_list<<<grid_for(n, 1024, 152 * 4), 1024, 0, st>>>((const int *)trow, n, theavy, d_nheavy);
     CK(cudaGetLastError());
     // in-rows hub-first (the in-neighbour of highest in-degree, the likeliest
     // to be reached early, is probed first), then their first entries
@@ -1167,18 +1436,18 @@ inline cudaError_t scan_rows(const int *in, long long *out, int64_t n, ScanScrat
 // columns move to row_out / col_out.
 template <typename RT>
 int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_dst, unsigned flags,
-               const int *deg, ScanScratch &ss, unsigned *lcnt, cudaStream_t st, RT *&row_out, int *&col_out,
-               int64_t &m_out, std::string &err)
+               const int *deg, ScanScratch &ss, cudaStream_t st, RT *&row_out, int *&col_out, int64_t &m_out,
+               std::string &err)
 {
     int rc = GBFS_OK;
     const bool dedup = flags & GBFS_DEDUP;
     RT *row = nullptr, *cursor = nullptr, *row2 = nullptr;
-    int *tmp = nullptr, *tmp2 = nullptr, *ucnt = nullptr, *med = nullptr, *large = nullptr, *w4 = nullptr,
-        *w16 = nullptr, *col = nullptr;
-    int key_bits = 1;
+    int *tmp = nullptr, *ucnt = nullptr, *col = nullptr;
     const int thr = 256;
+    RowSorter<RT> sorter;
     CK(cudaMalloc(&row, sizeof(RT) * ((size_t)n + 1)));
     CK(scan_rows(deg, row, n, ss, st));
+    CK(sorter.bin(row, n, md, st));
     CK(cudaMalloc(&cursor, sizeof(RT) * ((size_t)n + 1)));
     CK(cudaMemcpyAsync(cursor, row, sizeof(RT) * ((size_t)n + 1), cudaMemcpyDeviceToDevice, st));
     CK(cudaMalloc(&tmp, sizeof(int) * (size_t)std::max<int64_t>(md, 1)));
@@ -1186,30 +1455,13 @@ int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_
         k_scatter<RT><<<grid_for(m, thr), thr, 0, st>>>(d_src, d_dst, m, n, flags, cursor, tmp);
         CK(cudaGetLastError());
     }
+    CK(cudaMalloc(&ucnt, sizeof(int) * ((size_t)n + 1)));
     CK(cudaStreamSynchronize(st));
     cudaFree(cursor);
     cursor = nullptr;
 
     // Per-row sort (+ distinct count).
-    CK(cudaMalloc(&ucnt, sizeof(int) * ((size_t)n + 1)));
-    CK(cudaMalloc(&med, sizeof(int) * (size_t)n));
-    CK(cudaMalloc(&large, sizeof(int) * (size_t)n));
-    CK(cudaMalloc(&w4, sizeof(int) * (size_t)n));
-    CK(cudaMalloc(&w16, sizeof(int) * (size_t)n));
-    k_bin<RT><<<grid_for(n, BIN_THREADS, 152 * 4), BIN_THREADS, 0, st>>>(row, n, med, large, w4, w16, lcnt);
-    CK(cudaGetLastError());
-    k_sort_small<RT><<<grid_for((int64_t)n * 32, thr), thr, 0, st>>>(row, n, tmp, dedup, ucnt);
-    CK(cudaGetLastError());
-    k_sort_warp<4, RT><<<152 * 8, 256, 0, st>>>(row, w4, lcnt + 2, tmp, dedup, ucnt);
-    CK(cudaGetLastError());
-    k_sort_warp<16, RT><<<152 * 8, 256, 0, st>>>(row, w16, lcnt + 3, tmp, dedup, ucnt);
-    CK(cudaGetLastError());
-    k_sort_medium<RT><<<152 * 4, MED_THREADS, 0, st>>>(row, med, lcnt, tmp, dedup, ucnt);
-    CK(cudaGetLastError());
-    while (key_bits < 31 && (1LL << key_bits) < (int64_t)n) key_bits++;
-    CK(cudaMalloc(&tmp2, sizeof(int) * (size_t)std::max<int64_t>(md, 1)));
-    k_sort_large<RT><<<152 * 2, LARGE_THREADS, 0, st>>>(row, large, lcnt, tmp, tmp2, key_bits, dedup, ucnt);
-    CK(cudaGetLastError());
+    CK(sorter.sort(row, n, tmp, dedup, ucnt, st));
 
     if (dedup) {
         RT h_m2 = 0;
@@ -1217,13 +1469,11 @@ int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_
         CK(scan_rows(ucnt, row2, n, ss, st));
         CK(cudaMemcpyAsync(&h_m2, row2 + n, sizeof(RT), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        cudaFree(tmp2);  // the sorts are done; room for the compacted columns
-        tmp2 = nullptr;
+        sorter.drop_tmp2();
         CK(cudaMalloc(&col, sizeof(int) * (size_t)std::max<int64_t>((int64_t)h_m2, 1)));
         k_compact<RT><<<grid_for((int64_t)n * 32, thr), thr, 0, st>>>(row, row2, n, tmp, col);
         CK(cudaGetLastError());
-        k_compact_long<RT><<<152 * 2, 1024, 0, st>>>(row, row2, large, lcnt, tmp, col);
-        CK(cudaGetLastError());
+        CK(sorter.compact(row, row2, tmp, col, st));
         CK(cudaStreamSynchronize(st));
         cudaFree(row);
         row = row2;
@@ -1245,12 +1495,7 @@ done:
     if (cursor) cudaFree(cursor);
     if (col) cudaFree(col);
     if (tmp) cudaFree(tmp);
-    if (tmp2) cudaFree(tmp2);
     if (ucnt) cudaFree(ucnt);
-    if (med) cudaFree(med);
-    if (large) cudaFree(large);
-    if (w4) cudaFree(w4);
-    if (w16) cudaFree(w16);
     return rc;
 }
 
@@ -1261,7 +1506,6 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
 {
     int rc = GBFS_OK;
     int *deg = nullptr;
-    unsigned *lcnt = nullptr;
     int *status = nullptr;
     unsigned long long *total = nullptr;
     void *scan_mem = nullptr;
@@ -1281,7 +1525,6 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
     CK(cudaMalloc(&deg, sizeof(int) * ((size_t)n + 1)));
     CK(cudaMalloc(&status, 64));
     total = (unsigned long long *)(status + 2);
-    lcnt = (unsigned *)(status + 4);
     CK(cudaMemsetAsync(deg, 0, sizeof(int) * ((size_t)n + 1), st));
     CK(cudaMemsetAsync(status, 0, 64, st));
     if (m > 0) {
@@ -1303,11 +1546,11 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
     }
     out.wide = (flags & GBFS_WIDE_ROWS) || h_total > (unsigned long long)INT32_MAX;
     if (out.wide)
-        rc = build_rows<long long>(n, m, (int64_t)h_total, d_src, d_dst, flags, deg, ss, lcnt, st, out.row64,
-                                   out.col, out.m, err);
+        rc = build_rows<long long>(n, m, (int64_t)h_total, d_src, d_dst, flags, deg, ss, st, out.row64, out.col,
+                                   out.m, err);
     else
-        rc = build_rows<int>(n, m, (int64_t)h_total, d_src, d_dst, flags, deg, ss, lcnt, st, out.row, out.col,
-                             out.m, err);
+        rc = build_rows<int>(n, m, (int64_t)h_total, d_src, d_dst, flags, deg, ss, st, out.row, out.col, out.m,
+                             err);
     if (rc) goto done;
     out.sorted_rows = true;
     {
