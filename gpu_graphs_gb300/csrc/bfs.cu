@@ -1359,6 +1359,10 @@ cudaError_t bfs_enqueue(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, co
                         int max_steps, int max_ctas)
 {
     BfsArgs a = make_args(g, p, w, d_roots, k, single_root, d_level, slot, symmetric, resume, max_steps);
+    if (!resume && !max_steps && !max_ctas && bfs_small(g, p)) {
+        const cudaError_t es = bfs_small_launch(a, st);
+        if (es != cudaErrorInvalidConfiguration) return es;  // no room for such a cluster on this device
+    }
     if (resume || max_steps || !bfs_relax_tail(g, p))
         return bfs_launch_any(a, p.threads_per_block, p.blocks_per_sm, st, max_ctas);
     // a graph of small degree: a search still running at level

@@ -151,6 +151,8 @@ int bfs_run(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const int *d_r
 // label-correcting kernel, and the kernel launches one search enqueues
 // (2 then, else 1).
 bool bfs_relax_tail(const DeviceCsr &g, const gbfs_params &p);
+// Whether such a search runs on one cluster (bfs_small.cu).
+bool bfs_small(const DeviceCsr &g, const gbfs_params &p);
 // Whether that kernel runs on the graph's fixed-width adjacency
 // (csr_build_quads) when it has been built.
 bool bfs_wants_quads(const DeviceCsr &g, const gbfs_params &p);

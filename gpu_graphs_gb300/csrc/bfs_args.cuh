@@ -76,4 +76,7 @@ using BndT = typename RowSel<RT>::B;
 // with may_yield set: it finishes a search the grid launch parked.
 cudaError_t bfs_relax_launch(const BfsArgs &args, cudaStream_t st, int max_ctas);
 
+// The one-cluster search of a small graph (bfs_small.cu).
+cudaError_t bfs_small_launch(const BfsArgs &args, cudaStream_t st);
+
 }  // namespace gbfs
