@@ -35,6 +35,13 @@ struct gbfs_graphset {
     gbfs_graph *g = nullptr;           // the disjoint union
     std::vector<int64_t> offsets;      // count+1 vertex offsets
     std::vector<int32_t> sizes;        // n of each member
+    // per member, where its levels go and start in the union (batch.cu); on
+    // the device, allocated by the first call with device outputs
+    struct Slice {
+        int32_t *dst;
+        long long offset;
+    };
+    Slice *d_slices = nullptr;
 };
 
 namespace gbfs {
