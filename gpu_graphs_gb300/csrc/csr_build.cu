@@ -35,6 +35,10 @@ constexpr int SB_E = 8;           // values per thread of a CTA sort
 constexpr int MED_MAX = 4096;     // rows up to this length: CTA sort; longer ones in chunks of it
 constexpr int MED_THREADS = MED_MAX / SB_E;
 constexpr int BIN_THREADS = 1024;
+// CTAs of the passes over the edge list: more than fit at once, so that what
+// neighbouring CTAs write stays close together (RMAT-22 build 10.2 ms with 16
+// per SM, 9.7 with 64)
+constexpr int EDGE_CTAS = 152 * 64;
 // row classes of k_bin: warp sorts, CTA sorts of 1024, 2048 and 4096, long rows
 enum BinClass : int { BIN_W4, BIN_W16, BIN_1K, BIN_2K, BIN_4K, BIN_LONG, BIN_CLASSES };
 
@@ -55,10 +59,14 @@ __device__ __forceinline__ long long atomic_add_t(long long *p, long long v)
 }
 
 // All 32 lanes call; key < 0 means "no increment".  Returns the old value of
-// arr[key] plus this lane's rank among lanes with the same key.
+// arr[key] plus this lane's rank among lanes with the same key.  Lanes are
+// grouped by key (one atomic per group) only where two lanes beside each other
+// have the same one: random keys hardly ever do, a row that many lanes hit does.
 template <typename T>
 __device__ __forceinline__ T agg_atomic_add(T *arr, int key)
 {
+    const int beside = __shfl_xor_sync(FULL, key, 1);
+    if (!__any_sync(FULL, key >= 0 && key == beside)) return key >= 0 ? atomic_add_t(&arr[key], (T)1) : (T)0;
     unsigned peers = __match_any_sync(FULL, key);
     int leader = __ffs(peers) - 1;
     T old = 0;
@@ -244,9 +252,27 @@ __device__ __forceinline__ int warp_bitonic_sort(int x)
     return x;
 }
 
-// Rows of length <= 32, one warp per row: sort in registers, pack distinct
-// values.  A warp loads the offsets of 32 consecutive rows at once, then
-// sorts those of them that are short, one after another.
+// Sorts 8 values ascending (Batcher's odd-even merge network, 19 exchanges).
+__device__ __forceinline__ void sort8(int (&v)[8])
+{
+    auto cx = [&](int a, int b) {
+        const int lo = min(v[a], v[b]), hi = max(v[a], v[b]);
+        v[a] = lo;
+        v[b] = hi;
+    };
+    cx(0, 1); cx(2, 3); cx(4, 5); cx(6, 7);
+    cx(0, 2); cx(1, 3); cx(4, 6); cx(5, 7);
+    cx(1, 2); cx(5, 6);
+    cx(0, 4); cx(1, 5); cx(2, 6); cx(3, 7);
+    cx(2, 4); cx(3, 5);
+    cx(1, 2); cx(3, 4); cx(5, 6);
+}
+
+// Rows of length <= 32: sort in registers, pack distinct values.  A warp loads
+// the offsets of 32 consecutive rows at once.  Rows of up to 8 entries are
+// sorted by a lane each, all 32 at once (a grid of 16 M vertices: 1.93 ms with
+// a warp per row, 0.13 ms so), rows of up to 16 by half a warp, two at a time,
+// the others by the warp, one after another.
 template <typename RT>
 __global__ void k_sort_small(const RT *__restrict__ row, int n, int *tmp, int dedup, int *ucnt)
 {
@@ -259,27 +285,57 @@ __global__ void k_sort_small(const RT *__restrict__ row, int n, int *tmp, int de
             bl = row[r0 + lane];
             dl = (int)(row[r0 + lane + 1] - bl);
         }
-        for (int j = 0; j < 32; j++) {
-            const int64_t r = r0 + j;
+        if (dl <= 8) {
+            int v[8], k = 0;
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = e < dl ? tmp[bl + e] : INT_MAX;
+            sort8(v);
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                if (e < dl && (!dedup || e == 0 || v[e] != v[e - 1])) tmp[bl + k++] = v[e];
+            ucnt[r0 + lane] = k;
+        }
+        __syncwarp();
+        // half a warp per row: the first two rows left, and so on
+        unsigned left = __ballot_sync(FULL, dl > 8 && dl <= 16);
+        while (left) {
+            const int j0 = __ffs(left) - 1;
+            left &= left - 1u;
+            const int j1 = left ? __ffs(left) - 1 : j0;
+            const bool two = left != 0;
+            if (two) left &= left - 1u;
+            const unsigned h = lane & 15u;
+            const int j = lane < 16 ? j0 : j1;
             const RT b = __shfl_sync(FULL, bl, j);
             const int d = __shfl_sync(FULL, dl, j);
-            if (d > 32) continue;
-            if (d <= 1) {
-                if (lane == 0) ucnt[r] = d;
-                continue;
-            }
+            const bool on = lane < 16 || two;
+            int x = on && (int)h < d ? tmp[b + h] : INT_MAX;
+#pragma unroll
+            for (int k = 2; k <= 16; k <<= 1)
+#pragma unroll
+                for (int i = k >> 1; i > 0; i >>= 1) {
+                    const int y = __shfl_xor_sync(FULL, x, i);
+                    x = ((h & i) == 0) == ((h & k) == 0) ? min(x, y) : max(x, y);
+                }
+            const int prev = __shfl_up_sync(FULL, x, 1);
+            const bool keep = on && (int)h < d && (!dedup || h == 0 || x != prev);
+            const unsigned mask = __ballot_sync(FULL, keep) >> (lane & 16u) & 0xffffu;
+            if (keep) tmp[b + __popc(mask & ((1u << h) - 1u))] = x;
+            if (on && h == 0) ucnt[r0 + j] = __popc(mask);
+        }
+        left = __ballot_sync(FULL, dl > 16 && dl <= 32);
+        while (left) {
+            const int j = __ffs(left) - 1;
+            left &= left - 1u;
+            const RT b = __shfl_sync(FULL, bl, j);
+            const int d = __shfl_sync(FULL, dl, j);
             int x = (int)lane < d ? tmp[b + lane] : INT_MAX;
             x = warp_bitonic_sort(x);
-            if (dedup) {
-                int prev = __shfl_up_sync(FULL, x, 1);
-                bool uniq = (int)lane < d && (lane == 0 || x != prev);
-                unsigned mask = __ballot_sync(FULL, uniq);
-                if (uniq) tmp[b + __popc(mask & lanemask_lt())] = x;
-                if (lane == 0) ucnt[r] = __popc(mask);
-            } else {
-                if ((int)lane < d) tmp[b + lane] = x;
-                if (lane == 0) ucnt[r] = d;
-            }
+            const int prev = __shfl_up_sync(FULL, x, 1);
+            const bool keep = (int)lane < d && (!dedup || lane == 0 || x != prev);
+            const unsigned mask = __ballot_sync(FULL, keep);
+            if (keep) tmp[b + __popc(mask & lanemask_lt())] = x;
+            if (lane == 0) ucnt[r0 + j] = __popc(mask);
         }
     }
 }
@@ -655,9 +711,11 @@ k_compact_chunks(const RT *__restrict__ row, const RT *__restrict__ row2, const 
     }
 }
 
-// Copy the packed distinct prefix of each row.  A warp loads the offsets
-// of 32 consecutive rows at once (one coalesced load per array instead of
-// a dependent pair per row), then copies the 32 rows one after another.
+// Copy the packed distinct prefix of each row.  A warp loads the offsets of 32
+// consecutive rows at once; rows of up to 64 entries are copied as one
+// concatenated range (a lane finds its entry's row with shuffles), longer ones
+// one after another (all rows one after another: 0.50 ms for a grid of 16 M
+// vertices, 0.17 so).
 template <typename RT>
 __global__ void k_compact(const RT *__restrict__ row, const RT *__restrict__ row2, int n,
                           const int *__restrict__ tmp, int *col)
@@ -674,10 +732,35 @@ __global__ void k_compact(const RT *__restrict__ row, const RT *__restrict__ row
             o = row2[r];
             c = (int)(row2[r + 1] - o);
         }
-#pragma unroll 4
-        for (int j = 0; j < 32; j++) {
+        const int cs = c <= 64 ? c : 0;
+        const int incl = warp_incl_scan(cs), excl = incl - cs;
+        const int T = __shfl_sync(FULL, incl, 31);
+        for (int e0 = 0; e0 < T; e0 += 64) {
+            int x[2];
+            RT at[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int e = e0 + q * 32 + lane, ee = min(e, T - 1);
+                int j = 0;  // the last row that starts at or before entry ee
+#pragma unroll
+                for (int s = 16; s > 0; s >>= 1)
+                    if (__shfl_sync(FULL, excl, j + s) <= ee) j += s;
+                const int k = ee - __shfl_sync(FULL, excl, j);
+                const RT from = __shfl_sync(FULL, b, j) + k;
+                at[q] = __shfl_sync(FULL, o, j) + k;
+                x[q] = e < T ? tmp[from] : 0;
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+                if (e0 + q * 32 + lane < T) col[at[q]] = x[q];
+        }
+        unsigned left = __ballot_sync(FULL, c > 64);
+        while (left) {
+            const int j = __ffs(left) - 1;
+            left &= left - 1u;
             const RT bj = __shfl_sync(FULL, b, j), oj = __shfl_sync(FULL, o, j);
             const int cj = __shfl_sync(FULL, c, j);
+#pragma unroll 4
             for (int i = lane; i < cj; i += 32) col[oj + i] = tmp[bj + i];
         }
     }
@@ -1452,7 +1535,7 @@ int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_
     CK(cudaMemcpyAsync(cursor, row, sizeof(RT) * ((size_t)n + 1), cudaMemcpyDeviceToDevice, st));
     CK(cudaMalloc(&tmp, sizeof(int) * (size_t)std::max<int64_t>(md, 1)));
     if (m > 0) {
-        k_scatter<RT><<<grid_for(m, thr), thr, 0, st>>>(d_src, d_dst, m, n, flags, cursor, tmp);
+        k_scatter<RT><<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, cursor, tmp);
         CK(cudaGetLastError());
     }
     CK(cudaMalloc(&ucnt, sizeof(int) * ((size_t)n + 1)));
@@ -1528,7 +1611,7 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
     CK(cudaMemsetAsync(deg, 0, sizeof(int) * ((size_t)n + 1), st));
     CK(cudaMemsetAsync(status, 0, 64, st));
     if (m > 0) {
-        k_count<<<grid_for(m, thr), thr, 0, st>>>(d_src, d_dst, m, n, flags, deg, total, status);
+        k_count<<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, deg, total, status);
         CK(cudaGetLastError());
     }
     CK(cudaMemcpyAsync(&h_total, total, 8, cudaMemcpyDeviceToHost, st));

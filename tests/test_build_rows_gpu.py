@@ -7,7 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-LENGTHS = (1, 31, 32, 33, 128, 129, 512, 513, 1024, 1025, 2048, 2049, 4095, 4096, 4097, 8191, 8192, 8193, 12_289,
+LENGTHS = (1, 2, 7, 8, 9, 10, 15, 16, 17, 31, 32, 33, 8, 16, 12, 63, 64, 65, 128, 129, 512, 513, 1024, 1025, 2048, 2049, 4095, 4096, 4097, 8191, 8192, 8193, 12_289,
            16_384, 16_385, 40_000, 70_001)
 
 
