@@ -835,40 +835,77 @@ __global__ void k_validate_csr(const RT *__restrict__ row, const int *__restrict
     }
 }
 
-// Symmetry check on sorted rows: every (u,v) has (v,u).
-template <typename RT>
-__global__ void k_check_sym(const RT *__restrict__ row, const int *__restrict__ col, int n, int *flags)
+// Calls f(e, u, in) for the m entries e of the rows, u the entry's row: a warp
+// takes EDGE_CHUNK consecutive entries at a time, 32 a step (in: the lane has
+// one), so the work does not follow the rows' lengths.  All lanes call f.
+constexpr int EDGE_CHUNK = 1024;
+
+template <typename RT, typename F>
+__device__ __forceinline__ void for_edges(const RT *__restrict__ row, int n, int64_t m, F f)
 {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += stride) {
-        const RT b = row[u], e = row[u + 1];
-        for (RT i = b; i < e; i++) {
-            const int v = col[i];
-            RT lo = row[v], hi = row[v + 1];
-            while (lo < hi) {
-                const RT mid = (lo + hi) >> 1;
-                if (col[mid] < (int)u) lo = mid + 1; else hi = mid;
+    const int lane = (int)lane_id();
+    const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t base = gw * EDGE_CHUNK; base < m; base += nw * EDGE_CHUNK) {
+        int u = 0, hi = n;  // row[u] <= base < row[hi]
+        while (hi - u > 1) {
+            const int mid = u + (hi - u) / 2;
+            if ((int64_t)row[mid] <= base) u = mid; else hi = mid;
+        }
+        const int64_t end = min(m, base + EDGE_CHUNK);
+        for (int64_t e0 = base; e0 < end; e0 += 32) {
+            const int64_t e = e0 + lane;
+            const bool in = e < end;
+            int mine = -1;
+            for (int w = u;; w += 32) {  // 32 rows' ends at a time
+                const int64_t at = (int64_t)w + 1 + lane, r = at <= n ? (int64_t)row[at] : INT64_MAX;
+                int k = 0;  // of them at or before e
+#pragma unroll
+                for (int s = 16; s > 0; s >>= 1)
+                    if (__shfl_sync(FULL, r, k + s - 1) <= e) k += s;
+                if (__shfl_sync(FULL, r, k) <= e) ++k;
+                if (mine < 0 && k < 32) mine = w + k;
+                if (!__any_sync(FULL, in && mine < 0)) break;
             }
-            if (lo >= row[v + 1] || col[lo] != (int)u) {
-                flags[1] = 1;
-                break;
-            }
+            f(e, mine, in);
+            u = __shfl_sync(FULL, mine, (int)(min(end, e0 + 32) - e0) - 1);
         }
     }
 }
 
+// Symmetry check on sorted rows: every (u,v) has (v,u).
 template <typename RT>
-__global__ void k_check_sorted(const RT *__restrict__ row, const int *__restrict__ col, int n, int *flags)
+__global__ void k_check_sym(const RT *__restrict__ row, const int *__restrict__ col, int n, int64_t m, int *flags)
 {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += stride) {
-        const RT b = row[u], e = row[u + 1];
-        for (RT i = b + 1; i < e; i++)
-            if (col[i - 1] > col[i]) {
-                flags[0] = 1;
-                break;
-            }
+    for_edges(row, n, m, [&](int64_t e, int u, bool in) {
+        if (!in || ld_relaxed_i32(flags + 1)) return;
+        const int v = col[e];
+        const RT last = row[v + 1];
+        RT lo = row[v], hi = last;
+        while (lo < hi) {
+            const RT mid = (lo + hi) >> 1;
+            if (col[mid] < u) lo = mid + 1; else hi = mid;
+        }
+        if (lo >= last || col[lo] != u) flags[1] = 1;
+    });
+}
+
+// Rows ascend where every descent of the column array is at a row's start:
+// descents counted over all entries, less those at the rows' first ones.
+template <typename RT>
+__global__ void k_check_sorted(const RT *__restrict__ row, const int *__restrict__ col, int n, int64_t m,
+                               unsigned long long *descents)
+{
+    __shared__ unsigned long long s_red[32];
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long mine = 0;
+    for (int64_t i = t + 1; i < m; i += stride) mine += col[i - 1] > col[i];
+    for (int64_t u = t; u < n; u += stride) {
+        const int64_t b = (int64_t)row[u];
+        if (b > 0 && (int64_t)row[u + 1] > b) mine -= col[b - 1] > col[b];
     }
+    const unsigned long long d = block_sum(mine, s_red);
+    if (threadIdx.x == 0 && d) atomicAdd(descents, d);
 }
 
 // Hub-first order: each row's highest-degree neighbour (lowest id among
@@ -1240,19 +1277,24 @@ done:
 int csr_check_symmetric(DeviceCsr &c, cudaStream_t st, bool &sym, std::string &err)
 {
     int rc = GBFS_OK;
+    unsigned long long *descents = nullptr, h_descents = 0;
     int *flags = nullptr, *copy = nullptr;
     int h[2] = {0, 0};
-    const int grid = grid_for(c.n, 256, 152 * 8);
-    CK(cudaMalloc(&flags, 8));
-    CK(cudaMemsetAsync(flags, 0, 8, st));
-    if (c.wide) k_check_sorted<<<grid, 256, 0, st>>>((const long long *)c.row64, c.col, c.n, flags);
-    else k_check_sorted<<<grid, 256, 0, st>>>((const int *)c.row, c.col, c.n, flags);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(h, flags, 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    const int grid = grid_for(std::max<int64_t>(c.n, c.m), 256, 152 * 8);
+    CK(cudaMalloc(&descents, 16));
+    flags = (int *)(descents + 1);
+    CK(cudaMemsetAsync(descents, 0, 16, st));
+    if (!c.sorted_rows) {
+        if (c.wide) k_check_sorted<<<grid, 256, 0, st>>>((const long long *)c.row64, c.col, c.n, c.m, descents);
+        else k_check_sorted<<<grid, 256, 0, st>>>((const int *)c.row, c.col, c.n, c.m, descents);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(&h_descents, descents, 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        c.sorted_rows = h_descents == 0;
+    }
     {
         const int *col = c.col;
-        if (h[0]) {  // unsorted rows (hub-first ones, for instance): check a sorted copy
+        if (!c.sorted_rows) {  // hub-first rows, for instance: check a sorted copy
             CK(cudaMalloc(&copy, sizeof(int) * (size_t)std::max<int64_t>(c.m, 1)));
             CK(cudaMemcpyAsync(copy, c.col, sizeof(int) * (size_t)c.m, cudaMemcpyDeviceToDevice, st));
             rc = c.wide ? sort_rows_inplace((const long long *)c.row64, copy, c.n, c.m, st, err)
@@ -1260,16 +1302,15 @@ int csr_check_symmetric(DeviceCsr &c, cudaStream_t st, bool &sym, std::string &e
             if (rc) goto done;
             col = copy;
         }
-        if (c.wide) k_check_sym<<<grid, 256, 0, st>>>((const long long *)c.row64, col, c.n, flags);
-        else k_check_sym<<<grid, 256, 0, st>>>((const int *)c.row, col, c.n, flags);
+        if (c.wide) k_check_sym<<<grid, 256, 0, st>>>((const long long *)c.row64, col, c.n, c.m, flags);
+        else k_check_sym<<<grid, 256, 0, st>>>((const int *)c.row, col, c.n, c.m, flags);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(h, flags, 8, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         sym = h[1] == 0;
-        c.sorted_rows = h[0] == 0;
     }
 done:
-    if (flags) cudaFree(flags);
+    if (descents) cudaFree(descents);
     if (copy) cudaFree(copy);
     return rc;
 }
@@ -1307,12 +1348,14 @@ __global__ void k_first(const RT *__restrict__ row, const int *__restrict__ col,
     }
 }
 
-// One warp per row u: every out-edge u -> v lands in v's in-row.
-__global__ void k_in_scatter(const int *__restrict__ row, const int *__restrict__ col, int n, int *cursor, int *tcol)
+// Every out-edge u -> v lands in v's in-row (a warp per row took 610 us where
+// one hub of 40 K edges sat among 4.8 M).
+__global__ void k_in_scatter(const int *__restrict__ row, const int *__restrict__ col, int n, int64_t m, int *cursor,
+                             int *tcol)
 {
-    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps)
-        for (int i = row[u] + (int)lane_id(); i < row[u + 1]; i += 32) tcol[atomicAdd(&cursor[col[i]], 1)] = (int)u;
+    for_edges(row, n, m, [&](int64_t e, int u, bool in) {
+        if (in) tcol[atomicAdd(&cursor[col[e]], 1)] = u;
+    });
 }
 
 }  // namespace
@@ -1351,7 +1394,7 @@ int csr_build_transpose(DeviceCsr &c, cudaStream_t st, std::string &err)
     CK(scan_exclusive_i32_i32(indeg, trow, n, trow + n, ss, st));
     CK(cudaMemcpyAsync(cursor, trow, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToDevice, st));
     if (m > 0) {
-        k_in_scatter<<<grid_for((int64_t)n * 32, 256), 256, 0, st>>>(c.row, c.col, n, cursor, tcol);
+        k_in_scatter<<<grid_for(m, 256), 256, 0, st>>>(c.row, c.col, n, m, cursor, tcol);
         CK(cudaGetLastError());
     }
     k_heavy_list<<<grid_for(n, 1024, 152 * 4), 1024, 0, st>>>((const int *)trow, n, theavy, d_nheavy);
