@@ -36,6 +36,8 @@ constexpr int MS_BLOCK = 512;
 constexpr int MS_SEG = 2048;                 // queue entries per edge-balanced pass
 constexpr int MS_PER = MS_SEG / MS_BLOCK;    // entries per thread in the prefix
 constexpr int MS_BIG = 256;                  // push rows this long go to a grid-wide pass
+constexpr int MS_SUB = 4;                    // parts of a huge row's piece, each a warp's
+constexpr int MS_LIGHT_ILP = 2;              // entries per lane in flight in the light rows of a pull step
 
 struct MsArgs {
     int n, n_active, k;
@@ -96,17 +98,29 @@ __device__ __forceinline__ unsigned long long warp_or64(unsigned long long x)
     return x;
 }
 
-// Warp-wide level writes for 32 consecutive vertices u = base + lane: the loop
-// runs over the union of the lanes' masks, so each store instruction covers
-// one byte row and coalesces.  All 32 threads call it.
+// Warp-wide level writes for 32 consecutive vertices u = base + lane, lane by
+// lane of the search, so each store instruction covers one byte row and
+// coalesces; groups of 16 search lanes that no vertex has are skipped.  All 32
+// threads call it.
 __device__ __forceinline__ void write_levels_warp(unsigned char *lv8, int *out, int n, long long u,
                                                   unsigned long long bits, int nl)
 {
-    unsigned long long any = warp_or64(bits);
-    while (any) {
-        const int j = __ffsll((long long)any) - 1;
-        if ((bits >> j) & 1ull) record_level(lv8, out, n, u, j, nl);
-        any &= any - 1ull;
+    const unsigned long long any = warp_or64(bits);
+    if (nl >= LV8_DEEP) {
+        for (unsigned long long m = any; m; m &= m - 1ull) {
+            const int j = __ffsll((long long)m) - 1;
+            if ((bits >> j) & 1ull) record_level(lv8, out, n, u, j, nl);
+        }
+        return;
+    }
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+        if (!(any >> (16 * g) & 0xffffull)) continue;
+        const unsigned mine = (unsigned)(bits >> (16 * g)) & 0xffffu;
+        unsigned char *p = lv8 + (size_t)(16 * g) * n + u;
+#pragma unroll
+        for (int j = 0; j < 16; j++, p += n)
+            if (mine >> j & 1u) *p = (unsigned char)nl;
     }
 }
 
@@ -149,7 +163,7 @@ __device__ __forceinline__ void push_rows(const MsArgs &a, const int *list, long
                 const int v = __ldcg(list + seg + j);
                 const int b = __ldg(a.row + v);
                 s_beg[j] = b;
-                s_f[j] = __ldcg(Fc + v);
+                s_f[j] = Fc[v];
                 d[t] = __ldg(a.row + v + 1) - b;
                 if (defer && d[t] >= MS_BIG) {
                     a.bigl[atomicAdd(bigcnt, 1ull)] = v;
@@ -340,43 +354,86 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) k_msbfs(MsArgs a)
 
         if (pull) {
             ++pull_levels;
-            // light rows: one thread per vertex
+            // light rows, 32 vertices of a warp at a time: a lane reads its
+            // row's first four entries itself; what is left of the rows not yet
+            // covered is read as one concatenated range, its masks ORed into the
+            // rows' words in shared memory (s_f, free in pull steps).  One lane
+            // walking each row to its end took the time of the warp's longest:
+            // RMAT-20, 64 lanes: 223 of 617 us in the light rows, 120 so.  (The
+            // masks Fc were written in the level before alone: plain loads, which
+            // L1 may hold.)
+            unsigned long long *const s_acc = s_f + (threadIdx.x >> 5) * 64, *const s_need = s_acc + 32;
             for (long long base = gwarp * 32; base < n; base += nwarps * 32) {
                 const long long u = base + lane;
-                unsigned long long nw = 0;
+                int b = 0, e = 0;
+                unsigned long long vu = ~0ull;
                 if (u < n) {
-                    const int b = __ldg(a.prow + u), e = __ldg(a.prow + u + 1);
-                    if (e > b && e - b <= HEAVY_DEGREE) {
-                        const unsigned long long vu = __ldcg(a.vis + u);
-                        const unsigned long long need = ~vu & live;
-                        if (need) {
-                            unsigned long long acc = 0;
-                            for (int i = b; i < e; i += 4) {
-                                const int v0 = __ldg(a.pcol + i);
-                                const int v1 = i + 1 < e ? __ldg(a.pcol + i + 1) : v0;
-                                const int v2 = i + 2 < e ? __ldg(a.pcol + i + 2) : v0;
-                                const int v3 = i + 3 < e ? __ldg(a.pcol + i + 3) : v0;
-                                acc |= __ldcg(Fc + v0) | __ldcg(Fc + v1) | __ldcg(Fc + v2) | __ldcg(Fc + v3);
-                                if ((acc & need) == need) break;
-                            }
-                            nw = acc & need;
-                            if (nw) {
-                                a.vis[u] = vu | nw;
-                                Fn[u] = nw;
-                                my_or |= nw;
-                            }
-                        }
-                    }
+                    b = __ldg(a.prow + u);
+                    e = __ldg(a.prow + u + 1);
+                    vu = __ldcg(a.vis + u);
                 }
-                // level writes: one store per discovered lane, coalesced over the
-                // warp's 32 consecutive vertices
+                const unsigned long long need = e > b && e - b <= HEAVY_DEGREE ? ~vu & live : 0ull;
+                if (!__any_sync(FULL, need != 0)) continue;
+                unsigned long long acc = 0;
+                if (need) {
+                    const int v0 = __ldg(a.pcol + b);
+                    const int v1 = b + 1 < e ? __ldg(a.pcol + b + 1) : v0;
+                    const int v2 = b + 2 < e ? __ldg(a.pcol + b + 2) : v0;
+                    const int v3 = b + 3 < e ? __ldg(a.pcol + b + 3) : v0;
+                    acc = Fc[v0] | Fc[v1] | Fc[v2] | Fc[v3];
+                }
+                b += 4;
+                const int rest = (acc & need) != need && b < e ? e - b : 0;
+                const int incl = warp_incl_scan(rest), excl = incl - rest;
+                const int T = __shfl_sync(FULL, incl, 31);
+                if (T) {
+                    s_acc[lane] = acc;
+                    s_need[lane] = need;
+                    __syncwarp();
+                    for (int e0 = 0; e0 < T; e0 += 32 * MS_LIGHT_ILP) {
+                        int v[MS_LIGHT_ILP], r[MS_LIGHT_ILP];
+#pragma unroll
+                        for (int q = 0; q < MS_LIGHT_ILP; q++) {
+                            const int i = min(e0 + q * 32 + (int)lane, T - 1);
+                            int j = 0;  // the last row that starts at or before entry i
+#pragma unroll
+                            for (int st = 16; st > 0; st >>= 1)
+                                if (__shfl_sync(FULL, excl, j + st) <= i) j += st;
+                            const int at = __shfl_sync(FULL, b - excl, j) + i;
+                            r[q] = j;
+                            v[q] = (s_acc[j] & s_need[j]) != s_need[j] ? __ldg(a.pcol + at) : -1;
+                        }
+                        unsigned long long f[MS_LIGHT_ILP];
+#pragma unroll
+                        for (int q = 0; q < MS_LIGHT_ILP; q++) f[q] = v[q] >= 0 ? Fc[v[q]] : 0ull;
+#pragma unroll
+                        for (int q = 0; q < MS_LIGHT_ILP; q++) {
+                            f[q] &= s_need[r[q]] & ~s_acc[r[q]];
+                            unsigned *w = reinterpret_cast<unsigned *>(s_acc + r[q]);
+                            if ((unsigned)f[q]) atomicOr(w, (unsigned)f[q]);
+                            if (f[q] >> 32) atomicOr(w + 1, (unsigned)(f[q] >> 32));
+                        }
+                        __syncwarp();
+                    }
+                    acc = s_acc[lane];
+                    __syncwarp();
+                }
+                const unsigned long long nw = acc & need;
+                if (nw) {
+                    a.vis[u] = vu | nw;
+                    Fn[u] = nw;
+                    my_or |= nw;
+                }
+                // level writes: coalesced over the warp's 32 consecutive vertices
                 write_levels_warp(a.lv8, a.out, n, u, nw, nl);
                 wq_push(q, nw != 0, (int)u, qcnt_next, Qn);
             }
             // heavy rows up to MS_HUGE edges: a warp screens 32 of them at once
             // (one lane each, strided by the warp count so busy rows spread
-            // evenly over warps) and walks those with lanes to find, one by one
-            for (long long h0 = gwarp; h0 < a.nheavy; h0 += nwarps * 32) {
+            // evenly over warps) and walks those with lanes to find, one by one.
+            // From the last warp down: the huge rows' parts below go from the
+            // first one up, so what does not divide evenly falls on different ones
+            for (long long h0 = nwarps - 1 - gwarp; h0 < a.nheavy; h0 += nwarps * 32) {
                 const long long h = h0 + (long long)lane * nwarps;
                 int u = 0, b = 0, e = 0;
                 unsigned long long vu = 0, need = 0;
@@ -403,7 +460,7 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) k_msbfs(MsArgs a)
 #pragma unroll
                         for (int t = 0; t < 4; t++) {
                             const int i = i0 + t * 32 + (int)lane;
-                            if (i < re) x |= __ldcg(Fc + __ldg(a.pcol + i));
+                            if (i < re) x |= Fc[__ldg(a.pcol + i)];
                         }
                         acc |= warp_or64(x);
                         if ((acc & rneed) == rneed) break;
@@ -421,19 +478,20 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) k_msbfs(MsArgs a)
                     wq_push(q, lane == 0 && nw != 0, ru, qcnt_next, Qn);
                 }
             }
-            // huge rows: pieces of MS_PIECE edges spread over all warps, so a
-            // hub that must be scanned to its end is not one warp's tail.  Each
-            // piece ORs what it found into hacc[u] and counts itself in
+            // huge rows: quarters of pieces of MS_PIECE edges spread over all
+            // warps, so a hub that must be scanned to its end is not one warp's
+            // tail.  Each part ORs what it found into hacc[u] and counts itself in
             // hcnt[u]; the warp that counts a row's last piece settles the row.
             // vis[u] only changes when the row is settled, after all of its
             // pieces have counted, so every piece sees the same need: a row
             // with nothing to find is skipped by all of its pieces.
-            for (long long c0 = gwarp; c0 < a.npieces; c0 += nwarps * 32) {
+            for (long long c0 = gwarp; c0 < MS_SUB * (long long)a.npieces; c0 += nwarps * 32) {
                 const long long c = c0 + (long long)lane * nwarps;
                 int2 pc = make_int2(0, 0);
                 unsigned long long vu = 0, need = 0;
-                if (c < a.npieces) {
-                    pc = __ldg(a.pieces + c);
+                if (c < MS_SUB * (long long)a.npieces) {
+                    pc = __ldg(a.pieces + c / MS_SUB);
+                    pc.y = MS_SUB * pc.y + (int)(c % MS_SUB);
                     vu = __ldcg(a.vis + pc.x);
                     need = ~vu & live;
                 }
@@ -445,9 +503,9 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) k_msbfs(MsArgs a)
                     const unsigned long long rvu = __shfl_sync(FULL, vu, sl);
                     const unsigned long long rneed = __shfl_sync(FULL, need, sl);
                     const int rb = __ldg(a.prow + u), re = __ldg(a.prow + u + 1);
-                    const unsigned pn = (unsigned)((re - rb + MS_PIECE - 1) / MS_PIECE);
-                    const int b = rb + j * MS_PIECE;
-                    const int e = min(re, b + MS_PIECE);
+                    const unsigned pn = MS_SUB * (unsigned)((re - rb + MS_PIECE - 1) / MS_PIECE);
+                    const int b = rb + j * (MS_PIECE / MS_SUB);
+                    const int e = min(re, b + MS_PIECE / MS_SUB);  // (before b past the row's end: no edges)
                     unsigned long long acc = 0;
                     // skip a piece whose row the others have already covered (one
                     // read, broadcast: the loop below must be warp-uniform)
@@ -459,7 +517,7 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) k_msbfs(MsArgs a)
 #pragma unroll
                             for (int t = 0; t < 4; t++) {
                                 const int i = i0 + t * 32 + (int)lane;
-                                if (i < e) x |= __ldcg(Fc + __ldg(a.pcol + i));
+                                if (i < e) x |= Fc[__ldg(a.pcol + i)];
                             }
                             acc |= warp_or64(x);
                             if ((acc & rneed) == rneed) break;
