@@ -15,6 +15,7 @@
 #include "../../include/gbfs.h"
 #include "graph.cuh"
 #include "parents.cuh"
+#include "pinned.cuh"
 #include "scan.cuh"
 
 namespace gbfs {
@@ -214,7 +215,7 @@ extern "C" int gbfs_graph_from_edges(int32_t n, int64_t m, const int32_t *src, c
     rc = to_device(src, m, st, &d_src, &own_s);
     if (!rc) rc = to_device(dst, m, st, &d_dst, &own_d);
     if (!rc) {
-        rc = csr_build_from_edges(n, m, d_src, d_dst, flags & (7u | GBFS_WIDE_ROWS), st, csr, err);
+        rc = csr_build_from_edges(n, m, d_src, d_dst, flags & (7u | GBFS_WIDE_ROWS | GBFS_HUB_FIRST), st, csr, err);
         if (!rc && (flags & GBFS_HUB_FIRST)) rc = csr_hub_first(csr, st, err);
         if (rc) set_error(err);
     }
@@ -511,7 +512,7 @@ extern "C" int gbfs_bfs_many(gbfs_graph *g, const int32_t *sources, int32_t k, i
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(w.h_outs, w.d_outs, sizeof(BfsOut) * (size_t)k, cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(w.h_ctrl, w.ctrl, offsetof(BfsCtrl, t_entry), cudaMemcpyDeviceToHost, g->stream);
+        e = cudaMemcpyAsync(&w.h_ctrl->status, &w.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     if (e != cudaSuccess) return cuda_fail(e, "BFS launches");
     if (w.h_ctrl->status != DEV_OK) {
@@ -543,23 +544,31 @@ extern "C" int gbfs_last_trace(gbfs_graph *g, gbfs_level_trace *rows, int32_t ca
     int trace_len;
     const LevelTrace *trace;
     cudaError_t e;
+    // the control blocks' parts from t_entry on
+    std::unique_ptr<BfsCtrl> hb;
+    std::unique_ptr<MsCtrl> hm;
     if (g->last_multi) {
         if (!g->ms.ctrl) return 0;
-        MsCtrl *h = g->ms.h_ctrl;
-        e = cudaMemcpyAsync(&h->t_entry, &g->ms.ctrl->t_entry, sizeof(MsCtrl) - offsetof(MsCtrl, t_entry),
-                            cudaMemcpyDeviceToHost, g->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&h->trace_len, &g->ms.ctrl->trace_len, sizeof(int),
-                                                  cudaMemcpyDeviceToHost, g->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+        hm.reset(new (std::nothrow) MsCtrl);
+        MsCtrl *h = hm.get();
+        if (!h) return fail(GBFS_ERR_OOM, "host allocation failed for the trace");
+        e = cudaStreamSynchronize(g->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpy(&h->t_entry, &g->ms.ctrl->t_entry, sizeof(MsCtrl) - offsetof(MsCtrl, t_entry),
+                           cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaMemcpy(&h->trace_len, &g->ms.ctrl->trace_len, sizeof(int), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(e, "trace D2H");
         t_entry = h->t_entry; t_start = h->t_start; t_end = h->t_end; t_exit = h->t_exit;
         trace_len = h->trace_len; trace = h->trace;
     } else {
         if (!g->work.ctrl) return 0;
-        BfsCtrl *h = g->work.h_ctrl;
-        e = cudaMemcpyAsync(&h->t_entry, &g->work.ctrl->t_entry, sizeof(BfsCtrl) - offsetof(BfsCtrl, t_entry),
-                            cudaMemcpyDeviceToHost, g->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+        hb.reset(new (std::nothrow) BfsCtrl);
+        BfsCtrl *h = hb.get();
+        if (!h) return fail(GBFS_ERR_OOM, "host allocation failed for the trace");
+        e = cudaStreamSynchronize(g->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpy(&h->t_entry, &g->work.ctrl->t_entry, sizeof(BfsCtrl) - offsetof(BfsCtrl, t_entry),
+                           cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(e, "trace D2H");
         t_entry = h->t_entry; t_start = h->t_start; t_end = h->t_end; t_exit = h->t_exit;
         trace_len = h->trace_len; trace = h->trace;
@@ -691,6 +700,7 @@ struct ScanPool {
     void *mem = nullptr;
     int64_t tiles = 0;
     ScanScratch s;
+    unsigned *status = nullptr;  // pinned: written by a scan whose wait runs out
     int device = -1;
 };
 ScanPool g_scan_pool[64];
@@ -727,15 +737,15 @@ extern "C" int gbfs_exclusive_scan_i32(const int32_t *d_in, int64_t *d_out, int6
         pool.tiles = want;
         pool.s.epoch = 0;
     }
+    if (!pool.status && !(pool.status = (unsigned *)pinned_slot_take()))
+        return fail(GBFS_ERR_OOM, "pinned memory for the scan's status");
+    pool.s.status = pool.status;
     e = scan_exclusive_i32_i64(d_in, (long long *)d_out, n, nullptr, pool.s, st);
     if (e != cudaSuccess) return cuda_fail(e, "scan launch");
-    unsigned status = 0;
-    e = cudaMemcpyAsync(&status, pool.s.ctl + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "scan");
-    if (status != 0) {
-        unsigned zero = 0;
-        cudaMemcpy(pool.s.ctl + 2, &zero, sizeof(unsigned), cudaMemcpyHostToDevice);
+    if (*pool.status != 0) {
+        *pool.status = 0;
         return fail(GBFS_ERR_TIMEOUT, "scan look-back wait ran out");
     }
     return GBFS_OK;

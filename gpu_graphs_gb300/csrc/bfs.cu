@@ -43,6 +43,7 @@
 #include "bfs.cuh"
 #include "bfs_args.cuh"
 #include "blockq.cuh"
+#include "pinned.cuh"
 
 namespace gbfs {
 
@@ -1115,29 +1116,36 @@ int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide)
 {
     if (w.ctrl && w.n == n && w.wide == wide) return GBFS_OK;
     bfs_work_free(w);
-    const size_t W = ((size_t)n + 31) / 32;
-    const size_t bytes_int = sizeof(int) * (size_t)n;
-    auto al = [&](void **p, size_t b) -> bool {
-        cudaError_t e = cudaMalloc(p, std::max<size_t>(b, 16));
-        if (e != cudaSuccess) {
-            err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
-            return false;
-        }
-        w.bytes += (int64_t)std::max<size_t>(b, 16);
-        return true;
-    };
-    w.bytes = 0;
-    if (!al((void **)&w.level, bytes_int) || !al((void **)&w.visited, W * 4) ||
-        !al((void **)&w.fb0, W * 4) || !al((void **)&w.fb1, W * 4) || !al((void **)&w.fb2, W * 4) ||
-        !al((void **)&w.q0, bytes_int) || !al((void **)&w.q1, bytes_int) ||
-        !al((void **)&w.qb0, (wide ? 4 : 2) * bytes_int) || !al((void **)&w.qb1, (wide ? 4 : 2) * bytes_int) ||
-        !al((void **)&w.big, bytes_int) || !al((void **)&w.roots, bytes_int) ||
-        !al((void **)&w.ctrl, sizeof(BfsCtrl))) {
+    const size_t n4 = sizeof(int) * (size_t)n, w4 = sizeof(unsigned) * (((size_t)n + 31) / 32);
+    const size_t qb = (wide ? sizeof(longlong2) : sizeof(int2)) * (size_t)n;
+    Carve c;
+    const size_t level = c.add(n4), visited = c.add(w4), fb0 = c.add(w4), fb1 = c.add(w4), fb2 = c.add(w4),
+                 q0 = c.add(n4), q1 = c.add(n4), qb0 = c.add(qb), qb1 = c.add(qb), big = c.add(n4), roots = c.add(n4),
+                 ctrl = c.add(sizeof(BfsCtrl));
+    const cudaError_t e = cudaMalloc(&w.block, c.size);
+    if (e != cudaSuccess) {
+        w.block = nullptr;
+        err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
         bfs_work_free(w);
         return GBFS_ERR_OOM;
     }
-    if (cudaMemset(w.ctrl, 0, sizeof(BfsCtrl)) != cudaSuccess ||
-        cudaMallocHost(&w.h_ctrl, sizeof(BfsCtrl)) != cudaSuccess ||
+    char *p = (char *)w.block;
+    w.level = (int *)(p + level);
+    w.visited = (unsigned *)(p + visited);
+    w.fb0 = (unsigned *)(p + fb0);
+    w.fb1 = (unsigned *)(p + fb1);
+    w.fb2 = (unsigned *)(p + fb2);
+    w.q0 = (int *)(p + q0);
+    w.q1 = (int *)(p + q1);
+    w.qb0 = (int2 *)(p + qb0);
+    w.qb1 = (int2 *)(p + qb1);
+    w.big = (int *)(p + big);
+    w.roots = (int *)(p + roots);
+    w.ctrl = (BfsCtrl *)(p + ctrl);
+    w.bytes = (int64_t)c.size;
+    static_assert(offsetof(BfsCtrl, t_entry) <= PINNED_SLOT, "the results fit a pinned slot");
+    w.h_ctrl = (BfsCtrl *)pinned_slot_take();
+    if (!w.h_ctrl || cudaMemset(w.ctrl, 0, sizeof(BfsCtrl)) != cudaSuccess ||
         cudaEventCreate(&w.ev0) != cudaSuccess || cudaEventCreate(&w.ev1) != cudaSuccess) {
         err = "workspace setup failed";
         bfs_work_free(w);
@@ -1150,15 +1158,14 @@ int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide)
 
 void bfs_work_free(BfsWork &w)
 {
-    void *ps[] = {w.level, w.visited, w.fb0, w.fb1, w.fb2, w.q0, w.q1, w.qb0, w.qb1, w.big, w.roots, w.ctrl, w.d_outs};
-    for (void *p : ps)
-        if (p) cudaFree(p);
+    if (w.block) cudaFree(w.block);
+    if (w.d_outs) cudaFree(w.d_outs);
     if (w.h_outs) cudaFreeHost(w.h_outs);
     if (w.evs) {
         for (int i = 0; i < w.evs_cap; i++) cudaEventDestroy(w.evs[i]);
         delete[] w.evs;
     }
-    if (w.h_ctrl) cudaFreeHost(w.h_ctrl);
+    pinned_slot_give(w.h_ctrl);
     if (w.ev0) cudaEventDestroy(w.ev0);
     if (w.ev1) cudaEventDestroy(w.ev1);
     bfs_graph_free(w);
@@ -1396,7 +1403,7 @@ void bfs_graph_free(BfsWork &w)
 cudaError_t bfs_graph_launch(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, int k, int *d_level,
                              cudaStream_t st, bool symmetric)
 {
-    BfsArgs a0 = make_args(g, p, w, w.roots, k, -1, d_level, &w.ctrl->out, symmetric, 0, 1);
+    BfsArgs a0 = make_args(g, p, w, w.roots, k, -1, d_level, &w.h_ctrl->out, symmetric, 0, 1);
     const void *func = nullptr;
     int block = 0, grid = 0;
     size_t smem = 0;
@@ -1484,19 +1491,20 @@ int bfs_run(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const int *d_r
         else e = cudaMemcpyAsync(w.roots, &single_root, sizeof(int), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // single_root lives on this stack frame
     }
+    w.h_ctrl->out.levels = -1;  // overwritten by a search that ends
     if (e == cudaSuccess) e = cudaEventRecord(w.ev0, st);
     int launches = bfs_launches_per_search(g, p);
     if (p.per_level_launch == 2) {
         if (e == cudaSuccess) e = bfs_graph_launch(g, p, w, d_roots ? k : 1, d_level, st, symmetric);
         launches = -1;  // the graph's own launches: levels + 1, filled in below
     } else if (!p.per_level_launch) {
-        if (e == cudaSuccess) e = bfs_enqueue(g, p, w, d_roots, k, single_root, d_level, &w.ctrl->out, st, symmetric);
+        if (e == cudaSuccess) e = bfs_enqueue(g, p, w, d_roots, k, single_root, d_level, &w.h_ctrl->out, st, symmetric);
     } else {
         // The reference's shape: one launch per level, then a device->host
         // read of the loop state before deciding to launch again
         // (1D Partition/src/gpuBFS.cu:66-100).
         for (int resume = 0; e == cudaSuccess; resume = 1, ++launches) {
-            e = bfs_enqueue(g, p, w, d_roots, k, single_root, d_level, &w.ctrl->out, st, symmetric, resume, 1);
+            e = bfs_enqueue(g, p, w, d_roots, k, single_root, d_level, &w.h_ctrl->out, st, symmetric, resume, 1);
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(&w.h_ctrl->rs, &w.ctrl->rs, sizeof(BfsResume), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1507,15 +1515,15 @@ int bfs_run(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const int *d_r
         }
     }
     if (e == cudaSuccess) e = cudaEventRecord(w.ev1, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(w.h_ctrl, w.ctrl, offsetof(BfsCtrl, t_entry), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess && w.h_ctrl->out.levels < 0)
+        e = cudaMemcpy(&w.h_ctrl->status, &w.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) {
         err = std::string("BFS launch: ") + cudaGetErrorString(e);
         return GBFS_ERR_CUDA;
     }
     const BfsCtrl &h = *w.h_ctrl;
-    if (h.status != DEV_OK) {
+    if (h.out.levels < 0) {
         const int status = h.status;
         cudaMemsetAsync(w.ctrl, 0, sizeof(BfsCtrl), st);
         cudaStreamSynchronize(st);

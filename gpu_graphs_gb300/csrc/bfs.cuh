@@ -83,6 +83,7 @@ struct BfsCtrl {
 // Per-graph traversal workspace (allocated on first use, reused).
 struct BfsWork {
     int32_t n = 0;
+    void *block = nullptr;       // the device arrays from here to ctrl
     int *level = nullptr;        // n (used when the caller's buffer is on the host)
     unsigned *visited = nullptr; // W
     unsigned *fb0 = nullptr;     // W frontier bitmaps (three, rotating)
@@ -96,7 +97,8 @@ struct BfsWork {
     int *big = nullptr;          // n deferred rows
     int *roots = nullptr;        // root staging (n)
     BfsCtrl *ctrl = nullptr;
-    BfsCtrl *h_ctrl = nullptr;   // pinned mirror for results
+    BfsCtrl *h_ctrl = nullptr;   // pinned: the part of a control block before t_entry; searches
+                                 // write their results there (h_ctrl->out) themselves
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // back-to-back launches: per-launch result slots and events
     BfsOut *d_outs = nullptr;

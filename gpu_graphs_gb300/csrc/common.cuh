@@ -40,6 +40,18 @@ struct LaunchSetup {
     }
 };
 
+// Lays several arrays out in one device allocation (an allocation and its
+// release cost about 30 us each, whatever their size, up to some ten megabytes).
+struct Carve {
+    size_t size = 0;
+    size_t add(size_t bytes)
+    {
+        const size_t at = size;
+        size += (bytes + 255) & ~size_t(255);
+        return at;
+    }
+};
+
 constexpr unsigned FULL = 0xffffffffu;
 
 // ---- warp helpers ---------------------------------------------------------

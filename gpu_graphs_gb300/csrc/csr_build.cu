@@ -23,6 +23,7 @@
 
 #include "common.cuh"
 #include "csr_build.cuh"
+#include "pinned.cuh"
 #include "scan.cuh"
 
 namespace gbfs {
@@ -41,6 +42,14 @@ constexpr int BIN_THREADS = 1024;
 constexpr int EDGE_CTAS = 152 * 64;
 // row classes of k_bin: warp sorts, CTA sorts of 1024, 2048 and 4096, long rows
 enum BinClass : int { BIN_W4, BIN_W16, BIN_1K, BIN_2K, BIN_4K, BIN_LONG, BIN_CLASSES };
+
+#define NEED_PINNED(slot)                                                        \
+    do {                                                                         \
+        if (!(slot)) {                                                           \
+            err = "pinned memory for results";                                   \
+            return GBFS_ERR_OOM;                                                 \
+        }                                                                        \
+    } while (0)
 
 #define CK(call)                                                                 \
     do {                                                                         \
@@ -1062,33 +1071,50 @@ struct Scratch {
     ~Scratch() { if (p) cudaFree(p); }
 };
 
+// The block of c's vertex-sized arrays; row_bytes: room for row offsets in it,
+// returned in row (0: none).
+cudaError_t alloc_block(DeviceCsr &c, bool second, size_t row_bytes, void **row)
+{
+    const size_t n4 = sizeof(int) * (size_t)std::max(1, c.n);
+    Carve cv;
+    const size_t zmask = cv.add(sizeof(unsigned) * (((size_t)c.n + 31) / 32)), heavy = cv.add(n4), first = cv.add(n4);
+    const size_t sec = second ? cv.add(n4) : 0, rows = row_bytes ? cv.add(row_bytes) : 0;
+    const cudaError_t e = cudaMalloc(&c.block, cv.size);
+    if (e != cudaSuccess) {
+        c.block = nullptr;
+        return e;
+    }
+    char *p = (char *)c.block;
+    c.zmask = (unsigned *)(p + zmask);
+    c.heavy = (int *)(p + heavy);
+    c.first = (int *)(p + first);
+    c.second = second ? (int *)(p + sec) : nullptr;
+    if (row_bytes) *row = p + rows;
+    return cudaSuccess;
+}
+
 template <typename RT>
 int finalize_t(DeviceCsr &out, const RT *row, cudaStream_t st, std::string &err)
 {
     int rc = GBFS_OK;
-    struct Res { unsigned long long nonisolated; int maxdeg; unsigned nheavy, nover4, pad; } h{};
+    struct Res { unsigned long long nonisolated; int maxdeg; unsigned nheavy, nover4, pad; };
+    Pinned<Res> h;
+    NEED_PINNED(h);
     Res *d_res = nullptr;
     const int W = (out.n + 31) / 32;
-    CK(cudaMalloc(&out.zmask, sizeof(unsigned) * (size_t)W));
     CK(cudaMalloc(&d_res, sizeof(Res)));
     CK(cudaMemsetAsync(d_res, 0, sizeof(Res), st));
     k_finalize<<<grid_for((int64_t)W * 32, 256), 256, 0, st>>>(row, out.n, out.zmask, &d_res->maxdeg,
                                                                 &d_res->nonisolated, &d_res->nover4);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(&h, d_res, sizeof(Res), cudaMemcpyDeviceToHost, st));
+    k_heavy_list<<<grid_for(out.n, 1024, 152 * 4), 1024, 0, st>>>(row, out.n, out.heavy, &d_res->nheavy);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(h.p, d_res, sizeof(Res), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    out.max_degree = h.maxdeg;
-    out.nonisolated = (int64_t)h.nonisolated;
-    out.nover4 = (int32_t)h.nover4;
-    {
-        // heavy-row list (sized by a first count pass folded into k_heavy_list's atomic)
-        CK(cudaMalloc(&out.heavy, sizeof(int) * (size_t)std::max<int64_t>(1, out.n)));
-        k_heavy_list<<<grid_for(out.n, 1024, 152 * 4), 1024, 0, st>>>(row, out.n, out.heavy, &d_res->nheavy);
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(&h, d_res, sizeof(Res), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        out.nheavy = (int32_t)h.nheavy;
-    }
+    out.max_degree = h->maxdeg;
+    out.nonisolated = (int64_t)h->nonisolated;
+    out.nover4 = (int32_t)h->nover4;
+    out.nheavy = (int32_t)h->nheavy;
 done:
     if (d_res) cudaFree(d_res);
     return rc;
@@ -1104,19 +1130,17 @@ int finalize(DeviceCsr &out, cudaStream_t st, std::string &err)
 // length class.  The lists and the long rows' scratch are freed with it.
 template <typename RT>
 struct RowSorter {
-    void *mem = nullptr;       // lists and counts
     void *long_mem = nullptr;  // long rows: chunks and their counts
     int *tmp2 = nullptr;       // long rows: the merges' second place
     BinLists lists{};
     BinCounts *d_cnt = nullptr;
-    BinCounts h{};
+    Pinned<BinCounts> h;       // d_cnt's values once st has been synchronised
     Chunk *chunks = nullptr;
     int *ccnt = nullptr;
 
     ~RowSorter()
     {
         drop_tmp2();
-        if (mem) cudaFree(mem);
         if (long_mem) cudaFree(long_mem);
     }
 
@@ -1127,28 +1151,40 @@ struct RowSorter {
         tmp2 = nullptr;
     }
 
-    // Lists by length of n rows of m entries together; enqueued on st.
-    cudaError_t bin(const RT *row, int32_t n, int64_t m, cudaStream_t st)
+    // Bytes of scratch the lists take (bin's mem) for n rows of m entries together.
+    static size_t list_bytes(int32_t n, int64_t m)
+    {
+        int64_t cap[BIN_CLASSES];
+        return 256 + sizeof(int) * (size_t)list_caps(n, m, cap);
+    }
+    static int64_t list_caps(int32_t n, int64_t m, int64_t (&cap)[BIN_CLASSES])
     {
         static const int over[BIN_CLASSES] = {32, W4_MAX, W16_MAX, 1024, 2048, MED_MAX};
-        int64_t cap[BIN_CLASSES], total = 0;
+        int64_t total = 0;
         for (int c = 0; c < BIN_CLASSES; c++) {
             cap[c] = std::min<int64_t>(n, m / (over[c] + 1)) + 1;
             total += cap[c];
         }
-        cudaError_t e = cudaMalloc(&mem, 256 + sizeof(int) * (size_t)total);
-        if (e != cudaSuccess) return e;
+        return total;
+    }
+
+    // Lists by length; enqueued on st.  mem stays in use until the sorts are done.
+    cudaError_t bin(const RT *row, int32_t n, int64_t m, void *mem, cudaStream_t st)
+    {
+        int64_t cap[BIN_CLASSES];
+        list_caps(n, m, cap);
         d_cnt = (BinCounts *)mem;
         int *p = (int *)((char *)mem + 256);
         for (int c = 0; c < BIN_CLASSES; c++) {
             lists.list[c] = p;
             p += cap[c];
         }
+        cudaError_t e = cudaSuccess;
         e = cudaMemsetAsync(mem, 0, 256, st);
         if (e != cudaSuccess) return e;
         k_bin<RT><<<grid_for(n, BIN_THREADS, 152 * 4), BIN_THREADS, 0, st>>>(row, n, lists, d_cnt);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_cnt, sizeof(h), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h.p, d_cnt, sizeof(BinCounts), cudaMemcpyDeviceToHost, st);
         return e;
     }
 
@@ -1160,11 +1196,11 @@ struct RowSorter {
         const unsigned *rows = d_cnt->rows;
         const int thr = 256;
         cudaError_t e = cudaSuccess;
-        const int nch = (int)h.chunks;
+        const int nch = (int)h->chunks;
         if (nch) {
             const size_t cb = sizeof(Chunk) * (size_t)nch;
             e = cudaMalloc(&long_mem, 256 + cb + sizeof(int) * (size_t)nch);
-            if (e == cudaSuccess) e = cudaMalloc(&tmp2, sizeof(int) * (size_t)h.long_entries);
+            if (e == cudaSuccess) e = cudaMalloc(&tmp2, sizeof(int) * (size_t)h->long_entries);
             if (e != cudaSuccess) return e;
             ChunkNext *next = (ChunkNext *)long_mem;
             chunks = (Chunk *)((char *)long_mem + 256);
@@ -1172,27 +1208,27 @@ struct RowSorter {
             e = cudaMemsetAsync(next, 0, sizeof(ChunkNext), st);
             if (e == cudaSuccess) e = cudaMemsetAsync(ucnt, 0, sizeof(int) * (size_t)n, st);
             if (e != cudaSuccess) return e;
-            const int nl = (int)h.rows[BIN_LONG];
+            const int nl = (int)h->rows[BIN_LONG];
             const int grid = std::min(nch, 152 * 32);
             k_chunks<RT><<<grid_for(nl, 128), 128, 0, st>>>(row, lists.list[BIN_LONG], rows + BIN_LONG, chunks, next);
             k_sort_chunks<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, tmp2);
-            const int passes = merge_passes(h.longest);
+            const int passes = merge_passes(h->longest);
             for (int p = 0; p < passes; p++) k_merge<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, tmp2, p);
             if (dedup) k_chunk_unique<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, ccnt, ucnt);
         }
         auto ctas = [](unsigned rows_, int cap) { return std::max(1, std::min((int)rows_, cap)); };
-        if (h.rows[BIN_4K])
-            k_sort_block<512, RT><<<ctas(h.rows[BIN_4K], 152 * 16), 512, 0, st>>>(row, lists.list[BIN_4K],
+        if (h->rows[BIN_4K])
+            k_sort_block<512, RT><<<ctas(h->rows[BIN_4K], 152 * 16), 512, 0, st>>>(row, lists.list[BIN_4K],
                                                                                  rows + BIN_4K, tmp, dedup, ucnt);
-        if (h.rows[BIN_2K])
-            k_sort_block<256, RT><<<ctas(h.rows[BIN_2K], 152 * 32), 256, 0, st>>>(row, lists.list[BIN_2K],
+        if (h->rows[BIN_2K])
+            k_sort_block<256, RT><<<ctas(h->rows[BIN_2K], 152 * 32), 256, 0, st>>>(row, lists.list[BIN_2K],
                                                                                  rows + BIN_2K, tmp, dedup, ucnt);
-        if (h.rows[BIN_1K])
-            k_sort_block<128, RT><<<ctas(h.rows[BIN_1K], 152 * 64), 128, 0, st>>>(row, lists.list[BIN_1K],
+        if (h->rows[BIN_1K])
+            k_sort_block<128, RT><<<ctas(h->rows[BIN_1K], 152 * 64), 128, 0, st>>>(row, lists.list[BIN_1K],
                                                                                  rows + BIN_1K, tmp, dedup, ucnt);
-        if (h.rows[BIN_W16])
+        if (h->rows[BIN_W16])
             k_sort_warp<16, RT><<<152 * 8, 256, 0, st>>>(row, lists.list[BIN_W16], rows + BIN_W16, tmp, dedup, ucnt);
-        if (h.rows[BIN_W4])
+        if (h->rows[BIN_W4])
             k_sort_warp<4, RT><<<152 * 8, 256, 0, st>>>(row, lists.list[BIN_W4], rows + BIN_W4, tmp, dedup, ucnt);
         k_sort_small<RT><<<grid_for((int64_t)n * 32, thr), thr, 0, st>>>(row, n, tmp, dedup, ucnt);
         return cudaGetLastError();
@@ -1201,8 +1237,8 @@ struct RowSorter {
     // The long rows' distinct values into col (row2: the offsets there).
     cudaError_t compact(const RT *row, const RT *row2, const int *tmp, int *col, cudaStream_t st)
     {
-        if (!h.chunks) return cudaSuccess;
-        k_compact_chunks<RT><<<std::min((int)h.chunks, 152 * 32), MED_THREADS, 0, st>>>(row, row2, chunks, (int)h.chunks,
+        if (!h->chunks) return cudaSuccess;
+        k_compact_chunks<RT><<<std::min((int)h->chunks, 152 * 32), MED_THREADS, 0, st>>>(row, row2, chunks, (int)h->chunks,
                                                                                        ccnt, tmp, col);
         return cudaGetLastError();
     }
@@ -1214,15 +1250,18 @@ template <typename RT>
 int sort_rows_inplace(const RT *row, int *col, int32_t n, int64_t m, cudaStream_t st, std::string &err)
 {
     int rc = GBFS_OK;
-    int *ucnt = nullptr;
+    char *mem = nullptr;
     RowSorter<RT> sorter;
-    CK(cudaMalloc(&ucnt, sizeof(int) * ((size_t)n + 1)));
-    CK(sorter.bin(row, n, m, st));
+    NEED_PINNED(sorter.h);
+    Carve cv;
+    const size_t ucnt = cv.add(sizeof(int) * ((size_t)n + 1)), lists = cv.add(sorter.list_bytes(n, m));
+    CK(cudaMalloc(&mem, cv.size));
+    CK(sorter.bin(row, n, m, mem + lists, st));
     CK(cudaStreamSynchronize(st));
-    CK(sorter.sort(row, n, col, 0, ucnt, st));
+    CK(sorter.sort(row, n, col, 0, (int *)(mem + ucnt), st));
     CK(cudaStreamSynchronize(st));
 done:
-    if (ucnt) cudaFree(ucnt);
+    if (mem) cudaFree(mem);
     return rc;
 }
 
@@ -1437,9 +1476,7 @@ done:
 int csr_build_first(DeviceCsr &c, cudaStream_t st, std::string &err)
 {
     int rc = GBFS_OK;
-    if (!c.first) CK(cudaMalloc(&c.first, sizeof(int) * (size_t)std::max(1, c.n)));
-    // hub-first rows are probed at their first entry alone: no second array
-    if (!c.hub_rows && !c.second) CK(cudaMalloc(&c.second, sizeof(int) * (size_t)std::max(1, c.n)));
+    // (hub-first rows are probed at their first entry alone: no second array)
     if (c.n > 0) {
         if (c.wide)
             k_first<<<grid_for(c.n, 256), 256, 0, st>>>((const long long *)c.row64, (const int *)c.col, c.n, c.first,
@@ -1531,17 +1568,14 @@ void csr_free(DeviceCsr &c)
     if (c.tcol) cudaFree(c.tcol);
     if (c.theavy) cudaFree(c.theavy);
     if (c.tfirst) cudaFree(c.tfirst);
-    if (c.first) cudaFree(c.first);
-    if (c.second) cudaFree(c.second);
     if (c.tpieces) cudaFree(c.tpieces);
     if (c.quad) cudaFree(c.quad);
     if (c.over) cudaFree(c.over);
-    if (c.heavy) cudaFree(c.heavy);
     if (c.pieces) cudaFree(c.pieces);
-    if (c.row) cudaFree(c.row);
-    if (c.row64) cudaFree(c.row64);
+    if (c.own_row && c.row) cudaFree(c.row);
+    if (c.own_row && c.row64) cudaFree(c.row64);
     if (c.col) cudaFree(c.col);
-    if (c.zmask) cudaFree(c.zmask);
+    if (c.block) cudaFree(c.block);
     c = DeviceCsr{};
 }
 
@@ -1559,69 +1593,89 @@ inline cudaError_t scan_rows(const int *in, long long *out, int64_t n, ScanScrat
 // Steps 2-5 with row offsets of type RT (int, or long long for wide
 // graphs): offsets from the degrees, scatter, per-row sort, dedup
 // compaction.  md: edges before deduplication.  On success the offsets and
-// columns move to row_out / col_out.
+// columns are in row_out (n + 1, the caller's) and col_out.  scratch: of
+// BuildScratch's size, or null to allocate it here.
+// Scratch of build_rows: row fill counts, later the rows' distinct counts; the
+// lists of the sorts; and, where deduplication leaves them behind, the rows and
+// columns before it.
+template <typename RT>
+struct BuildScratch {
+    size_t fill, lists, rows = 0, cols = 0, size;
+    BuildScratch(int32_t n, int64_t md, bool dedup)
+    {
+        const size_t row_bytes = sizeof(RT) * ((size_t)n + 1);
+        Carve cv;
+        fill = cv.add(row_bytes);
+        lists = cv.add(RowSorter<RT>::list_bytes(n, md));
+        if (dedup) {
+            rows = cv.add(row_bytes);
+            cols = cv.add(sizeof(int) * (size_t)std::max<int64_t>(md, 1));
+        }
+        size = cv.size;
+    }
+};
+
 template <typename RT>
 int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_dst, unsigned flags,
-               const int *deg, ScanScratch &ss, cudaStream_t st, RT *&row_out, int *&col_out, int64_t &m_out,
+               const int *deg, char *scratch, ScanScratch &ss, cudaStream_t st, RT *row_out, int *&col_out, int64_t &m_out,
                std::string &err)
 {
     int rc = GBFS_OK;
     const bool dedup = flags & GBFS_DEDUP;
-    RT *row = nullptr, *cursor = nullptr, *row2 = nullptr;
-    int *tmp = nullptr, *ucnt = nullptr, *col = nullptr;
+    const size_t row_bytes = sizeof(RT) * ((size_t)n + 1);
+    char *mem = nullptr;
+    int *tmp = nullptr, *col = nullptr;
     const int thr = 256;
+    const BuildScratch<RT> sc(n, md, dedup);
     RowSorter<RT> sorter;
-    CK(cudaMalloc(&row, sizeof(RT) * ((size_t)n + 1)));
-    CK(scan_rows(deg, row, n, ss, st));
-    CK(sorter.bin(row, n, md, st));
-    CK(cudaMalloc(&cursor, sizeof(RT) * ((size_t)n + 1)));
-    CK(cudaMemcpyAsync(cursor, row, sizeof(RT) * ((size_t)n + 1), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMalloc(&tmp, sizeof(int) * (size_t)std::max<int64_t>(md, 1)));
-    if (m > 0) {
-        k_scatter<RT><<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, cursor, tmp);
-        CK(cudaGetLastError());
+    Pinned<RT> h_m2;
+    NEED_PINNED(sorter.h);
+    NEED_PINNED(h_m2);
+    if (!scratch) {
+        CK(cudaMalloc(&mem, sc.size));
+        scratch = mem;
     }
-    CK(cudaMalloc(&ucnt, sizeof(int) * ((size_t)n + 1)));
-    CK(cudaStreamSynchronize(st));
-    cudaFree(cursor);
-    cursor = nullptr;
+    if (!dedup) CK(cudaMalloc(&tmp, sizeof(int) * (size_t)std::max<int64_t>(md, 1)));
+    {
+        RT *const row = dedup ? (RT *)(scratch + sc.rows) : row_out;
+        RT *const cursor = (RT *)(scratch + sc.fill);
+        int *const ucnt = (int *)(scratch + sc.fill);
+        int *const to = dedup ? (int *)(scratch + sc.cols) : tmp;
+        CK(scan_rows(deg, row, n, ss, st));
+        CK(sorter.bin(row, n, md, scratch + sc.lists, st));
+        CK(cudaMemcpyAsync(cursor, row, row_bytes, cudaMemcpyDeviceToDevice, st));
+        if (m > 0) {
+            k_scatter<RT><<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, cursor, to);
+            CK(cudaGetLastError());
+        }
+        CK(cudaStreamSynchronize(st));  // the sorter's counts are here
 
-    // Per-row sort (+ distinct count).
-    CK(sorter.sort(row, n, tmp, dedup, ucnt, st));
+        // Per-row sort (+ distinct count).
+        CK(sorter.sort(row, n, to, dedup, ucnt, st));
 
-    if (dedup) {
-        RT h_m2 = 0;
-        CK(cudaMalloc(&row2, sizeof(RT) * ((size_t)n + 1)));
-        CK(scan_rows(ucnt, row2, n, ss, st));
-        CK(cudaMemcpyAsync(&h_m2, row2 + n, sizeof(RT), cudaMemcpyDeviceToHost, st));
+        if (dedup) {
+            CK(scan_rows(ucnt, row_out, n, ss, st));
+            CK(cudaMemcpyAsync(h_m2.p, row_out + n, sizeof(RT), cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            sorter.drop_tmp2();
+            CK(cudaMalloc(&col, sizeof(int) * (size_t)std::max<int64_t>((int64_t)*h_m2.p, 1)));
+            k_compact<RT><<<grid_for((int64_t)n * 32, thr), thr, 0, st>>>(row, row_out, n, to, col);
+            CK(cudaGetLastError());
+            CK(sorter.compact(row, row_out, to, col, st));
+            m_out = (int64_t)*h_m2.p;
+        } else {
+            col = tmp;
+            tmp = nullptr;
+            m_out = md;
+        }
         CK(cudaStreamSynchronize(st));
-        sorter.drop_tmp2();
-        CK(cudaMalloc(&col, sizeof(int) * (size_t)std::max<int64_t>((int64_t)h_m2, 1)));
-        k_compact<RT><<<grid_for((int64_t)n * 32, thr), thr, 0, st>>>(row, row2, n, tmp, col);
-        CK(cudaGetLastError());
-        CK(sorter.compact(row, row2, tmp, col, st));
-        CK(cudaStreamSynchronize(st));
-        cudaFree(row);
-        row = row2;
-        row2 = nullptr;
-        m_out = (int64_t)h_m2;
-    } else {
-        CK(cudaStreamSynchronize(st));
-        col = tmp;
-        tmp = nullptr;
-        m_out = md;
     }
-    row_out = row;
     col_out = col;
-    row = nullptr;
     col = nullptr;
 done:
-    if (row) cudaFree(row);
-    if (row2) cudaFree(row2);
-    if (cursor) cudaFree(cursor);
+    if (mem) cudaFree(mem);
     if (col) cudaFree(col);
     if (tmp) cudaFree(tmp);
-    if (ucnt) cudaFree(ucnt);
     return rc;
 }
 
@@ -1631,70 +1685,86 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
                          cudaStream_t st, DeviceCsr &out, std::string &err)
 {
     int rc = GBFS_OK;
-    int *deg = nullptr;
-    int *status = nullptr;
+    char *mem = nullptr;
+    int *deg = nullptr, *status = nullptr;
     unsigned long long *total = nullptr;
-    void *scan_mem = nullptr;
     ScanScratch ss;
-    unsigned long long h_total = 0;
-    int h_status = 0;
+    struct Counted {
+        int status, pad;
+        unsigned long long total;
+        unsigned scan[3];
+    };
+    Pinned<Counted> h;
+    NEED_PINNED(h);
     const int thr = 256;
     out = DeviceCsr{};
     out.n = n;
 
-    // Scratch for both scans (n+1 elements at most).
+    // Degrees, scratch for both scans (n+1 elements at most), and the counters.
     const int64_t tiles = scan_tiles((int64_t)n + 1);
-    CK(cudaMalloc(&scan_mem, scan_scratch_bytes(tiles)));
-    CK(cudaMemsetAsync(scan_mem, 0, scan_scratch_bytes(tiles), st));
-    scan_scratch_carve(scan_mem, tiles, ss);
-
-    CK(cudaMalloc(&deg, sizeof(int) * ((size_t)n + 1)));
-    CK(cudaMalloc(&status, 64));
+    Carve cv;
+    const size_t at_deg = cv.add(sizeof(int) * ((size_t)n + 1)), at_scan = cv.add(scan_scratch_bytes(tiles)),
+                 at_status = cv.add(64);
+    const size_t zeroed = cv.size;
+    // with it the scratch of the steps after the count, sized by the input, if
+    // that is small (a large one waits for the count, which may be smaller)
+    const int64_t most = m * (flags & GBFS_SYMMETRIZE ? 2 : 1);
+    const size_t later = flags & GBFS_WIDE_ROWS ? BuildScratch<long long>(n, most, flags & GBFS_DEDUP).size
+                                                : BuildScratch<int>(n, most, flags & GBFS_DEDUP).size;
+    const bool together = later <= (size_t)64 << 20;
+    const size_t at_later = together ? cv.add(later) : 0;
+    CK(cudaMalloc(&mem, cv.size));
+    CK(cudaMemsetAsync(mem, 0, zeroed, st));
+    scan_scratch_carve(mem + at_scan, tiles, ss);
+    deg = (int *)(mem + at_deg);
+    status = (int *)(mem + at_status);
     total = (unsigned long long *)(status + 2);
-    CK(cudaMemsetAsync(deg, 0, sizeof(int) * ((size_t)n + 1), st));
-    CK(cudaMemsetAsync(status, 0, 64, st));
     if (m > 0) {
         k_count<<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, deg, total, status);
         CK(cudaGetLastError());
     }
-    CK(cudaMemcpyAsync(&h_total, total, 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&h_status, status, 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(h.p, status, 16, cudaMemcpyDeviceToHost, st));  // status and total
     CK(cudaStreamSynchronize(st));
-    if (h_status == DEV_OVERFLOW) {
+    if (h->status == DEV_OVERFLOW) {
         err = "a vertex with 2^30 or more edges";
         rc = GBFS_ERR_TOO_LARGE;
         goto done;
     }
-    if (h_status != DEV_OK) {
+    if (h->status != DEV_OK) {
         err = "edge endpoint outside [0, n)";
         rc = GBFS_ERR_INVALID_ARG;
         goto done;
     }
-    out.wide = (flags & GBFS_WIDE_ROWS) || h_total > (unsigned long long)INT32_MAX;
-    if (out.wide)
-        rc = build_rows<long long>(n, m, (int64_t)h_total, d_src, d_dst, flags, deg, ss, st, out.row64, out.col,
-                                   out.m, err);
-    else
-        rc = build_rows<int>(n, m, (int64_t)h_total, d_src, d_dst, flags, deg, ss, st, out.row, out.col, out.m,
-                             err);
+    out.wide = (flags & GBFS_WIDE_ROWS) || h->total > (unsigned long long)INT32_MAX;
+    {
+        const size_t row_bytes = (out.wide ? sizeof(long long) : sizeof(int)) * ((size_t)n + 1);
+        void *row = nullptr;
+        CK(alloc_block(out, !(flags & GBFS_HUB_FIRST), row_bytes, &row));
+        if (out.wide) out.row64 = (long long *)row;
+        else out.row = (int *)row;
+    }
+    {
+        char *const later_mem = together ? mem + at_later : nullptr;
+        const int64_t md = (int64_t)h->total;
+        if (out.wide)
+            rc = build_rows<long long>(n, m, md, d_src, d_dst, flags, deg, later_mem, ss, st, out.row64, out.col, out.m,
+                                       err);
+        else
+            rc = build_rows<int>(n, m, md, d_src, d_dst, flags, deg, later_mem, ss, st, out.row, out.col, out.m, err);
+    }
     if (rc) goto done;
     out.sorted_rows = true;
-    {
-        unsigned h_scan_status[3] = {0, 0, 0};
-        CK(cudaMemcpyAsync(h_scan_status, ss.ctl, 12, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        if (h_scan_status[2] != 0) {
-            err = "scan look-back timed out";
-            rc = GBFS_ERR_TIMEOUT;
-            goto done;
-        }
+    CK(cudaMemcpyAsync(h->scan, ss.ctl, 12, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (h->scan[2] != 0) {
+        err = "scan look-back timed out";
+        rc = GBFS_ERR_TIMEOUT;
+        goto done;
     }
     rc = finalize(out, st, err);
 
 done:
-    if (deg) cudaFree(deg);
-    if (status) cudaFree(status);
-    if (scan_mem) cudaFree(scan_mem);
+    if (mem) cudaFree(mem);
     if (rc != GBFS_OK) csr_free(out);
     return rc;
 }
@@ -1722,6 +1792,7 @@ int csr_adopt_t(int32_t n, int64_t m, RT *d_row, int *d_col, cudaStream_t st, De
         rc = GBFS_ERR_INVALID_ARG;
         goto done;
     }
+    CK(alloc_block(out, true, 0, nullptr));
     rc = finalize(out, st, err);
 done:
     if (status) cudaFree(status);
@@ -1738,6 +1809,7 @@ int csr_adopt(int32_t n, int64_t m, int *d_row, int *d_col, cudaStream_t st, Dev
     out.n = n;
     out.m = m;
     out.row = d_row;
+    out.own_row = true;
     out.col = d_col;
     return csr_adopt_t(n, m, d_row, d_col, st, out, err);
 }
@@ -1749,6 +1821,7 @@ int csr_adopt64(int32_t n, int64_t m, long long *d_row, int *d_col, cudaStream_t
     out.n = n;
     out.m = m;
     out.row64 = d_row;
+    out.own_row = true;
     out.wide = true;
     out.col = d_col;
     return csr_adopt_t(n, m, d_row, d_col, st, out, err);

@@ -11,6 +11,10 @@ namespace gbfs {
 // A CSR resident in HBM.  Rows of graphs built from edges are sorted
 // ascending.  zmask bit v is set when out-degree(v) == 0.
 struct DeviceCsr {
+    // one allocation for the arrays of a vertex's size: zmask, heavy, first and
+    // second, and the row offsets of a graph built here (a given CSR's are its own)
+    void *block = nullptr;
+    bool own_row = false;      // row / row64 is an allocation of its own
     int32_t n = 0;
     int64_t m = 0;
     int *row = nullptr;        // n+1 (null when wide)

@@ -27,6 +27,7 @@
 
 #include "blockq.cuh"
 #include "msbfs.cuh"
+#include "pinned.cuh"
 
 namespace gbfs {
 
@@ -783,29 +784,36 @@ int ms_work_alloc(MsWork &w, int32_t n, std::string &err)
 {
     if (w.ctrl && w.n == n) return GBFS_OK;
     ms_work_free(w);
-    auto al = [&](void **p, size_t b) -> bool {
-        cudaError_t e = cudaMalloc(p, std::max<size_t>(b, 16));
-        if (e != cudaSuccess) {
-            err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
-            return false;
-        }
-        w.bytes += (int64_t)std::max<size_t>(b, 16);
-        return true;
-    };
-    w.bytes = 0;
     const size_t b8 = sizeof(unsigned long long) * (size_t)n, b4 = sizeof(int) * (size_t)n;
-    bool ok = al((void **)&w.vis, b8) && al((void **)&w.hacc, b8) && al((void **)&w.hcnt, b4) &&
-              al((void **)&w.lv8, (size_t)n * MS_LANES) && al((void **)&w.bigl, b4) &&
-              al((void **)&w.out, b4 * MS_LANES) && al((void **)&w.src, sizeof(int) * MS_LANES) &&
-              al((void **)&w.ctrl, sizeof(MsCtrl));
-    for (int i = 0; ok && i < 3; i++) ok = al((void **)&w.F[i], b8);
-    for (int i = 0; ok && i < 4; i++) ok = al((void **)&w.Q[i], b4);
-    if (!ok) {
+    Carve c;
+    const size_t vis = c.add(b8), hacc = c.add(b8), hcnt = c.add(b4), lv8 = c.add((size_t)n * MS_LANES),
+                 bigl = c.add(b4), out = c.add(b4 * MS_LANES), src = c.add(sizeof(int) * MS_LANES),
+                 ctrl = c.add(sizeof(MsCtrl));
+    size_t F[3], Q[4];
+    for (size_t &f : F) f = c.add(b8);
+    for (size_t &x : Q) x = c.add(b4);
+    const cudaError_t e = cudaMalloc(&w.block, c.size);
+    if (e != cudaSuccess) {
+        w.block = nullptr;
+        err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
         ms_work_free(w);
         return GBFS_ERR_OOM;
     }
-    if (cudaMemset(w.ctrl, 0, sizeof(MsCtrl)) != cudaSuccess ||
-        cudaMallocHost(&w.h_ctrl, sizeof(MsCtrl)) != cudaSuccess ||
+    char *p = (char *)w.block;
+    w.vis = (unsigned long long *)(p + vis);
+    w.hacc = (unsigned long long *)(p + hacc);
+    w.hcnt = (unsigned *)(p + hcnt);
+    w.lv8 = (unsigned char *)(p + lv8);
+    w.bigl = (int *)(p + bigl);
+    w.out = (int *)(p + out);
+    w.src = (int *)(p + src);
+    w.ctrl = (MsCtrl *)(p + ctrl);
+    for (int i = 0; i < 3; i++) w.F[i] = (unsigned long long *)(p + F[i]);
+    for (int i = 0; i < 4; i++) w.Q[i] = (int *)(p + Q[i]);
+    w.bytes = (int64_t)c.size;
+    static_assert(offsetof(MsCtrl, t_entry) <= PINNED_SLOT, "the results fit a pinned slot");
+    w.h_ctrl = (MsCtrl *)pinned_slot_take();
+    if (!w.h_ctrl || cudaMemset(w.ctrl, 0, sizeof(MsCtrl)) != cudaSuccess ||
         cudaEventCreate(&w.ev0) != cudaSuccess || cudaEventCreate(&w.ev1) != cudaSuccess) {
         err = "multi-source workspace setup failed";
         ms_work_free(w);
@@ -817,10 +825,8 @@ int ms_work_alloc(MsWork &w, int32_t n, std::string &err)
 
 void ms_work_free(MsWork &w)
 {
-    void *ps[] = {w.vis, w.hacc, w.hcnt, w.lv8, w.bigl, w.out, w.src, w.ctrl, w.F[0], w.F[1], w.F[2], w.Q[0], w.Q[1], w.Q[2], w.Q[3]};
-    for (void *p : ps)
-        if (p) cudaFree(p);
-    if (w.h_ctrl) cudaFreeHost(w.h_ctrl);
+    if (w.block) cudaFree(w.block);
+    pinned_slot_give(w.h_ctrl);
     if (w.ev0) cudaEventDestroy(w.ev0);
     if (w.ev1) cudaEventDestroy(w.ev1);
     w = MsWork{};

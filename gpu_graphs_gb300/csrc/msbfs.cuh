@@ -32,6 +32,7 @@ struct MsCtrl {
 
 struct MsWork {
     int32_t n = 0;
+    void *block = nullptr;               // the device arrays from here to ctrl
     unsigned long long *vis = nullptr;   // n lane masks: lanes that reached v
     unsigned long long *F[3] = {nullptr, nullptr, nullptr};  // frontier masks, rotating
     int *Q[4] = {nullptr, nullptr, nullptr, nullptr};        // active queues, rotating
@@ -42,7 +43,7 @@ struct MsWork {
     int *out = nullptr;                  // MS_LANES * n levels (host-bound results)
     int *src = nullptr;                  // MS_LANES sources
     MsCtrl *ctrl = nullptr;
-    MsCtrl *h_ctrl = nullptr;
+    MsCtrl *h_ctrl = nullptr;            // pinned: the part of a control block before t_entry
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int64_t bytes = 0;
 };

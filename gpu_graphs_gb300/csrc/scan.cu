@@ -64,7 +64,7 @@ __device__ __forceinline__ void store4(long long *o, long long e, int4 x)
 template <typename Tin, typename Tout>
 __global__ void __launch_bounds__(SCAN_THREADS, SCAN_MIN_BLOCKS)
 k_scan_exclusive(const Tin *__restrict__ in, Tout *__restrict__ out, int64_t n,
-                 Tout *__restrict__ total_out, ScanDesc *desc, unsigned *ctl, unsigned epoch, int64_t ntiles,
+                 Tout *__restrict__ total_out, ScanDesc *desc, unsigned *status, unsigned epoch, int64_t ntiles,
                  int vec)
 {
     static_assert(sizeof(Tin) == 4, "4-byte inputs");
@@ -102,7 +102,7 @@ k_scan_exclusive(const Tin *__restrict__ in, Tout *__restrict__ out, int64_t n,
             // the copy did not land in time: report it, and let it land
             // (bounded) before this CTA's shared memory goes away
             if (t == 0) {
-                atomicExch(&ctl[2], (unsigned)DEV_TIMEOUT);
+                *(volatile unsigned *)status = (unsigned)DEV_TIMEOUT;
                 const unsigned long long w1 = globaltimer_ns();
                 while (!mbar_try_wait(&s_bar, 0u) && globaltimer_ns() - w1 < LOOKBACK_TIMEOUT_NS) {
                 }
@@ -209,7 +209,7 @@ k_scan_exclusive(const Tin *__restrict__ in, Tout *__restrict__ out, int64_t n,
             const bool abort = s_abort;
             __syncthreads();
             if (abort) {
-                if (t == 0) atomicExch(&ctl[2], (unsigned)DEV_TIMEOUT);
+                if (t == 0) *(volatile unsigned *)status = (unsigned)DEV_TIMEOUT;
                 prefix = 0;
                 break;
             }
@@ -268,7 +268,7 @@ cudaError_t launch_scan(const Tin *in, Tout *out, int64_t n, Tout *total_out, Sc
     if (e != cudaSuccess) return e;
     const int vec = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
     k_scan_exclusive<Tin, Tout><<<(unsigned)ntiles, SCAN_THREADS, scan_smem_bytes(), st>>>(
-        in, out, n, total_out, s.desc, s.ctl, s.epoch, ntiles, vec);
+        in, out, n, total_out, s.desc, s.status, s.epoch, ntiles, vec);
     return cudaGetLastError();
 }
 
@@ -283,6 +283,7 @@ void scan_scratch_carve(void *mem, int64_t max_tiles, ScanScratch &s)
 {
     char *p = (char *)mem;
     s.ctl = (unsigned *)p;
+    s.status = s.ctl + 2;
     s.desc = (ScanDesc *)(p + 256);
     s.max_tiles = max_tiles;
 }

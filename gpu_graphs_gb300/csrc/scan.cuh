@@ -36,6 +36,7 @@ struct alignas(16) ScanDesc {
 struct ScanScratch {
     ScanDesc *desc = nullptr;       // per tile
     unsigned *ctl = nullptr;        // [2] status (a bounded wait ran out); [0], [1] unused
+    unsigned *status = nullptr;     // where a wait that ran out is reported: &ctl[2], or pinned host memory
     int64_t max_tiles = 0;
     unsigned epoch = 0;             // host-side call counter
 };
