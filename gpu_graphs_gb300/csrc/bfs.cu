@@ -9,10 +9,10 @@
 // Here one cooperative launch runs the whole traversal.  Levels are
 // separated by a bounded grid barrier and every CTA takes the same
 // direction decision from the same counters:
-//   top-down step   frontier queue -> next queue.  Small frontiers: every
-//                   edge balanced over the whole grid (degree prefix in
-//                   shared memory).  Large ones: each warp takes 32
-//                   frontier vertices and walks their rows (below
+//   top-down step   frontier queue -> next queue.  Small frontiers of long
+//                   rows: every edge balanced over the whole grid (degree
+//                   prefix in shared memory).  Others: each warp takes up to
+//                   32 frontier vertices and walks their rows (below
 //                   big_degree) as one concatenated edge range; rows of
 //                   degree >= big_degree are deferred to a grid-wide pass.
 //                   A vertex is claimed with an atomicOr on the visited
@@ -57,6 +57,16 @@ constexpr int COOP_ROWS = 4; // bottom-up rows left in a warp below which the wa
 // of the warp queue's entries, in bottom-up steps the deferred rows' bounds
 // (under 64 left plus a 128-vertex round)
 constexpr int BU_DEF = QCAP;
+// Top-down steps over a queue of at most SEG vertices whose rows average more
+// entries than this balance single edges over the grid; other queues are dealt
+// by rows, as few per warp as keep all warps busy.  Dealing 32 rows to each warp
+// left most warps without any (4,000 rows of 17 entries: 47 us a level), and
+// balancing short rows costs every CTA a scan of them.  Mean searches before and
+// now: uniform random of 1 M vertices 156 -> 106 us, 200,000 vertices 103 -> 81,
+// 3 M vertices 228 -> 194, RMAT 50 -> 50 and 66 -> 63.  Above the line the queue
+// may hold hubs, whose rows would be put off to a pass of their own (RMAT-22
+// with rows always: 95 -> 118 us).
+constexpr unsigned long long BALANCE_DEGREE = 64;
 constexpr unsigned long long BMTD_EDGES = 65536;  // top-down from the bitmap up to this many frontier edges
 // Long searches on graphs whose largest out-degree is at most
 // RELAX_MAX_DEGREE (meshes, grids, road networks: thousands of levels of
@@ -697,21 +707,24 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
             const float growth = fmaxf(1.f, (float)mf / (float)(prev_mf ? prev_mf : 1ull));
             const bool likely_bu = (float)mf * growth * (float)a.alpha > (float)m_u;
             unsigned *fnw = a.direction == GBFS_DIR_OPTIMIZING && brow && likely_bu ? fn : nullptr;
+            const bool balance = nf <= (unsigned long long)SEG && mf > BALANCE_DEGREE * nf;
             if (from_bitmap) {
                 bitmap_expand(fc, W, (long long)nf, a, nl, q, cnt_next, qn, qbn, my_deg, &ctrl->big[L % 3], gwarp, nwarps,
                               lane, fnw);
-            } else if (nf <= (unsigned long long)SEG) {
+            } else if (balance) {
                 // small frontier: every edge of it balanced over the whole grid
                 grid_expand_list<BLOCK, RT>(qc, qbc, (int)nf, a, nl, q, cnt_next, qn, qbn, my_deg, s_pre, s_beg,
                                             s_warp, fnw);
             } else {
-                // large frontier: 32 rows per warp as one concatenated edge
-                // range, rows of degree >= big_degree deferred to a grid pass
-                for (long long base = gwarp * 32; base < (long long)nf; base += nwarps * 32) {
+                // up to 32 rows per warp as one concatenated edge range (fewer
+                // where that would leave warps without rows), rows of degree >=
+                // big_degree deferred to a grid pass
+                const int per = (int)max(1ll, min(32ll, ((long long)nf + nwarps - 1) / nwarps));
+                for (long long base = gwarp * per; base < (long long)nf; base += nwarps * per) {
                     const long long i = base + lane;
                     int v = 0, d = 0;
                     RT b = 0;
-                    if (i < (long long)nf) {
+                    if ((int)lane < per && i < (long long)nf) {
                         v = __ldcg(qc + i);
                         const B be = __ldcg(qbc + i);
                         b = be.x;
@@ -723,10 +736,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
             block_flush_bounds(q, cnt_next, qn, qbn, my_deg, s_wq, s_red, &s_base);
             if (!grid_sync(&ctrl->bar, &ctrl->status, a.timeout_ns, epoch)) return;
 
-            // rows deferred to the grid pass (only large frontiers defer, and
+            // rows deferred to the grid pass (not by edge-balanced steps, and
             // only when some row is that long)
             int nb = 0;
-            if (a.has_big && (nf > (unsigned long long)SEG || from_bitmap)) {
+            if (a.has_big && (!balance || from_bitmap)) {
                 if (threadIdx.x == 0) s_nb = __ldcg(&ctrl->big[L % 3]);
                 __syncthreads();
                 nb = (int)s_nb;
