@@ -9,6 +9,9 @@
 //                lanes with the same source so hubs take one atomic)
 //   2. scan      decoupled look-back exclusive scan -> row offsets
 //   3. k_scatter each edge to its row (aggregated atomic cursors)
+//      Large inputs with ids all over take two steps instead of 1 to 3:
+//      k_bucket_scatter sorts the entries into buckets of 1024 rows, then
+//      k_bucket_rows lays out one bucket per CTA
 //   4. k_bin + per-row sorts by length: up to 32 entries in a warp's registers
 //                (k_sort_small), up to 512 (k_sort_warp), up to 4096 in a CTA's
 //                (k_sort_block), longer rows in sorted chunks of 4096 merged
@@ -178,6 +181,271 @@ __global__ void k_scatter(const int *__restrict__ src, const int *__restrict__ d
             if (v >= 0) tmp[q] = u;
         }
     }
+}
+
+// ---- entries by buckets of rows ----
+// Scattering a power-law graph's entries straight to their rows writes each
+// 32-byte sector of the columns in eight pieces, far apart in time: RMAT-22
+// (134 M entries) spent 1.2 ms counting and 2.8 ms scattering, most of it on
+// partly written sectors leaving L2.  With buckets of 2^BK_LOG rows in between,
+// every write lands beside others of its time: first each entry goes to its
+// bucket as one 32-bit word (row within the bucket, column), in runs gathered
+// in shared memory; then one CTA per bucket counts its rows in shared memory,
+// writes their offsets and places the columns, all within a range that L2 holds.
+// For inputs of BK_MIN_M entries (below, the direct scatter's range fits L2: whole
+// builds, buckets and direct, RMAT of 8 M entries 1.26 and 1.29 ms, 25 M 2.04 and
+// 2.20, 34 M 2.34 and 2.63, 134 M 7.1 and 8.9; uniform random of 12 M entries 1.19
+// and 1.16, 67 M 2.8 and 4.6) on up to BK_MAX_N vertices (a word holds 10 + 22
+// bits), unless one bucket holds more than BK_MAX_BUCKET entries, which would be
+// one CTA's tail, or edges beside each other mostly have both ends in the same
+// buckets (a grid's in order, 17 M entries: 1.44 and 1.20 ms).
+constexpr int BK_LOG = 10;
+constexpr int BK_MAX_N = 1 << 22;
+constexpr int BK_BUCKETS = BK_MAX_N >> BK_LOG;
+constexpr int64_t BK_MIN_M = 20 << 20;
+constexpr unsigned BK_MAX_BUCKET = 1 << 20;
+constexpr int BK_BLOCK = 1024;
+constexpr int BK_ILP = 8;                          // entries per thread in flight in k_bucket_rows
+constexpr int BK_STAGE = 48 << 10;                 // entries of a bucket laid out in shared memory
+constexpr int BK_EDGES = 8;                        // input edges per thread and tile
+constexpr int BK_SBLOCK = 1024;                    // k_bucket_scatter: one CTA per SM
+constexpr int BK_TILE = 2 * BK_SBLOCK * BK_EDGES;  // entries per tile at most
+constexpr int BK_PER = BK_BUCKETS / BK_SBLOCK;     // buckets per thread there
+static_assert(BK_BUCKETS == 4 * BK_BLOCK, "four buckets per thread");
+
+struct BucketPlan {
+    unsigned long long total;
+    unsigned largest, near;          // near, seen: edges of a sample beside one in the same buckets, and all
+    unsigned seen, bigs, others, pad;
+    unsigned hist[BK_BUCKETS];       // zeroed by the caller
+    int start[BK_BUCKETS + 1];
+    int cursor[BK_BUCKETS];
+    int order[BK_BUCKETS];           // the large buckets first
+};
+
+// The input edge i as up to two entries (u -> v, and v -> u with sym); u = -1:
+// none.  Ids outside [0, n) are reported.
+__device__ __forceinline__ void load_edge(const int *__restrict__ src, const int *__restrict__ dst, int64_t i, int64_t m,
+                                          int n, bool noself, int *status, int &u, int &v)
+{
+    u = v = -1;
+    if (i >= m) return;
+    u = src[i];
+    v = dst[i];
+    if ((unsigned)u >= (unsigned)n || (unsigned)v >= (unsigned)n) {
+        atomicExch(status, DEV_BAD_ID);
+        u = v = -1;
+    } else if (noself && u == v) {
+        u = v = -1;
+    }
+}
+
+__global__ void __launch_bounds__(BK_BLOCK)
+k_bucket_hist(const int *__restrict__ src, const int *__restrict__ dst, int64_t m, int n, unsigned flags,
+              BucketPlan *plan, int *status)
+{
+    __shared__ unsigned s_hist[BK_BUCKETS];
+    const bool sym = flags & GBFS_SYMMETRIZE, noself = flags & GBFS_DROP_SELF_LOOPS;
+    for (int b = (int)threadIdx.x; b < BK_BUCKETS; b += BK_BLOCK) s_hist[b] = 0;
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * BK_BLOCK;
+    unsigned near = 0, seen = 0;
+    for (int64_t w0 = (int64_t)blockIdx.x * BK_BLOCK + (threadIdx.x & ~31u); w0 < m; w0 += 4 * stride) {
+        const int64_t i0 = w0 + lane_id();  // (whole warps go round)
+        int u[4], v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) load_edge(src, dst, i0 + q * stride, m, n, noself, status, u[q], v[q]);
+        // (every lane calls the shuffles)
+        const int u1 = __shfl_xor_sync(FULL, u[0], 1), v1 = __shfl_xor_sync(FULL, v[0], 1);
+        if (u[0] >= 0) {
+            near += (u[0] ^ u1) >> BK_LOG == 0 && (v[0] ^ v1) >> BK_LOG == 0;
+            seen++;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (u[q] < 0) continue;
+            atomicAdd(&s_hist[u[q] >> BK_LOG], 1u);
+            if (sym) atomicAdd(&s_hist[v[q] >> BK_LOG], 1u);
+        }
+    }
+    __syncthreads();
+    for (int b = (int)threadIdx.x; b < BK_BUCKETS; b += BK_BLOCK)
+        if (s_hist[b]) atomicAdd(&plan->hist[b], s_hist[b]);
+    near = warp_sum(near);
+    seen = warp_sum(seen);
+    if (lane_id() == 0) {
+        atomicAdd(&plan->near, near);
+        atomicAdd(&plan->seen, seen);
+    }
+}
+
+// One CTA: where each bucket starts, the largest, and the order to lay them out.
+__global__ void __launch_bounds__(BK_BLOCK) k_bucket_plan(BucketPlan *plan, int nb)
+{
+    __shared__ int s_warp[33];
+    const int b0 = 4 * (int)threadIdx.x;
+    int c[4], sum = 0, most = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        c[k] = (int)plan->hist[b0 + k];
+        sum += c[k];
+        most = max(most, c[k]);
+    }
+    int total;
+    int at = block_excl_scan(sum, s_warp, &total);
+    if (threadIdx.x == 0) {
+        plan->total = (unsigned long long)total;
+        plan->start[BK_BUCKETS] = total;
+    }
+    atomicMax(&plan->largest, (unsigned)most);
+    const int big = 2 * (total / nb) + 1;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        plan->start[b0 + k] = at;
+        plan->cursor[b0 + k] = at;
+        at += c[k];
+        if (b0 + k >= nb) continue;
+        const int pos = c[k] >= big ? (int)atomicAdd(&plan->bigs, 1u) : nb - 1 - (int)atomicAdd(&plan->others, 1u);
+        plan->order[pos] = b0 + k;
+    }
+}
+
+struct BucketShared {
+    int2 run[BK_BUCKETS];   // x: entries of the bucket in the tile, then where its run starts there; y: and in the output
+    uint2 entry[BK_TILE];   // the runs: word, place in the output
+    int warp[33];
+};
+
+__global__ void __launch_bounds__(BK_SBLOCK, 1)
+k_bucket_scatter(const int *__restrict__ src, const int *__restrict__ dst, int64_t m, int n, unsigned flags, int vbits,
+                 BucketPlan *plan, int *status, unsigned *__restrict__ packed)
+{
+    extern __shared__ __align__(16) unsigned char bk_smem[];
+    auto &sh = *reinterpret_cast<BucketShared *>(bk_smem);
+    const bool sym = flags & GBFS_SYMMETRIZE, noself = flags & GBFS_DROP_SELF_LOOPS;
+    const int t = (int)threadIdx.x;
+    constexpr int64_t TILE = BK_SBLOCK * BK_EDGES;
+    for (int64_t base = (int64_t)blockIdx.x * TILE; base < m; base += (int64_t)gridDim.x * TILE) {
+        for (int b = t; b < BK_BUCKETS; b += BK_SBLOCK) sh.run[b].x = 0;
+        int u[BK_EDGES], v[BK_EDGES];
+#pragma unroll
+        for (int q = 0; q < BK_EDGES; q++) load_edge(src, dst, base + q * BK_SBLOCK + t, m, n, noself, status, u[q], v[q]);
+        // the next tile's edges on their way to L2
+        const int64_t ahead = base + (int64_t)gridDim.x * TILE + 32 * (int64_t)t;
+        if (32 * t < TILE && ahead < m) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(src + ahead));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(dst + ahead));
+        }
+        __syncthreads();
+        unsigned rank[BK_EDGES];  // within the tile's runs: of (u -> v), and << 16 of (v -> u)
+#pragma unroll
+        for (int q = 0; q < BK_EDGES; q++) {
+            rank[q] = 0;
+            if (u[q] < 0) continue;
+            rank[q] = (unsigned)atomicAdd(&sh.run[u[q] >> BK_LOG].x, 1);
+            if (sym) rank[q] |= (unsigned)atomicAdd(&sh.run[v[q] >> BK_LOG].x, 1) << 16;
+        }
+        __syncthreads();
+        int c[BK_PER], sum = 0;
+#pragma unroll
+        for (int k = 0; k < BK_PER; k++) {
+            c[k] = sh.run[k * BK_SBLOCK + t].x;
+            sum += c[k];
+        }
+        int total;
+        int at = block_excl_scan(sum, sh.warp, &total);
+#pragma unroll
+        for (int k = 0; k < BK_PER; k++) {
+            sh.run[k * BK_SBLOCK + t] = make_int2(at, c[k] ? atomicAdd(&plan->cursor[k * BK_SBLOCK + t], c[k]) : 0);
+            at += c[k];
+        }
+        __syncthreads();
+        auto put = [&](int row, int colv, unsigned r) {
+            const int2 run = sh.run[row >> BK_LOG];
+            sh.entry[run.x + r] =
+                make_uint2((unsigned)(row & ((1 << BK_LOG) - 1)) << vbits | (unsigned)colv, (unsigned)run.y + r);
+        };
+#pragma unroll
+        for (int q = 0; q < BK_EDGES; q++) {
+            if (u[q] < 0) continue;
+            put(u[q], v[q], rank[q] & 0xffffu);
+            if (sym) put(v[q], u[q], rank[q] >> 16);
+        }
+        __syncthreads();
+        for (int j = t; j < total; j += BK_SBLOCK) {
+            const uint2 x = sh.entry[j];
+            packed[x.y] = x.x;
+        }
+        __syncthreads();
+    }
+}
+
+// agg_atomic_add on shared memory, where only a row that several lanes hit at
+// once is worth a group (one atomic instead of a conflict per lane): the lanes
+// that share lane 0's key, if they are half of them.
+__device__ __forceinline__ int shared_rank_add(int *arr, int key)
+{
+    const unsigned same = __ballot_sync(FULL, key == __shfl_sync(FULL, key, 0));
+    const bool grouped = __popc(same) >= 16;
+    const bool mine = grouped && (same >> lane_id() & 1u);
+    int old = 0;
+    if (key >= 0 && (!mine || lane_id() == 0)) old = atomicAdd(arr + key, mine ? __popc(same) : 1);
+    if (!grouped) return old;
+    const int base = __shfl_sync(FULL, old, 0);
+    return mine ? base + __popc(same & lanemask_lt()) : old;
+}
+
+// One CTA per bucket: row offsets, and the columns to their rows (in no
+// particular order within a row), put together in shared memory where the
+// bucket fits there (a scattered global store costs a cycle per lane).
+__global__ void __launch_bounds__(BK_BLOCK, 1)
+k_bucket_rows(const BucketPlan *__restrict__ plan, const unsigned *__restrict__ packed, int vbits, int n, int *row,
+              int *tmp)
+{
+    extern __shared__ int s_stage[];  // BK_STAGE columns
+    __shared__ int s_cnt[1 << BK_LOG];
+    __shared__ int s_warp[33];
+    static_assert(BK_BLOCK == 1 << BK_LOG, "a thread per row");
+    const int t = (int)threadIdx.x, b = plan->order[blockIdx.x];
+    const int s = plan->start[b], e = plan->start[b + 1];
+    const unsigned mask = (1u << vbits) - 1u;
+    s_cnt[t] = 0;
+    __syncthreads();
+    for (int i0 = s; i0 < e; i0 += BK_ILP * BK_BLOCK) {
+        unsigned w[BK_ILP];
+#pragma unroll
+        for (int q = 0; q < BK_ILP; q++) w[q] = i0 + q * BK_BLOCK + t < e ? packed[i0 + q * BK_BLOCK + t] : 0u;
+#pragma unroll
+        for (int q = 0; q < BK_ILP; q++) shared_rank_add(s_cnt, i0 + q * BK_BLOCK + t < e ? (int)(w[q] >> vbits) : -1);
+    }
+    __syncthreads();
+    const int c = s_cnt[t];
+    int total;
+    const int off = block_excl_scan(c, s_warp, &total);
+    const int v = (b << BK_LOG) + t;
+    if (v < n) row[v] = s + off;
+    if (v == n - 1) row[n] = s + off + c;
+    s_cnt[t] = off;
+    __syncthreads();
+    const bool staged = e - s <= BK_STAGE;
+    int *const out = tmp + s;
+    for (int i0 = s; i0 < e; i0 += BK_ILP * BK_BLOCK) {
+        unsigned w[BK_ILP];
+#pragma unroll
+        for (int q = 0; q < BK_ILP; q++) w[q] = i0 + q * BK_BLOCK + t < e ? packed[i0 + q * BK_BLOCK + t] : 0u;
+#pragma unroll
+        for (int q = 0; q < BK_ILP; q++) {
+            const bool in = i0 + q * BK_BLOCK + t < e;
+            const int pos = shared_rank_add(s_cnt, in ? (int)(w[q] >> vbits) : -1);
+            if (!in) continue;
+            if (staged) s_stage[pos] = (int)(w[q] & mask);
+            else out[pos] = (int)(w[q] & mask);
+        }
+    }
+    if (!staged) return;
+    __syncthreads();
+    for (int i = t; i < e - s; i += BK_BLOCK) out[i] = s_stage[i];
 }
 
 struct BinLists {
@@ -1191,7 +1459,8 @@ struct RowSorter {
     // Sorts the rows of tmp (the caller has synchronised st since bin).  Rows
     // are packed in place and counted in ucnt (n entries), distinct values only
     // with dedup; then the long rows' are left for compact().
-    cudaError_t sort(const RT *row, int32_t n, int *tmp, int dedup, int *ucnt, cudaStream_t st)
+    // spare (may be null): room for the long rows' entries.
+    cudaError_t sort(const RT *row, int32_t n, int *tmp, int dedup, int *ucnt, int *spare, cudaStream_t st)
     {
         const unsigned *rows = d_cnt->rows;
         const int thr = 256;
@@ -1200,7 +1469,8 @@ struct RowSorter {
         if (nch) {
             const size_t cb = sizeof(Chunk) * (size_t)nch;
             e = cudaMalloc(&long_mem, 256 + cb + sizeof(int) * (size_t)nch);
-            if (e == cudaSuccess) e = cudaMalloc(&tmp2, sizeof(int) * (size_t)h->long_entries);
+            if (e == cudaSuccess && !spare) e = cudaMalloc(&tmp2, sizeof(int) * (size_t)h->long_entries);
+            int *const two = spare ? spare : tmp2;
             if (e != cudaSuccess) return e;
             ChunkNext *next = (ChunkNext *)long_mem;
             chunks = (Chunk *)((char *)long_mem + 256);
@@ -1211,9 +1481,9 @@ struct RowSorter {
             const int nl = (int)h->rows[BIN_LONG];
             const int grid = std::min(nch, 152 * 32);
             k_chunks<RT><<<grid_for(nl, 128), 128, 0, st>>>(row, lists.list[BIN_LONG], rows + BIN_LONG, chunks, next);
-            k_sort_chunks<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, tmp2);
+            k_sort_chunks<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, two);
             const int passes = merge_passes(h->longest);
-            for (int p = 0; p < passes; p++) k_merge<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, tmp2, p);
+            for (int p = 0; p < passes; p++) k_merge<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, two, p);
             if (dedup) k_chunk_unique<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, ccnt, ucnt);
         }
         auto ctas = [](unsigned rows_, int cap) { return std::max(1, std::min((int)rows_, cap)); };
@@ -1258,7 +1528,7 @@ int sort_rows_inplace(const RT *row, int *col, int32_t n, int64_t m, cudaStream_
     CK(cudaMalloc(&mem, cv.size));
     CK(sorter.bin(row, n, m, mem + lists, st));
     CK(cudaStreamSynchronize(st));
-    CK(sorter.sort(row, n, col, 0, (int *)(mem + ucnt), st));
+    CK(sorter.sort(row, n, col, 0, (int *)(mem + ucnt), nullptr, st));
     CK(cudaStreamSynchronize(st));
 done:
     if (mem) cudaFree(mem);
@@ -1594,7 +1864,9 @@ inline cudaError_t scan_rows(const int *in, long long *out, int64_t n, ScanScrat
 // graphs): offsets from the degrees, scatter, per-row sort, dedup
 // compaction.  md: edges before deduplication.  On success the offsets and
 // columns are in row_out (n + 1, the caller's) and col_out.  scratch: of
-// BuildScratch's size, or null to allocate it here.
+// BuildScratch's size, or null to allocate it here.  With packed (room for md
+// entries; freed here when the sorts are done, or left to the caller), by
+// buckets (plan) instead of by the degrees.
 // Scratch of build_rows: row fill counts, later the rows' distinct counts; the
 // lists of the sorts; and, where deduplication leaves them behind, the rows and
 // columns before it.
@@ -1617,7 +1889,7 @@ struct BuildScratch {
 
 template <typename RT>
 int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_dst, unsigned flags,
-               const int *deg, char *scratch, ScanScratch &ss, cudaStream_t st, RT *row_out, int *&col_out, int64_t &m_out,
+               const int *deg, BucketPlan *plan, unsigned *&packed, char *scratch, ScanScratch &ss, cudaStream_t st, RT *row_out, int *&col_out, int64_t &m_out,
                std::string &err)
 {
     int rc = GBFS_OK;
@@ -1641,23 +1913,42 @@ int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_
         RT *const cursor = (RT *)(scratch + sc.fill);
         int *const ucnt = (int *)(scratch + sc.fill);
         int *const to = dedup ? (int *)(scratch + sc.cols) : tmp;
-        CK(scan_rows(deg, row, n, ss, st));
-        CK(sorter.bin(row, n, md, scratch + sc.lists, st));
-        CK(cudaMemcpyAsync(cursor, row, row_bytes, cudaMemcpyDeviceToDevice, st));
-        if (m > 0) {
-            k_scatter<RT><<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, cursor, to);
+        if (packed) {
+            int vbits = 1;
+            while ((1 << vbits) < n) vbits++;
+            CK(cudaFuncSetAttribute(k_bucket_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(BucketShared)));
+            k_bucket_scatter<<<152, BK_SBLOCK, sizeof(BucketShared), st>>>(d_src, d_dst, m, n, flags, vbits, plan,
+                                                                          (int *)(scratch + sc.fill), packed);
             CK(cudaGetLastError());
+            CK(cudaFuncSetAttribute(k_bucket_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(int) * BK_STAGE));
+            if constexpr (sizeof(RT) == sizeof(int))
+                k_bucket_rows<<<((n - 1) >> BK_LOG) + 1, BK_BLOCK, sizeof(int) * BK_STAGE, st>>>(plan, packed, vbits, n,
+                                                                                               row, to);
+            CK(cudaGetLastError());
+            CK(sorter.bin(row, n, md, scratch + sc.lists, st));
+        } else {
+            CK(scan_rows(deg, row, n, ss, st));
+            CK(sorter.bin(row, n, md, scratch + sc.lists, st));
+            CK(cudaMemcpyAsync(cursor, row, row_bytes, cudaMemcpyDeviceToDevice, st));
+            if (m > 0) {
+                k_scatter<RT><<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, cursor, to);
+                CK(cudaGetLastError());
+            }
         }
         CK(cudaStreamSynchronize(st));  // the sorter's counts are here
 
         // Per-row sort (+ distinct count).
-        CK(sorter.sort(row, n, to, dedup, ucnt, st));
+        CK(sorter.sort(row, n, to, dedup, ucnt, (int *)packed, st));
 
         if (dedup) {
             CK(scan_rows(ucnt, row_out, n, ss, st));
             CK(cudaMemcpyAsync(h_m2.p, row_out + n, sizeof(RT), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             sorter.drop_tmp2();
+            if (packed) cudaFree(packed);
+            packed = nullptr;
             CK(cudaMalloc(&col, sizeof(int) * (size_t)std::max<int64_t>((int64_t)*h_m2.p, 1)));
             k_compact<RT><<<grid_for((int64_t)n * 32, thr), thr, 0, st>>>(row, row_out, n, to, col);
             CK(cudaGetLastError());
@@ -1693,7 +1984,11 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
         int status, pad;
         unsigned long long total;
         unsigned scan[3];
+        unsigned long long bucket_total;
+        unsigned bucket_largest, bucket_near, bucket_seen, pad2;
     };
+    unsigned *packed = nullptr;
+    BucketPlan *plan = nullptr;
     Pinned<Counted> h;
     NEED_PINNED(h);
     const int thr = 256;
@@ -1704,7 +1999,7 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
     const int64_t tiles = scan_tiles((int64_t)n + 1);
     Carve cv;
     const size_t at_deg = cv.add(sizeof(int) * ((size_t)n + 1)), at_scan = cv.add(scan_scratch_bytes(tiles)),
-                 at_status = cv.add(64);
+                 at_status = cv.add(64), at_plan = cv.add(sizeof(BucketPlan));
     const size_t zeroed = cv.size;
     // with it the scratch of the steps after the count, sized by the input, if
     // that is small (a large one waits for the count, which may be smaller)
@@ -1719,7 +2014,22 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
     deg = (int *)(mem + at_deg);
     status = (int *)(mem + at_status);
     total = (unsigned long long *)(status + 2);
-    if (m > 0) {
+    plan = (BucketPlan *)(mem + at_plan);
+    if (!(flags & GBFS_WIDE_ROWS) && most >= BK_MIN_M && most <= INT32_MAX && n <= BK_MAX_N) {
+        k_bucket_hist<<<152 * 2, BK_BLOCK, 0, st>>>(d_src, d_dst, m, n, flags, plan, status);
+        CK(cudaGetLastError());
+        k_bucket_plan<<<1, BK_BLOCK, 0, st>>>(plan, ((n - 1) >> BK_LOG) + 1);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(&h->bucket_total, plan, 20, cudaMemcpyDeviceToHost, st));  // total to seen
+        CK(cudaStreamSynchronize(st));
+        if (h->bucket_largest <= BK_MAX_BUCKET && h->bucket_total > 0 && h->bucket_near <= h->bucket_seen / 2 &&
+            cudaMalloc(&packed, sizeof(unsigned) * (size_t)h->bucket_total) != cudaSuccess) {
+            cudaGetLastError();  // no room: straight to the rows
+            packed = nullptr;
+        }
+        if (packed) CK(cudaMemcpyAsync(total, &plan->total, 8, cudaMemcpyDeviceToDevice, st));
+    }
+    if (m > 0 && !packed) {
         k_count<<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, deg, total, status);
         CK(cudaGetLastError());
     }
@@ -1747,10 +2057,11 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
         char *const later_mem = together ? mem + at_later : nullptr;
         const int64_t md = (int64_t)h->total;
         if (out.wide)
-            rc = build_rows<long long>(n, m, md, d_src, d_dst, flags, deg, later_mem, ss, st, out.row64, out.col, out.m,
-                                       err);
+            rc = build_rows<long long>(n, m, md, d_src, d_dst, flags, deg, plan, packed, later_mem, ss, st, out.row64,
+                                       out.col, out.m, err);
         else
-            rc = build_rows<int>(n, m, md, d_src, d_dst, flags, deg, later_mem, ss, st, out.row, out.col, out.m, err);
+            rc = build_rows<int>(n, m, md, d_src, d_dst, flags, deg, plan, packed, later_mem, ss, st, out.row, out.col,
+                                 out.m, err);
     }
     if (rc) goto done;
     out.sorted_rows = true;
@@ -1765,6 +2076,7 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
 
 done:
     if (mem) cudaFree(mem);
+    if (packed) cudaFree(packed);
     if (rc != GBFS_OK) csr_free(out);
     return rc;
 }
