@@ -255,17 +255,18 @@ k_bucket_hist(const int *__restrict__ src, const int *__restrict__ dst, int64_t 
         int u[4], v[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) load_edge(src, dst, i0 + q * stride, m, n, noself, status, u[q], v[q]);
-        // (every lane calls the shuffles)
-        const int u1 = __shfl_xor_sync(FULL, u[0], 1), v1 = __shfl_xor_sync(FULL, v[0], 1);
-        if (u[0] >= 0) {
-            near += (u[0] ^ u1) >> BK_LOG == 0 && (v[0] ^ v1) >> BK_LOG == 0;
-            seen++;
-        }
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             if (u[q] < 0) continue;
             atomicAdd(&s_hist[u[q] >> BK_LOG], 1u);
             if (sym) atomicAdd(&s_hist[v[q] >> BK_LOG], 1u);
+        }
+        if (w0 < stride) {  // the sample: the warps' first edges (every lane calls the shuffles)
+            const int u1 = __shfl_xor_sync(FULL, u[0], 1), v1 = __shfl_xor_sync(FULL, v[0], 1);
+            if (u[0] >= 0) {
+                near = (u[0] ^ u1) >> BK_LOG == 0 && (v[0] ^ v1) >> BK_LOG == 0;
+                seen = 1;
+            }
         }
     }
     __syncthreads();
@@ -1190,37 +1191,68 @@ __global__ void k_check_sorted(const RT *__restrict__ row, const int *__restrict
 // probes first.  One warp per row below HUB_CTA_ROW, one CTA above.
 constexpr int HUB_CTA_ROW = 4096;
 
-template <typename RT>
-__device__ __forceinline__ unsigned long long hub_key(const RT *row, int v, int pos)
+// deg: the rows' lengths (one 4-byte gather per entry instead of two offsets).
+__device__ __forceinline__ unsigned long long hub_key(const int *__restrict__ deg, int v, int pos)
 {
-    const unsigned d = (unsigned)(row[v + 1] - row[v]);
-    return ((unsigned long long)d << 32) | (unsigned)(0x7fffffff - pos);
+    return ((unsigned long long)(unsigned)__ldg(deg + v) << 32) | (unsigned)(0x7fffffff - pos);
 }
 
 template <typename RT>
-__global__ void k_hub_first_warp(const RT *__restrict__ row, int n, int *col)
+__global__ void k_row_lengths(const RT *__restrict__ row, int n, int *deg)
+{
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+        deg[v] = (int)(row[v + 1] - row[v]);
+}
+
+__device__ __forceinline__ void hub_swap(int *row_col, int pos)
+{
+    if (pos <= 0) return;
+    const int t = row_col[0];
+    row_col[0] = row_col[pos];
+    row_col[pos] = t;
+}
+
+// A warp takes 32 consecutive rows: those of up to 8 entries a lane each, all
+// at once, the others one after another (RMAT-22: 633 us with a warp per row and
+// two offsets read per entry, 400 so).
+template <typename RT>
+__global__ void k_hub_first_warp(const RT *__restrict__ row, const int *__restrict__ deg, int n, int *col)
 {
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
-        const RT b = row[r];
-        const int d = (int)(row[r + 1] - b);
-        if (d < 2 || d >= HUB_CTA_ROW) continue;
-        unsigned long long best = 0;
-        for (int i = lane_id(); i < d; i += 32) {
-            const unsigned long long k = hub_key(row, col[b + i], i);
-            best = k > best ? k : best;
-        }
+    const int lane = (int)lane_id();
+    for (int64_t r0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; r0 < n; r0 += warps * 32) {
+        const RT bl = r0 + lane < n ? row[r0 + lane] : 0;
+        const int dl = r0 + lane < n ? deg[r0 + lane] : 0;
+        if (dl >= 2 && dl <= 8) {
+            int v[8];
+            unsigned long long best = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long y = __shfl_xor_sync(FULL, best, o);
-            best = y > best ? y : best;
+            for (int e = 0; e < 8; e++) v[e] = e < dl ? col[bl + e] : -1;
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                if (v[e] >= 0) {
+                    const unsigned long long k = hub_key(deg, v[e], e);
+                    best = k > best ? k : best;
+                }
+            hub_swap(col + bl, 0x7fffffff - (int)(best & 0xffffffffu));
         }
-        const int pos = 0x7fffffff - (int)(best & 0xffffffffu);
-        __syncwarp();
-        if (lane_id() == 0 && pos > 0) {
-            const int t = col[b];
-            col[b] = col[b + pos];
-            col[b + pos] = t;
+        unsigned left = __ballot_sync(FULL, dl > 8 && dl < HUB_CTA_ROW);
+        while (left) {
+            const int j = __ffs(left) - 1;
+            left &= left - 1u;
+            const RT b = __shfl_sync(FULL, bl, j);
+            const int d = __shfl_sync(FULL, dl, j);
+            unsigned long long best = 0;
+#pragma unroll 4
+            for (int i = lane; i < d; i += 32) {
+                const unsigned long long k = hub_key(deg, col[b + i], i);
+                best = k > best ? k : best;
+            }
+            // the longest length among the lanes, then its first place
+            const unsigned top = __reduce_max_sync(FULL, (unsigned)(best >> 32));
+            const unsigned at = __reduce_max_sync(FULL, (unsigned)(best >> 32) == top ? (unsigned)best : 0u);
+            __syncwarp();
+            if (lane == 0) hub_swap(col + b, 0x7fffffff - (int)at);
         }
     }
 }
@@ -1251,7 +1283,7 @@ __global__ void k_rows_by_len(const RT *__restrict__ row, int n, int lo, int hi,
 
 // One CTA per listed row (list[0, *cnt)).
 template <typename RT>
-__global__ void k_hub_first_cta(const RT *__restrict__ row, const int *__restrict__ list, const unsigned *cnt, int *col)
+__global__ void k_hub_first_cta(const RT *__restrict__ row, const int *__restrict__ deg, const int *__restrict__ list, const unsigned *cnt, int *col)
 {
     __shared__ unsigned long long s_best[32];
     const int count = (int)*cnt;
@@ -1261,7 +1293,7 @@ __global__ void k_hub_first_cta(const RT *__restrict__ row, const int *__restric
         const int d = (int)(row[r + 1] - b);
         unsigned long long best = 0;
         for (int i = threadIdx.x; i < d; i += blockDim.x) {
-            const unsigned long long k = hub_key(row, col[b + i], i);
+            const unsigned long long k = hub_key(deg, col[b + i], i);
             best = k > best ? k : best;
         }
 #pragma unroll
@@ -1288,7 +1320,7 @@ __global__ void k_hub_first_cta(const RT *__restrict__ row, const int *__restric
 // every warp folds its entries' keys and takes the row's maximum with one
 // atomicMax (best[g], zeroed by the caller); k_hub_giant_swap then moves it.
 template <typename RT>
-__global__ void k_hub_giant_max(const RT *__restrict__ row, const int *__restrict__ list, const unsigned *cnt,
+__global__ void k_hub_giant_max(const RT *__restrict__ row, const int *__restrict__ deg, const int *__restrict__ list, const unsigned *cnt,
                                 const int *__restrict__ col, unsigned long long *best)
 {
     const int count = (int)*cnt;
@@ -1300,7 +1332,7 @@ __global__ void k_hub_giant_max(const RT *__restrict__ row, const int *__restric
         const int d = (int)(row[r + 1] - b);
         unsigned long long mine = 0;
         for (int64_t i = tid; i < d; i += stride) {
-            const unsigned long long k = hub_key(row, col[b + i], (int)i);
+            const unsigned long long k = hub_key(deg, col[b + i], (int)i);
             mine = k > mine ? k : mine;
         }
 #pragma unroll
@@ -1544,39 +1576,49 @@ template <typename RT>
 int hub_first_rows(const RT *row, int n, int64_t m, int *col, cudaStream_t st, std::string &err)
 {
     int rc = GBFS_OK;
-    int *lists = nullptr;
+    char *mem = nullptr;
+    int *deg = nullptr, *lists = nullptr;
     unsigned *cnts = nullptr;
     unsigned long long *best = nullptr;
-    unsigned h[2] = {0, 0};
+    struct Counts {
+        unsigned rows[2];  // long, giant
+    };
+    Pinned<Counts> h;
+    NEED_PINNED(h);
     const int64_t cap_long = std::min<int64_t>(n, m / HUB_CTA_ROW + 1);
     const int64_t cap_giant = std::min<int64_t>(n, m / HUB_GIANT_ROW + 1);
-    CK(cudaMalloc(&lists, sizeof(int) * (size_t)(cap_long + cap_giant)));
-    CK(cudaMalloc(&cnts, 2 * sizeof(unsigned)));
+    Carve cv;
+    const size_t at_deg = cv.add(sizeof(int) * (size_t)n), at_lists = cv.add(sizeof(int) * (size_t)(cap_long + cap_giant)),
+                 at_cnts = cv.add(2 * sizeof(unsigned));
+    CK(cudaMalloc(&mem, cv.size));
+    deg = (int *)(mem + at_deg);
+    lists = (int *)(mem + at_lists);
+    cnts = (unsigned *)(mem + at_cnts);
     CK(cudaMemsetAsync(cnts, 0, 2 * sizeof(unsigned), st));
-    k_hub_first_warp<RT><<<grid_for((int64_t)n * 32, 256), 256, 0, st>>>(row, n, col);
+    k_row_lengths<RT><<<grid_for(n, 256), 256, 0, st>>>(row, n, deg);
+    k_hub_first_warp<RT><<<grid_for(n, 256, 152 * 64), 256, 0, st>>>(row, deg, n, col);
     CK(cudaGetLastError());
     k_rows_by_len<RT><<<grid_for(n, 256), 256, 0, st>>>(row, n, HUB_CTA_ROW, HUB_GIANT_ROW, lists, cnts);
     CK(cudaGetLastError());
     k_rows_by_len<RT><<<grid_for(n, 256), 256, 0, st>>>(row, n, HUB_GIANT_ROW, INT_MAX, lists + cap_long, cnts + 1);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(h, cnts, sizeof(h), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(h.p, cnts, sizeof(Counts), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (h[0]) {
-        k_hub_first_cta<RT><<<152 * 2, 512, 0, st>>>(row, lists, cnts, col);
+    if (h->rows[0]) {
+        k_hub_first_cta<RT><<<152 * 2, 512, 0, st>>>(row, deg, lists, cnts, col);
         CK(cudaGetLastError());
     }
-    if (h[1]) {
-        CK(cudaMalloc(&best, sizeof(unsigned long long) * h[1]));
-        CK(cudaMemsetAsync(best, 0, sizeof(unsigned long long) * h[1], st));
-        k_hub_giant_max<RT><<<152 * 4, 512, 0, st>>>(row, lists + cap_long, cnts + 1, col, best);
+    if (h->rows[1]) {
+        CK(cudaMalloc(&best, sizeof(unsigned long long) * h->rows[1]));
+        CK(cudaMemsetAsync(best, 0, sizeof(unsigned long long) * h->rows[1], st));
+        k_hub_giant_max<RT><<<152 * 4, 512, 0, st>>>(row, deg, lists + cap_long, cnts + 1, col, best);
         CK(cudaGetLastError());
         k_hub_giant_swap<RT><<<1, 256, 0, st>>>(row, lists + cap_long, cnts + 1, best, col);
         CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(st));
 done:
-    if (lists) cudaFree(lists);
-    if (cnts) cudaFree(cnts);
+    if (mem) cudaFree(mem);
     if (best) cudaFree(best);
     return rc;
 }
