@@ -216,11 +216,13 @@ static_assert(BK_BUCKETS == 4 * BK_BLOCK, "four buckets per thread");
 struct BucketPlan {
     unsigned long long total;
     unsigned largest, near;          // near, seen: edges of a sample beside one in the same buckets, and all
-    unsigned seen, bigs, others, pad;
+    unsigned seen, over;             // over: entries in buckets too large for shared memory, together
+    unsigned bigs, others;
     unsigned hist[BK_BUCKETS];       // zeroed by the caller
     int start[BK_BUCKETS + 1];
     int cursor[BK_BUCKETS];
     int order[BK_BUCKETS];           // the large buckets first
+    int over_at[BK_BUCKETS];         // of those too large: where in the spare buffer
 };
 
 // The input edge i as up to two entries (u -> v, and v -> u with sym); u = -1:
@@ -299,6 +301,16 @@ __global__ void __launch_bounds__(BK_BLOCK) k_bucket_plan(BucketPlan *plan, int 
         plan->start[BK_BUCKETS] = total;
     }
     atomicMax(&plan->largest, (unsigned)most);
+    int mine_over = 0, over;
+#pragma unroll
+    for (int k = 0; k < 4; k++) mine_over += c[k] > BK_STAGE ? c[k] : 0;
+    int over_at = block_excl_scan(mine_over, s_warp, &over);
+    if (threadIdx.x == 0) plan->over = (unsigned)over;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        plan->over_at[b0 + k] = over_at;
+        over_at += c[k] > BK_STAGE ? c[k] : 0;
+    }
     const int big = 2 * (total / nb) + 1;
     __syncthreads();
 #pragma unroll
@@ -397,12 +409,12 @@ __device__ __forceinline__ int shared_rank_add(int *arr, int key)
     return mine ? base + __popc(same & lanemask_lt()) : old;
 }
 
-// One CTA per bucket: row offsets, and the columns to their rows (in no
-// particular order within a row), put together in shared memory where the
-// bucket fits there (a scattered global store costs a cycle per lane).
+// One CTA per bucket: row offsets, and the words replaced by the columns in
+// their rows (in no particular order within a row), put together in shared
+// memory where the bucket fits there (a scattered global store costs a cycle per
+// lane), else in the spare buffer.
 __global__ void __launch_bounds__(BK_BLOCK, 1)
-k_bucket_rows(const BucketPlan *__restrict__ plan, const unsigned *__restrict__ packed, int vbits, int n, int *row,
-              int *tmp)
+k_bucket_rows(const BucketPlan *__restrict__ plan, unsigned *packed, int vbits, int n, int *row, int *spare)
 {
     extern __shared__ int s_stage[];  // BK_STAGE columns
     __shared__ int s_cnt[1 << BK_LOG];
@@ -430,7 +442,7 @@ k_bucket_rows(const BucketPlan *__restrict__ plan, const unsigned *__restrict__ 
     s_cnt[t] = off;
     __syncthreads();
     const bool staged = e - s <= BK_STAGE;
-    int *const out = tmp + s;
+    int *const over = spare + plan->over_at[b];
     for (int i0 = s; i0 < e; i0 += BK_ILP * BK_BLOCK) {
         unsigned w[BK_ILP];
 #pragma unroll
@@ -441,12 +453,11 @@ k_bucket_rows(const BucketPlan *__restrict__ plan, const unsigned *__restrict__ 
             const int pos = shared_rank_add(s_cnt, in ? (int)(w[q] >> vbits) : -1);
             if (!in) continue;
             if (staged) s_stage[pos] = (int)(w[q] & mask);
-            else out[pos] = (int)(w[q] & mask);
+            else over[pos] = (int)(w[q] & mask);
         }
     }
-    if (!staged) return;
-    __syncthreads();
-    for (int i = t; i < e - s; i += BK_BLOCK) out[i] = s_stage[i];
+    __syncthreads();  // every word has been read
+    for (int i = t; i < e - s; i += BK_BLOCK) packed[s + i] = (unsigned)(staged ? s_stage[i] : over[i]);
 }
 
 struct BinLists {
@@ -1491,8 +1502,9 @@ struct RowSorter {
     // Sorts the rows of tmp (the caller has synchronised st since bin).  Rows
     // are packed in place and counted in ucnt (n entries), distinct values only
     // with dedup; then the long rows' are left for compact().
-    // spare (may be null): room for the long rows' entries.
-    cudaError_t sort(const RT *row, int32_t n, int *tmp, int dedup, int *ucnt, int *spare, cudaStream_t st)
+    // spare (may be null): spare_n entries of scratch.
+    cudaError_t sort(const RT *row, int32_t n, int *tmp, int dedup, int *ucnt, int *spare, int64_t spare_n,
+                     cudaStream_t st)
     {
         const unsigned *rows = d_cnt->rows;
         const int thr = 256;
@@ -1501,6 +1513,7 @@ struct RowSorter {
         if (nch) {
             const size_t cb = sizeof(Chunk) * (size_t)nch;
             e = cudaMalloc(&long_mem, 256 + cb + sizeof(int) * (size_t)nch);
+            if ((int64_t)h->long_entries > spare_n) spare = nullptr;
             if (e == cudaSuccess && !spare) e = cudaMalloc(&tmp2, sizeof(int) * (size_t)h->long_entries);
             int *const two = spare ? spare : tmp2;
             if (e != cudaSuccess) return e;
@@ -1560,7 +1573,7 @@ int sort_rows_inplace(const RT *row, int *col, int32_t n, int64_t m, cudaStream_
     CK(cudaMalloc(&mem, cv.size));
     CK(sorter.bin(row, n, m, mem + lists, st));
     CK(cudaStreamSynchronize(st));
-    CK(sorter.sort(row, n, col, 0, (int *)(mem + ucnt), nullptr, st));
+    CK(sorter.sort(row, n, col, 0, (int *)(mem + ucnt), nullptr, 0, st));
     CK(cudaStreamSynchronize(st));
 done:
     if (mem) cudaFree(mem);
@@ -1902,20 +1915,44 @@ inline cudaError_t scan_rows(const int *in, long long *out, int64_t n, ScanScrat
     return scan_exclusive_i32_i64(in, out, n, out + n, ss, st);
 }
 
-// Steps 2-5 with row offsets of type RT (int, or long long for wide
-// graphs): offsets from the degrees, scatter, per-row sort, dedup
-// compaction.  md: edges before deduplication.  On success the offsets and
-// columns are in row_out (n + 1, the caller's) and col_out.  scratch: of
-// BuildScratch's size, or null to allocate it here.  With packed (room for md
-// entries; freed here when the sorts are done, or left to the caller), by
-// buckets (plan) instead of by the degrees.
+// Memory for a build by buckets: the entries (words, then the columns before
+// deduplication) and spare ones, for the overfull buckets and, as far as it
+// goes, the long rows' second place.  Without packed: no buckets.
+struct Buckets {
+    BucketPlan *plan = nullptr;  // the caller's
+    unsigned *packed = nullptr;
+    int *spare = nullptr;
+    int64_t spare_n = 0;
+
+    bool take(int64_t md, int64_t over)
+    {
+        spare_n = std::max<int64_t>(over, md / 5 + 1);
+        if (cudaMalloc(&packed, sizeof(unsigned) * (size_t)md) == cudaSuccess &&
+            cudaMalloc(&spare, sizeof(int) * (size_t)spare_n) == cudaSuccess)
+            return true;
+        cudaGetLastError();
+        drop();
+        return false;
+    }
+    void drop()
+    {
+        if (packed) cudaFree(packed);
+        if (spare) cudaFree(spare);
+        packed = nullptr;
+        spare = nullptr;
+        spare_n = 0;
+    }
+    ~Buckets() { drop(); }
+};
+
 // Scratch of build_rows: row fill counts, later the rows' distinct counts; the
 // lists of the sorts; and, where deduplication leaves them behind, the rows and
 // columns before it.
 template <typename RT>
 struct BuildScratch {
     size_t fill, lists, rows = 0, cols = 0, size;
-    BuildScratch(int32_t n, int64_t md, bool dedup)
+    // (with_cols: the entries go straight to their rows, not by buckets)
+    BuildScratch(int32_t n, int64_t md, bool dedup, bool with_cols = true)
     {
         const size_t row_bytes = sizeof(RT) * ((size_t)n + 1);
         Carve cv;
@@ -1923,16 +1960,22 @@ struct BuildScratch {
         lists = cv.add(RowSorter<RT>::list_bytes(n, md));
         if (dedup) {
             rows = cv.add(row_bytes);
-            cols = cv.add(sizeof(int) * (size_t)std::max<int64_t>(md, 1));
+            if (with_cols) cols = cv.add(sizeof(int) * (size_t)std::max<int64_t>(md, 1));
         }
         size = cv.size;
     }
 };
 
+// Steps 2-5 with row offsets of type RT (int, or long long for wide
+// graphs): offsets from the degrees, scatter, per-row sort, dedup
+// compaction.  md: edges before deduplication.  On success the offsets and
+// columns are in row_out (n + 1, the caller's) and col_out.  scratch: of
+// BuildScratch's size, or null to allocate it here.  With room for buckets
+// (taken over), by those instead of by the degrees.
 template <typename RT>
 int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_dst, unsigned flags,
-               const int *deg, BucketPlan *plan, unsigned *&packed, char *scratch, ScanScratch &ss, cudaStream_t st, RT *row_out, int *&col_out, int64_t &m_out,
-               std::string &err)
+               const int *deg, Buckets &bk, char *scratch, ScanScratch &ss, cudaStream_t st, RT *row_out, int *&col_out,
+               int64_t &m_out, std::string &err)
 {
     int rc = GBFS_OK;
     const bool dedup = flags & GBFS_DEDUP;
@@ -1940,7 +1983,8 @@ int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_
     char *mem = nullptr;
     int *tmp = nullptr, *col = nullptr;
     const int thr = 256;
-    const BuildScratch<RT> sc(n, md, dedup);
+    const bool buckets = bk.packed != nullptr;
+    const BuildScratch<RT> sc(n, md, dedup, !buckets);
     RowSorter<RT> sorter;
     Pinned<RT> h_m2;
     NEED_PINNED(sorter.h);
@@ -1949,25 +1993,30 @@ int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_
         CK(cudaMalloc(&mem, sc.size));
         scratch = mem;
     }
-    if (!dedup) CK(cudaMalloc(&tmp, sizeof(int) * (size_t)std::max<int64_t>(md, 1)));
+    if (buckets) {
+        tmp = (int *)bk.packed;  // laid out in place
+        bk.packed = nullptr;
+    } else if (!dedup) {
+        CK(cudaMalloc(&tmp, sizeof(int) * (size_t)std::max<int64_t>(md, 1)));
+    }
     {
         RT *const row = dedup ? (RT *)(scratch + sc.rows) : row_out;
         RT *const cursor = (RT *)(scratch + sc.fill);
         int *const ucnt = (int *)(scratch + sc.fill);
-        int *const to = dedup ? (int *)(scratch + sc.cols) : tmp;
-        if (packed) {
+        int *const to = tmp ? tmp : (int *)(scratch + sc.cols);
+        if (buckets) {
             int vbits = 1;
             while ((1 << vbits) < n) vbits++;
             CK(cudaFuncSetAttribute(k_bucket_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sizeof(BucketShared)));
-            k_bucket_scatter<<<152, BK_SBLOCK, sizeof(BucketShared), st>>>(d_src, d_dst, m, n, flags, vbits, plan,
-                                                                          (int *)(scratch + sc.fill), packed);
+            k_bucket_scatter<<<152, BK_SBLOCK, sizeof(BucketShared), st>>>(d_src, d_dst, m, n, flags, vbits, bk.plan,
+                                                                          (int *)(scratch + sc.fill), (unsigned *)tmp);
             CK(cudaGetLastError());
             CK(cudaFuncSetAttribute(k_bucket_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sizeof(int) * BK_STAGE));
             if constexpr (sizeof(RT) == sizeof(int))
-                k_bucket_rows<<<((n - 1) >> BK_LOG) + 1, BK_BLOCK, sizeof(int) * BK_STAGE, st>>>(plan, packed, vbits, n,
-                                                                                               row, to);
+                k_bucket_rows<<<((n - 1) >> BK_LOG) + 1, BK_BLOCK, sizeof(int) * BK_STAGE, st>>>(
+                    bk.plan, (unsigned *)tmp, vbits, n, row, bk.spare);
             CK(cudaGetLastError());
             CK(sorter.bin(row, n, md, scratch + sc.lists, st));
         } else {
@@ -1982,15 +2031,14 @@ int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_
         CK(cudaStreamSynchronize(st));  // the sorter's counts are here
 
         // Per-row sort (+ distinct count).
-        CK(sorter.sort(row, n, to, dedup, ucnt, (int *)packed, st));
+        CK(sorter.sort(row, n, to, dedup, ucnt, bk.spare, bk.spare_n, st));
 
         if (dedup) {
             CK(scan_rows(ucnt, row_out, n, ss, st));
             CK(cudaMemcpyAsync(h_m2.p, row_out + n, sizeof(RT), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             sorter.drop_tmp2();
-            if (packed) cudaFree(packed);
-            packed = nullptr;
+            bk.drop();
             CK(cudaMalloc(&col, sizeof(int) * (size_t)std::max<int64_t>((int64_t)*h_m2.p, 1)));
             k_compact<RT><<<grid_for((int64_t)n * 32, thr), thr, 0, st>>>(row, row_out, n, to, col);
             CK(cudaGetLastError());
@@ -2027,10 +2075,9 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
         unsigned long long total;
         unsigned scan[3];
         unsigned long long bucket_total;
-        unsigned bucket_largest, bucket_near, bucket_seen, pad2;
+        unsigned bucket_largest, bucket_near, bucket_seen, bucket_over;
     };
-    unsigned *packed = nullptr;
-    BucketPlan *plan = nullptr;
+    Buckets bk;
     Pinned<Counted> h;
     NEED_PINNED(h);
     const int thr = 256;
@@ -2056,22 +2103,20 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
     deg = (int *)(mem + at_deg);
     status = (int *)(mem + at_status);
     total = (unsigned long long *)(status + 2);
-    plan = (BucketPlan *)(mem + at_plan);
+    bk.plan = (BucketPlan *)(mem + at_plan);
     if (!(flags & GBFS_WIDE_ROWS) && most >= BK_MIN_M && most <= INT32_MAX && n <= BK_MAX_N) {
-        k_bucket_hist<<<152 * 2, BK_BLOCK, 0, st>>>(d_src, d_dst, m, n, flags, plan, status);
+        k_bucket_hist<<<152 * 2, BK_BLOCK, 0, st>>>(d_src, d_dst, m, n, flags, bk.plan, status);
         CK(cudaGetLastError());
-        k_bucket_plan<<<1, BK_BLOCK, 0, st>>>(plan, ((n - 1) >> BK_LOG) + 1);
+        k_bucket_plan<<<1, BK_BLOCK, 0, st>>>(bk.plan, ((n - 1) >> BK_LOG) + 1);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(&h->bucket_total, plan, 20, cudaMemcpyDeviceToHost, st));  // total to seen
+        CK(cudaMemcpyAsync(&h->bucket_total, bk.plan, 24, cudaMemcpyDeviceToHost, st));  // total to over
         CK(cudaStreamSynchronize(st));
+        // (no room for them: straight to the rows)
         if (h->bucket_largest <= BK_MAX_BUCKET && h->bucket_total > 0 && h->bucket_near <= h->bucket_seen / 2 &&
-            cudaMalloc(&packed, sizeof(unsigned) * (size_t)h->bucket_total) != cudaSuccess) {
-            cudaGetLastError();  // no room: straight to the rows
-            packed = nullptr;
-        }
-        if (packed) CK(cudaMemcpyAsync(total, &plan->total, 8, cudaMemcpyDeviceToDevice, st));
+            bk.take((int64_t)h->bucket_total, h->bucket_over))
+            CK(cudaMemcpyAsync(total, &bk.plan->total, 8, cudaMemcpyDeviceToDevice, st));
     }
-    if (m > 0 && !packed) {
+    if (m > 0 && !bk.packed) {
         k_count<<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, deg, total, status);
         CK(cudaGetLastError());
     }
@@ -2099,11 +2144,10 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
         char *const later_mem = together ? mem + at_later : nullptr;
         const int64_t md = (int64_t)h->total;
         if (out.wide)
-            rc = build_rows<long long>(n, m, md, d_src, d_dst, flags, deg, plan, packed, later_mem, ss, st, out.row64,
-                                       out.col, out.m, err);
+            rc = build_rows<long long>(n, m, md, d_src, d_dst, flags, deg, bk, later_mem, ss, st, out.row64, out.col,
+                                       out.m, err);
         else
-            rc = build_rows<int>(n, m, md, d_src, d_dst, flags, deg, plan, packed, later_mem, ss, st, out.row, out.col,
-                                 out.m, err);
+            rc = build_rows<int>(n, m, md, d_src, d_dst, flags, deg, bk, later_mem, ss, st, out.row, out.col, out.m, err);
     }
     if (rc) goto done;
     out.sorted_rows = true;
@@ -2118,7 +2162,6 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
 
 done:
     if (mem) cudaFree(mem);
-    if (packed) cudaFree(packed);
     if (rc != GBFS_OK) csr_free(out);
     return rc;
 }
