@@ -14,8 +14,10 @@
 //      k_bucket_rows lays out one bucket per CTA
 //   4. k_bin + per-row sorts by length: up to 32 entries in a warp's registers
 //                (k_sort_small), up to 512 (k_sort_warp), up to 4096 in a CTA's
-//                (k_sort_block), longer rows in sorted chunks of 4096 merged
-//                pairwise, every chunk of every row in parallel (k_merge);
+//                (k_sort_block); longer rows through bitmaps of the vertices
+//                (k_long_rows, deduplicating builds of up to 4.3 M vertices),
+//                else in sorted chunks of 4096 merged pairwise, every chunk of
+//                every row in parallel (k_merge);
 //                each row also counts (and packs to its front) its distinct
 //                values when deduplicating
 //   5. scan + k_compact   packed rows -> final col_idx (dedup only)
@@ -817,6 +819,152 @@ __global__ void __launch_bounds__(T) k_sort_block(const RT *__restrict__ row, co
 }
 
 // ---- rows longer than MED_MAX ----
+// Distinct values of rows over not too many vertices: a bitmap of the vertices
+// in shared memory, of which each CTA of a cluster holds a range.  All CTAs read
+// the row and set their range's bits, count them, and after the cluster barrier
+// (every entry has been read, and every CTA's count is known to the others)
+// write their range's values over the row, in ascending order.  A row costs two
+// reads of the bitmap and no comparisons.  What bounds it: the smem atomics of a
+// row's entries, and a handful of barriers per row (two CTAs per SM overlap
+// them; one CTA with twice the threads and range was 1 % slower).  Builds with
+// the long rows sorted in chunks and merged, and so: RMAT-22 6.95 and 6.30 ms
+// (their kernels 0.98 and 0.6), RMAT-21 3.89 and 3.33, RMAT-20 2.52 and 2.07,
+// 4,096 vertices of 4,096 neighbours 4.75 and 3.77.  More CTAs per row mean more
+// readers of its entries and more of the bitmap per entry: RMAT-23 with five CTAs
+// of twice the range 16.7 and 16.6 ms, so larger graphs keep the chunks.  Rows of
+// 2,049 to 4,096 entries pay off where one or two CTAs hold the bitmap (RMAT-20
+// 2.07 and 2.04 ms, RMAT-19 1.50 and 1.46; RMAT-22 6.45 and 7.48).
+
+constexpr int BMR_THREADS = 512;
+constexpr int BMR_WORDS = 53;    // words of the bitmap per thread, at most
+constexpr int BMR_CTAS = 5;      // CTAs of the largest cluster (4.3 M vertices)
+constexpr int BMR_CTAS_4K = 2;   // and where rows of 2,049 to 4,096 entries take part
+constexpr int BMR_ILP = 8;       // a thread's entries in flight
+constexpr int BMR_CLUSTERS = 16; // clusters per one that the SMs hold (long rows differ much:
+                                 // RMAT-22 6.45 ms with 2, 6.37 with 16)
+
+// Words per thread (odd: the lanes' pieces start on different banks) and CTAs per
+// row for n vertices.
+struct BitmapShape {
+    int words, ctas;
+    explicit BitmapShape(int64_t n)
+    {
+        const int64_t all = (n + 32 * BMR_THREADS - 1) / (32 * BMR_THREADS);
+        ctas = (int)((all + BMR_WORDS - 1) / BMR_WORDS);
+        words = (int)((all + ctas - 1) / ctas) | 1;
+    }
+    size_t smem() const { return sizeof(unsigned) * BMR_THREADS * (size_t)words; }
+};
+
+template <typename RT>
+__global__ void __launch_bounds__(BMR_THREADS)
+k_long_rows(const RT *__restrict__ row, const int *__restrict__ list, const unsigned *cnt, int words, int *tmp,
+            int *ucnt)
+{
+    extern __shared__ __align__(16) unsigned s_bits[];
+    __shared__ int s_warp[33];
+    __shared__ int s_count[2][BMR_CTAS];  // each CTA's, by the parity of the cluster's row
+    const int t = (int)threadIdx.x;
+    unsigned rank, ctas;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+    const unsigned range = 32u * BMR_THREADS * (unsigned)words, v0 = rank * range;
+    unsigned *const mine = s_bits + t * words;
+    for (int k = 0; k < words; k++) mine[k] = 0;
+    __syncthreads();
+    const int count = (int)*cnt, step = (int)(gridDim.x / ctas);
+    int par = 0, li = (int)(blockIdx.x / ctas);
+    int r = 0, rn = li < count ? list[li] : 0;  // the row, and the next one
+    RT b = 0, bn = row[rn], en = row[rn + 1];
+    for (; li < count; li += step, par ^= 1) {
+        r = rn;
+        b = bn;
+        const int d = (int)(en - b);
+        int *const at = tmp + b;
+        if (li + step < count) rn = list[li + step];
+        for (unsigned i0 = (unsigned)t; i0 < (unsigned)d; i0 += BMR_ILP * BMR_THREADS) {
+            unsigned u[BMR_ILP];
+#pragma unroll
+            for (int q = 0; q < BMR_ILP; q++) {
+                const unsigned i = i0 + (unsigned)(q * BMR_THREADS);
+                u[q] = i < (unsigned)d ? (unsigned)at[i] - v0 : range;
+            }
+#pragma unroll
+            for (int q = 0; q < BMR_ILP; q++)
+                if (u[q] < range) atomicOr(&s_bits[u[q] >> 5], 1u << (u[q] & 31));
+        }
+        bn = row[rn];
+        en = row[rn + 1];
+        __syncthreads();
+        unsigned set[2] = {0, 0};  // this thread's words with set bits
+        int c = 0, total;
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll 8
+            for (int k = 32 * h; k < min(words, 32 * h + 32); k++) {
+                const unsigned w = mine[k];
+                c += __popc(w);
+                if (w) set[h] |= 1u << (k - 32 * h);
+            }
+        int o = block_excl_scan(c, s_warp, &total);
+        if (t < (int)ctas) {
+            unsigned to;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_addr(&s_count[par][rank])), "r"(t));
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to), "r"(total) : "memory");
+        }
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        int all = 0;
+        for (unsigned k = 0; k < ctas; k++) {
+            if (k == rank) o += all;
+            all += s_count[par][k];
+        }
+        if (rank == 0 && t == 0) ucnt[r] = all;
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            while (set[h]) {
+                const int k = 32 * h + __ffs(set[h]) - 1;
+                set[h] &= set[h] - 1;
+                unsigned w = mine[k];
+                mine[k] = 0;
+                const int v = (int)(v0 + 32u * (unsigned)(t * words + k));
+                while (w) {
+                    at[o++] = v + __ffs(w) - 1;
+                    w &= w - 1;
+                }
+            }
+        __syncthreads();  // the bitmap is clear
+    }
+}
+
+// Copies the packed long rows, each by up to eight CTAs.
+constexpr int CPL_THREADS = 512, CPL_PER = 8;
+
+template <typename RT>
+__global__ void __launch_bounds__(CPL_THREADS)
+k_compact_long(const RT *__restrict__ row, const RT *__restrict__ row2, const int *__restrict__ list,
+               const int *__restrict__ tmp, int *col)
+{
+    const int r = list[blockIdx.x];
+    const int *const from = tmp + row[r];
+    int *const to = col + row2[r];
+    const int c = (int)(row2[r + 1] - row2[r]);
+    for (int64_t i0 = (int64_t)blockIdx.y * (CPL_THREADS * CPL_PER); i0 < c;
+         i0 += (int64_t)gridDim.y * (CPL_THREADS * CPL_PER)) {
+        int x[CPL_PER];
+#pragma unroll
+        for (int q = 0; q < CPL_PER; q++) {
+            const int64_t i = i0 + q * CPL_THREADS + threadIdx.x;
+            x[q] = i < c ? from[i] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < CPL_PER; q++) {
+            const int64_t i = i0 + q * CPL_THREADS + threadIdx.x;
+            if (i < c) to[i] = x[q];
+        }
+    }
+}
+
+// Other long rows:
 // A long row is sorted in chunks of MED_MAX, all chunks of all such rows at
 // once, and its chunks are merged pairwise, one tile of MED_MAX outputs per
 // CTA.  RMAT-22 has 1,794 long rows of 25.5 M entries, the longest 320 K: a
@@ -1448,6 +1596,7 @@ struct RowSorter {
     Pinned<BinCounts> h;       // d_cnt's values once st has been synchronised
     Chunk *chunks = nullptr;
     int *ccnt = nullptr;
+    bool bitmaps = false;      // the long rows have been sorted by k_long_rows
 
     ~RowSorter()
     {
@@ -1499,6 +1648,49 @@ struct RowSorter {
         return e;
     }
 
+    // The rows of list c by k_long_rows, where they may; taken: they are sorted.
+    cudaError_t sort_long(int c, const RT *row, int32_t n, int *tmp, int *ucnt, cudaStream_t st, bool &taken)
+    {
+        taken = false;
+        const BitmapShape shape(n);
+        if (shape.ctas > BMR_CTAS) return cudaSuccess;
+        static LaunchSetup setup;  // per row offset type
+        auto config = [&](int ctas, int clusters, size_t smem, cudaLaunchAttribute *at) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(ctas * clusters));
+            cfg.blockDim = dim3(BMR_THREADS);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            at->id = cudaLaunchAttributeClusterDimension;
+            at->val.clusterDim.x = (unsigned)ctas;
+            at->val.clusterDim.y = at->val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            return cfg;
+        };
+        int sms = 0, fits = 0;
+        cudaError_t e = setup.get(sms, fits, [&](int dev, int &s_out, int &f_out) {
+            const size_t most = sizeof(unsigned) * BMR_THREADS * BMR_WORDS;
+            cudaError_t x = cudaFuncSetAttribute(k_long_rows<RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+            if (x == cudaSuccess) x = cudaDeviceGetAttribute(&s_out, cudaDevAttrMultiProcessorCount, dev);
+            cudaLaunchAttribute at;
+            const cudaLaunchConfig_t cfg = config(BMR_CTAS, 1, most, &at);
+            if (x == cudaSuccess) x = cudaOccupancyMaxActiveClusters(&f_out, k_long_rows<RT>, &cfg);
+            return x;
+        });
+        if (e != cudaSuccess || fits < 1) {
+            (void)cudaGetLastError();
+            return cudaSuccess;
+        }
+        const int clusters = std::min((int)h->rows[c], std::max(1, BMR_CLUSTERS * sms / shape.ctas));
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = config(shape.ctas, clusters, shape.smem(), &at);
+        e = cudaLaunchKernelEx(&cfg, k_long_rows<RT>, row, (const int *)lists.list[c],
+                               (const unsigned *)(d_cnt->rows + c), shape.words, tmp, ucnt);
+        taken = e == cudaSuccess;
+        return e;
+    }
+
     // Sorts the rows of tmp (the caller has synchronised st since bin).  Rows
     // are packed in place and counted in ucnt (n entries), distinct values only
     // with dedup; then the long rows' are left for compact().
@@ -1510,7 +1702,11 @@ struct RowSorter {
         const int thr = 256;
         cudaError_t e = cudaSuccess;
         const int nch = (int)h->chunks;
-        if (nch) {
+        if (nch && dedup) {
+            e = sort_long(BIN_LONG, row, n, tmp, ucnt, st, bitmaps);
+            if (e != cudaSuccess) return e;
+        }
+        if (nch && !bitmaps) {
             const size_t cb = sizeof(Chunk) * (size_t)nch;
             e = cudaMalloc(&long_mem, 256 + cb + sizeof(int) * (size_t)nch);
             if ((int64_t)h->long_entries > spare_n) spare = nullptr;
@@ -1532,7 +1728,11 @@ struct RowSorter {
             if (dedup) k_chunk_unique<RT><<<grid, MED_THREADS, 0, st>>>(row, chunks, nch, tmp, ccnt, ucnt);
         }
         auto ctas = [](unsigned rows_, int cap) { return std::max(1, std::min((int)rows_, cap)); };
-        if (h->rows[BIN_4K])
+        bool done4k = false;
+        if (h->rows[BIN_4K] && dedup && BitmapShape(n).ctas <= BMR_CTAS_4K)
+            e = sort_long(BIN_4K, row, n, tmp, ucnt, st, done4k);
+        if (e != cudaSuccess) return e;
+        if (h->rows[BIN_4K] && !done4k)
             k_sort_block<512, RT><<<ctas(h->rows[BIN_4K], 152 * 16), 512, 0, st>>>(row, lists.list[BIN_4K],
                                                                                  rows + BIN_4K, tmp, dedup, ucnt);
         if (h->rows[BIN_2K])
@@ -1553,6 +1753,12 @@ struct RowSorter {
     cudaError_t compact(const RT *row, const RT *row2, const int *tmp, int *col, cudaStream_t st)
     {
         if (!h->chunks) return cudaSuccess;
+        if (bitmaps) {
+            const int tiles = (h->longest + CPL_THREADS * CPL_PER - 1) / (CPL_THREADS * CPL_PER);
+            const dim3 grid(h->rows[BIN_LONG], (unsigned)std::min(tiles, 8));
+            k_compact_long<RT><<<grid, CPL_THREADS, 0, st>>>(row, row2, lists.list[BIN_LONG], tmp, col);
+            return cudaGetLastError();
+        }
         k_compact_chunks<RT><<<std::min((int)h->chunks, 152 * 32), MED_THREADS, 0, st>>>(row, row2, chunks, (int)h->chunks,
                                                                                        ccnt, tmp, col);
         return cudaGetLastError();
