@@ -108,8 +108,8 @@ typedef struct gbfs_graph_info {
     int64_t m;                  /* stored directed edges                     */
     int64_t nonisolated;        /* vertices with out-degree > 0              */
     int64_t device_bytes;       /* CSR and what is built on it (first-entry
-                                   arrays, pull pieces, transpose) + per-graph
-                                   search workspace                          */
+                                   arrays, fixed-width adjacency, pull pieces,
+                                   transpose) + per-graph search workspace   */
     int32_t wide;               /* 1: 64-bit row offsets                     */
     int32_t reserved;
 } gbfs_graph_info;
