@@ -436,7 +436,7 @@ extern "C" int gbfs_bfs_parents(gbfs_graph *g, int32_t source, int32_t *levels_o
     if (rc) return fail(rc, err);
     // long rows in pieces; a graph without room for those is walked by whole rows
     if (ms_prepare(g->csr, g->stream, err) != GBFS_OK) cudaGetLastError();
-    cudaError_t e = parents_enqueue(g->csr, g->symmetric, source, d_level, d_parent, g->stream);
+    cudaError_t e = parents_enqueue(g->csr, g->symmetric, source, d_level, w.ctrl, d_parent, g->stream);
     if (e == cudaSuccess && !dev_par)
         e = cudaMemcpyAsync(parents_out, d_parent, sizeof(int) * n, cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess && levels_out && !dev_lv)

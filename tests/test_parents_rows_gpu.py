@@ -43,3 +43,44 @@ def test_parents_row_classes(gb, orc, order):
         want = orc.bfs_queue(o, s)
         assert np.array_equal(lv, want)
         assert np.array_equal(par, orc.min_parents(o, want))
+
+
+@pytest.mark.parametrize("order", ["hub_first", "hub_first_wide", "unsorted", "star_chain"])
+def test_parents_offered(gb, orc, order):
+    """Large symmetric graphs with rows that do not ascend: some levels offer themselves."""
+    if order == "star_chain":  # light, heavy and split rows offer, below a dense core
+        n, src, dst = _star_chain(4)
+        rng = np.random.default_rng(5)
+        u = rng.integers(n - 20_000, n, (2, 4_800_000)).astype(np.int32)
+        src, dst = np.concatenate([src, u[0]]), np.concatenate([dst, u[1]])
+    else:
+        n = 1 << 19
+        src, dst = gb.gen_rmat(19, 16, seed=9)
+    o = orc.csr_build(n, src, dst, orc.SYMMETRIZE | orc.DROP_SELF_LOOPS | orc.DEDUP)
+    assert o.row_offset[-1] >= 1 << 23
+    if order == "unsorted":
+        g = gb.Graph.from_csr(o.row_offset.astype(np.int32), _rotated(o))
+    else:
+        g = gb.Graph.from_edges(n, src, dst, gb.UNDIRECTED | gb.HUB_FIRST | (gb.WIDE_ROWS if "wide" in order else 0))
+    deg = np.diff(o.row_offset)
+    light = np.flatnonzero(deg > 0)
+    for s in (0, int(np.argmax(deg)), int(light[np.argmin(deg[light])])):
+        lv, par = g.bfs_parents(s)
+        want = orc.bfs_queue(o, s)
+        assert np.array_equal(lv, want)
+        assert np.array_equal(par, orc.min_parents(o, want))
+
+
+def _rotated(o):
+    """The columns with every row's first entry moved to its end."""
+    col = o.col_idx.copy()
+    row = o.row_offset
+    some = np.flatnonzero(np.diff(row) > 1)
+    first = col[row[some]].copy()
+    nxt = np.arange(1, len(col) + 1)
+    nxt[-1] = len(col) - 1
+    out = col[nxt]
+    out[row[some + 1] - 1] = first
+    single = np.flatnonzero(np.diff(row) == 1)
+    out[row[single]] = col[row[single]]
+    return np.ascontiguousarray(out)
