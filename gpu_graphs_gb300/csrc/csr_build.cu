@@ -865,13 +865,11 @@ k_long_rows(const RT *__restrict__ row, const int *__restrict__ list, const unsi
     __shared__ int s_warp[33];
     __shared__ int s_count[2][BMR_CTAS];  // each CTA's, by the parity of the cluster's row
     const int t = (int)threadIdx.x;
-    unsigned rank, ctas;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+    const unsigned rank = cluster_rank(), ctas = cluster_size();
     const unsigned range = 32u * BMR_THREADS * (unsigned)words, v0 = rank * range;
     unsigned *const mine = s_bits + t * words;
     for (int k = 0; k < words; k++) mine[k] = 0;
-    __syncthreads();
+    cluster_barrier();  // the bitmaps are clear, and every CTA has started: the first row's counts may go out
     const int count = (int)*cnt, step = (int)(gridDim.x / ctas);
     int par = 0, li = (int)(blockIdx.x / ctas);
     int r = 0, rn = li < count ? list[li] : 0;  // the row, and the next one
@@ -907,12 +905,9 @@ k_long_rows(const RT *__restrict__ row, const int *__restrict__ list, const unsi
                 if (w) set[h] |= 1u << (k - 32 * h);
             }
         int o = block_excl_scan(c, s_warp, &total);
-        if (t < (int)ctas) {
-            unsigned to;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_addr(&s_count[par][rank])), "r"(t));
-            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to), "r"(total) : "memory");
-        }
-        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        if (t < (int)ctas)
+            remote_store_u32(map_rank(smem_addr(&s_count[par][rank]), (unsigned)t), (unsigned)total);
+        cluster_barrier();
         int all = 0;
         for (unsigned k = 0; k < ctas; k++) {
             if (k == rank) o += all;
