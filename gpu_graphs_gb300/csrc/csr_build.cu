@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "csr_build.cuh"
+#include "index.h"
 #include "pinned.cuh"
 #include "scan.cuh"
 
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(BK_BLOCK) k_bucket_plan(BucketPlan *plan, int 
         plan->over_at[b0 + k] = over_at;
         over_at += c[k] > BK_STAGE ? c[k] : 0;
     }
-    const int big = 2 * (total / nb) + 1;
+    const long long big = 2ll * (total / nb) + 1;
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -427,13 +428,9 @@ k_bucket_rows(const BucketPlan *__restrict__ plan, unsigned *packed, int vbits, 
     const unsigned mask = (1u << vbits) - 1u;
     s_cnt[t] = 0;
     __syncthreads();
-    for (int i0 = s; i0 < e; i0 += BK_ILP * BK_BLOCK) {
-        unsigned w[BK_ILP];
-#pragma unroll
-        for (int q = 0; q < BK_ILP; q++) w[q] = i0 + q * BK_BLOCK + t < e ? packed[i0 + q * BK_BLOCK + t] : 0u;
-#pragma unroll
-        for (int q = 0; q < BK_ILP; q++) shared_rank_add(s_cnt, i0 + q * BK_BLOCK + t < e ? (int)(w[q] >> vbits) : -1);
-    }
+    auto load = [&](int i) { return packed[i]; };
+    walk_range<BK_BLOCK, BK_ILP>(s, e, t, load,
+                                 [&](unsigned w, bool in) { shared_rank_add(s_cnt, in ? (int)(w >> vbits) : -1); });
     __syncthreads();
     const int c = s_cnt[t];
     int total;
@@ -445,19 +442,12 @@ k_bucket_rows(const BucketPlan *__restrict__ plan, unsigned *packed, int vbits, 
     __syncthreads();
     const bool staged = e - s <= BK_STAGE;
     int *const over = spare + plan->over_at[b];
-    for (int i0 = s; i0 < e; i0 += BK_ILP * BK_BLOCK) {
-        unsigned w[BK_ILP];
-#pragma unroll
-        for (int q = 0; q < BK_ILP; q++) w[q] = i0 + q * BK_BLOCK + t < e ? packed[i0 + q * BK_BLOCK + t] : 0u;
-#pragma unroll
-        for (int q = 0; q < BK_ILP; q++) {
-            const bool in = i0 + q * BK_BLOCK + t < e;
-            const int pos = shared_rank_add(s_cnt, in ? (int)(w[q] >> vbits) : -1);
-            if (!in) continue;
-            if (staged) s_stage[pos] = (int)(w[q] & mask);
-            else over[pos] = (int)(w[q] & mask);
-        }
-    }
+    walk_range<BK_BLOCK, BK_ILP>(s, e, t, load, [&](unsigned w, bool in) {
+        const int pos = shared_rank_add(s_cnt, in ? (int)(w >> vbits) : -1);
+        if (!in) return;
+        if (staged) s_stage[pos] = (int)(w & mask);
+        else over[pos] = (int)(w & mask);
+    });
     __syncthreads();  // every word has been read
     for (int i = t; i < e - s; i += BK_BLOCK) packed[s + i] = (unsigned)(staged ? s_stage[i] : over[i]);
 }

@@ -1,0 +1,35 @@
+"""CPU: index arithmetic of the kernels at the end of the 32-bit range.
+
+tests/cpp/index_test.cpp includes gpu_graphs_gb300/csrc/index.h (the walks the
+kernels make) and runs them over ranges that end at 2^31 - 1, with traps on
+signed overflow.
+"""
+from __future__ import annotations
+
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+CSRC = ROOT / "gpu_graphs_gb300" / "csrc"
+
+
+def test_walks_at_the_end_of_the_index_range(tmp_path):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("no C++ compiler")
+    exe = tmp_path / "index_test"
+    subprocess.run([cxx, "-std=c++17", "-O1", "-Wall", "-Werror", "-Wno-unknown-pragmas", "-ftrapv", "-I", str(CSRC),
+                    str(ROOT / "tests" / "cpp" / "index_test.cpp"), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
+def test_buckets_are_walked_by_the_checked_loop():
+    """A build by buckets admits inputs whose last bucket ends at 2^31 - 1."""
+    text = (CSRC / "csr_build.cu").read_text()
+    body = text[text.index("k_bucket_rows(const BucketPlan"):text.index("struct BinLists")]
+    assert body.count("walk_range<BK_BLOCK, BK_ILP>(s, e, t,") == 2
+    assert "i0" not in body
