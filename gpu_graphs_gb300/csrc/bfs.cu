@@ -523,6 +523,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
     } else if (gtid == 0) {
         ctrl->t_entry = globaltimer_ns();
     }
+    // a search queued behind one that failed has a barrier in an unknown state:
+    // it ends before its first (the load is on its way during initialisation)
+    const bool failed = threadIdx.x == 0 && ld_relaxed_i32(&ctrl->status) != DEV_OK;
 
     // ---- init ----------------------------------------------------------
     if (!a.resume) {
@@ -548,7 +551,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
             Sel::qb(a, 0)[0] = Sel::mk(__ldg(row + root), __ldg(row + root + 1));
             ctrl->cd[0] = cd_pack(1, (unsigned long long)(__ldg(row + root + 1) - __ldg(row + root)));
         }
-        if (!grid_sync(&ctrl->bar, &ctrl->status, a.timeout_ns, epoch)) return;
+        if (!grid_sync(&ctrl->bar, &ctrl->status, a.timeout_ns, epoch, failed)) return;
         if (root >= 0) {
             if (gtid == 0) a.level[root] = 0;
         } else {
@@ -1030,14 +1033,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
     if (gtid == 0) {
         ctrl->t_end = globaltimer_ns();
         ctrl->trace_len = L < TRACE_CAP ? L : TRACE_CAP;
-        BfsOut o;
-        o.levels = L;
-        o.td_levels = td_levels;
-        o.bu_levels = bu_levels;
-        o.roots = (int)roots;
-        o.reached = reached;
-        o.edges_c = edges_c;
-        *a.out = o;
         ctrl->rs.done = 1;
         ctrl->rs.mode = RESUME_LEVEL;
         for (int i = 0; i < 3; i++) {
@@ -1046,7 +1041,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
         }
         ctrl->fill = 0;
     }
-    grid_exit(&ctrl->bar, &ctrl->t_exit);
+    grid_exit(&ctrl->bar, &ctrl->t_exit, [&] {
+        BfsOut o;
+        o.levels = L;
+        o.td_levels = td_levels;
+        o.bu_levels = bu_levels;
+        o.roots = (int)roots;
+        o.reached = reached;
+        o.edges_c = edges_c;
+        publish_out(a, o);
+    });
 }
 
 template <int BLOCK, typename RT = int>
@@ -1504,7 +1508,7 @@ int bfs_run(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const int *d_r
         else e = cudaMemcpyAsync(w.roots, &single_root, sizeof(int), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // single_root lives on this stack frame
     }
-    w.h_ctrl->out.levels = -1;  // overwritten by a search that ends
+    w.h_ctrl->out.levels = -1;  // overwritten by a search that ends with all of its CTAs (publish_out)
     if (e == cudaSuccess) e = cudaEventRecord(w.ev0, st);
     int launches = bfs_launches_per_search(g, p);
     if (p.per_level_launch == 2) {

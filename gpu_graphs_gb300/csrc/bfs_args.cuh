@@ -72,6 +72,13 @@ struct RowSel<long long> {
 template <typename RT>
 using BndT = typename RowSel<RT>::B;
 
+// The results of a search, from the last CTA out of it (grid_exit): a search that
+// left a status other than DEV_OK has none, which is how the host sees it.
+__device__ __forceinline__ void publish_out(const BfsArgs &a, const BfsOut &o)
+{
+    if (ld_relaxed_i32(&a.ctrl->status) == DEV_OK) *a.out = o;
+}
+
 // The label-correcting kernel (bfs_relax.cu), queued after a grid launch
 // with may_yield set: it finishes a search the grid launch parked.
 cudaError_t bfs_relax_launch(const BfsArgs &args, cudaStream_t st, int max_ctas);

@@ -124,20 +124,8 @@ __device__ __forceinline__ void rx_close(const BfsArgs &a, const BfsResume &rs, 
     }
     if (!grid_sync(&ctrl->bar, &ctrl->status, a.timeout_ns, epoch)) return;
     if (gtid == 0) {
-        const int levels = ctrl->rx_max + 1;
-        BfsOut o;
-        o.levels = levels;
-        o.td_levels = levels - rs.bu_levels;
-        o.bu_levels = rs.bu_levels;
-        o.roots = (int)rs.roots;
-        o.reached = rs.reached + cd_count(cd0) + ctrl->rx_reached;
-        o.edges_c = rs.edges_c + cd_degree(cd0) + ctrl->rx_edges;
-        *a.out = o;
         ctrl->t_end = globaltimer_ns();
         ctrl->trace_len = tl < TRACE_CAP ? tl : TRACE_CAP;
-        ctrl->rx_max = 0;
-        ctrl->rx_reached = 0;
-        ctrl->rx_edges = 0;
         for (int i = 0; i < 3; i++) {
             ctrl->cd[i] = 0;
             ctrl->big[i] = 0;
@@ -146,7 +134,20 @@ __device__ __forceinline__ void rx_close(const BfsArgs &a, const BfsResume &rs, 
         ctrl->rs.done = 1;
         ctrl->rs.mode = RESUME_LEVEL;
     }
-    grid_exit(&ctrl->bar, &ctrl->t_exit);
+    grid_exit(&ctrl->bar, &ctrl->t_exit, [&] {
+        const int levels = ctrl->rx_max + 1;
+        BfsOut o;
+        o.levels = levels;
+        o.td_levels = levels - rs.bu_levels;
+        o.bu_levels = rs.bu_levels;
+        o.roots = (int)rs.roots;
+        o.reached = rs.reached + cd_count(cd0) + ctrl->rx_reached;
+        o.edges_c = rs.edges_c + cd_degree(cd0) + ctrl->rx_edges;
+        publish_out(a, o);
+        ctrl->rx_max = 0;
+        ctrl->rx_reached = 0;
+        ctrl->rx_edges = 0;
+    });
 }
 
 template <typename RT>

@@ -262,7 +262,9 @@ enum DevStatus : int {
 // status while waiting also returns false, so every CTA leaves the kernel
 // shortly after the first one gives up.  grid_exit() (called once by every
 // CTA at the end of a successful launch) lets the last CTA out reset the
-// counters for the next launch.
+// counters for the next launch; only that CTA knows that none gave up (another
+// one's wait may run out in the very barrier that this one has passed), so what
+// tells the host of success is written there.
 struct GridBarrier {
     unsigned count;
     unsigned exit;
@@ -273,13 +275,16 @@ __device__ __forceinline__ void red_release_add(unsigned *p, unsigned v)
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// leave (thread 0's): do not wait, nor arrive; the CTA gets false.
 __device__ __forceinline__ bool grid_sync(GridBarrier *bar, int *status, unsigned long long timeout_ns,
-                                          unsigned &epoch)
+                                          unsigned &epoch, bool leave = false)
 {
     __shared__ int s_ok;
     __syncthreads();
     ++epoch;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && leave) {
+        s_ok = 0;
+    } else if (threadIdx.x == 0) {
         const unsigned target = epoch * gridDim.x;
         red_release_add(&bar->count, 1u);
         int ok = 1;
@@ -307,20 +312,27 @@ __device__ __forceinline__ bool grid_sync(GridBarrier *bar, int *status, unsigne
     return s_ok != 0;
 }
 
-// Count this CTA out; the last one resets the barrier for the next launch
-// and, if t_exit is given, stamps %globaltimer there.
-__device__ __forceinline__ void grid_exit(GridBarrier *bar, unsigned long long *t_exit = nullptr)
+// Count this CTA out; in the last one, thread 0 calls last(), resets the barrier
+// for the next launch and stamps %globaltimer in *t_exit.
+template <typename F>
+__device__ __forceinline__ void grid_exit(GridBarrier *bar, unsigned long long *t_exit, F last)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned old = atomicAdd(&bar->exit, 1u);
         if (old == gridDim.x - 1) {
+            last();
             bar->count = 0;
             bar->exit = 0;
-            if (t_exit) *t_exit = globaltimer_ns();
+            *t_exit = globaltimer_ns();
             __threadfence();
         }
     }
+}
+
+__device__ __forceinline__ void grid_exit(GridBarrier *bar, unsigned long long *t_exit)
+{
+    grid_exit(bar, t_exit, [] {});
 }
 
 }  // namespace gbfs

@@ -4,6 +4,9 @@
 // the grid barrier: CTA 0's wait (the same grid_sync every persistent kernel
 // of the engine uses) must run out after timeout_ms, record DEV_TIMEOUT and
 // return, leaving the CUDA context usable.  Nothing faults, traps or hangs.
+//
+// And a mark on a graph's control block, as left by a search in which some
+// CTA's wait ran out: the next search has to report and clear it.
 #include "graph.cuh"
 
 using namespace gbfs;
@@ -42,4 +45,15 @@ extern "C" int gbfs_selftest_wait_timeout(int32_t timeout_ms)
     if (e != cudaSuccess) return cuda_fail(e, "wait probe");
     if (h.status == DEV_TIMEOUT && h.passed == 0) return fail(GBFS_ERR_TIMEOUT, "bounded wait ran out as expected");
     return fail(GBFS_ERR_CUDA, "bounded wait did not report a timeout");
+}
+
+extern "C" int gbfs_selftest_mark_timeout(gbfs_graph *g)
+{
+    if (!g) return fail(GBFS_ERR_INVALID_ARG, "graph is NULL");
+    std::lock_guard<std::mutex> lk(g->mu);
+    if (!g->work.ctrl) return fail(GBFS_ERR_INVALID_ARG, "the graph has not been searched yet");
+    const int status = DEV_TIMEOUT;
+    cudaError_t e = cudaMemcpyAsync(&g->work.ctrl->status, &status, sizeof(int), cudaMemcpyHostToDevice, g->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    return e == cudaSuccess ? GBFS_OK : cuda_fail(e, "status mark");
 }

@@ -338,6 +338,12 @@ int gbfs_exclusive_scan_i32_noalloc(const int32_t *d_in, int64_t *d_out,
  * and the context is still usable; any other status is a failure.
  */
 int gbfs_selftest_wait_timeout(int32_t timeout_ms);
+/*
+ * Marks g (searched before) as if a wait of its last search had run out
+ * unnoticed: the next single-source search of it has to return
+ * GBFS_ERR_TIMEOUT, and the one after that to succeed.
+ */
+int gbfs_selftest_mark_timeout(gbfs_graph *g);
 
 /* ---- file format and workload generators ------------------------------ */
 /*
