@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_bfs_small(BfsArgs a)
                 b[i] = sh.row[v];
                 d[i] = sh.row[v + 1] - b[i];
             }
+            __syncwarp();  // every lane has read the word
             if (lane == (unsigned)i && nw) {
                 sh.visited[v >> 5] |= nw;
                 sh.fresh[v >> 5] = 0;

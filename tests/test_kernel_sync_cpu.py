@@ -47,3 +47,11 @@ def test_remote_shared_memory_lies_between_cluster_barriers(name):
     remote = [m.start() for m in REMOTE.finditer(body)]
     assert barriers and barriers[0] < remote[0], "no cluster barrier before the first remote access"
     assert barriers[-1] > remote[-1], "no cluster barrier after the last remote access"
+
+
+def test_small_search_reads_a_word_of_new_vertices_before_it_is_cleared():
+    """All lanes of a warp read the word that one of them clears."""
+    body = kernels()["k_bfs_small"]
+    read = body.index("= sh.fresh[v >> 5]")
+    clear = body.index("sh.fresh[v >> 5] = 0")
+    assert read < clear and "__syncwarp()" in body[read:clear]
