@@ -1305,7 +1305,7 @@ __global__ void k_check_sym(const RT *__restrict__ row, const int *__restrict__ 
         const RT last = row[v + 1];
         RT lo = row[v], hi = last;
         while (lo < hi) {
-            const RT mid = (lo + hi) >> 1;
+            const RT mid = idx_mid(lo, hi);
             if (col[mid] < u) lo = mid + 1; else hi = mid;
         }
         if (lo >= last || col[lo] != u) flags[1] = 1;

@@ -13,6 +13,37 @@
 
 namespace gbfs {
 
+// i + k, which may lie past the type's largest value: then it is before no end.
+template <typename T>
+GBFS_HD T idx_add(T i, int k)
+{
+    if constexpr (sizeof(T) == sizeof(int)) return (T)((unsigned)i + (unsigned)k);
+    else return i + k;
+}
+
+// i < e for an entry index i from idx_add and a range's end e (less than 2^31 apart).
+template <typename T>
+GBFS_HD bool idx_before(T i, T e)
+{
+    if constexpr (sizeof(T) == sizeof(int)) return (int)((unsigned)e - (unsigned)i) > 0;
+    else return i < e;
+}
+
+// min(i + k, e)
+template <typename T>
+GBFS_HD T idx_end(T i, int k, T e)
+{
+    const T x = idx_add(i, k);
+    return idx_before(x, e) ? x : e;
+}
+
+// (lo + hi) / 2 for 0 <= lo <= hi
+template <typename T>
+GBFS_HD T idx_mid(T lo, T hi)
+{
+    return lo + (hi - lo) / 2;
+}
+
 // Thread t's part of the entries [s, e), BLOCK threads wide and ILP at a time:
 // v = load(i) of each entry i, then use(v, true), and use(0, false) past the end,
 // so that all threads make the same calls of use.

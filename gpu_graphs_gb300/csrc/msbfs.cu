@@ -26,6 +26,7 @@
 #include <cstddef>
 
 #include "blockq.cuh"
+#include "index.h"
 #include "msbfs.cuh"
 #include "pinned.cuh"
 
@@ -378,13 +379,13 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) k_msbfs(MsArgs a)
                 unsigned long long acc = 0;
                 if (need) {
                     const int v0 = __ldg(a.pcol + b);
-                    const int v1 = b + 1 < e ? __ldg(a.pcol + b + 1) : v0;
-                    const int v2 = b + 2 < e ? __ldg(a.pcol + b + 2) : v0;
-                    const int v3 = b + 3 < e ? __ldg(a.pcol + b + 3) : v0;
+                    const int v1 = e - b > 1 ? __ldg(a.pcol + b + 1) : v0;
+                    const int v2 = e - b > 2 ? __ldg(a.pcol + b + 2) : v0;
+                    const int v3 = e - b > 3 ? __ldg(a.pcol + b + 3) : v0;
                     acc = Fc[v0] | Fc[v1] | Fc[v2] | Fc[v3];
                 }
-                b += 4;
-                const int rest = (acc & need) != need && b < e ? e - b : 0;
+                const int rest = (acc & need) != need && e - b > 4 ? e - b - 4 : 0;
+                if (rest) b += 4;
                 const int incl = warp_incl_scan(rest), excl = incl - rest;
                 const int T = __shfl_sync(FULL, incl, 31);
                 if (T) {
@@ -456,12 +457,12 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) k_msbfs(MsArgs a)
                     const unsigned long long rneed = __shfl_sync(FULL, need, sl);
                     const unsigned long long rvu = __shfl_sync(FULL, vu, sl);
                     unsigned long long acc = 0;
-                    for (int i0 = rb; i0 < re; i0 += 128) {
+                    for (int i0 = rb; idx_before(i0, re); i0 = idx_add(i0, 128)) {
                         unsigned long long x = 0;
 #pragma unroll
                         for (int t = 0; t < 4; t++) {
-                            const int i = i0 + t * 32 + (int)lane;
-                            if (i < re) x |= Fc[__ldg(a.pcol + i)];
+                            const int i = idx_add(i0, t * 32 + (int)lane);
+                            if (idx_before(i, re)) x |= Fc[__ldg(a.pcol + i)];
                         }
                         acc |= warp_or64(x);
                         if ((acc & rneed) == rneed) break;
@@ -505,20 +506,20 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) k_msbfs(MsArgs a)
                     const unsigned long long rneed = __shfl_sync(FULL, need, sl);
                     const int rb = __ldg(a.prow + u), re = __ldg(a.prow + u + 1);
                     const unsigned pn = MS_SUB * (unsigned)((re - rb + MS_PIECE - 1) / MS_PIECE);
-                    const int b = rb + j * (MS_PIECE / MS_SUB);
-                    const int e = min(re, b + MS_PIECE / MS_SUB);  // (before b past the row's end: no edges)
+                    const int b = idx_add(rb, j * (MS_PIECE / MS_SUB));
+                    const int e = idx_end(b, MS_PIECE / MS_SUB, re);  // (before b past the row's end: no edges)
                     unsigned long long acc = 0;
                     // skip a piece whose row the others have already covered (one
                     // read, broadcast: the loop below must be warp-uniform)
                     unsigned long long seen = lane == 0 ? ld_relaxed_u64(a.hacc + u) : 0ull;
                     seen = __shfl_sync(FULL, seen, 0);
                     if ((seen & rneed) != rneed) {
-                        for (int i0 = b; i0 < e; i0 += 128) {
+                        for (int i0 = b; idx_before(i0, e); i0 = idx_add(i0, 128)) {
                             unsigned long long x = 0;
 #pragma unroll
                             for (int t = 0; t < 4; t++) {
-                                const int i = i0 + t * 32 + (int)lane;
-                                if (i < e) x |= Fc[__ldg(a.pcol + i)];
+                                const int i = idx_add(i0, t * 32 + (int)lane);
+                                if (idx_before(i, e)) x |= Fc[__ldg(a.pcol + i)];
                             }
                             acc |= warp_or64(x);
                             if ((acc & rneed) == rneed) break;

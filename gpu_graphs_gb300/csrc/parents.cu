@@ -30,6 +30,7 @@
 
 #include "bfs.cuh"
 #include "common.cuh"
+#include "index.h"
 #include "msbfs.cuh"
 #include "parents.cuh"
 
@@ -52,12 +53,12 @@ __device__ __forceinline__ int warp_min_at(const int *__restrict__ col, RT b, RT
                                            int want, bool sorted, int lane)
 {
     int best = INT_MAX;
-    for (RT i0 = b; i0 < e; i0 += 128) {
+    for (RT i0 = b; idx_before(i0, e); i0 = idx_add(i0, 128)) {
         int u[4], l[4];
 #pragma unroll
         for (int t = 0; t < 4; t++) {
-            const RT i = i0 + t * 32 + lane;
-            u[t] = i < e ? __ldg(col + i) : -1;
+            const RT i = idx_add(i0, t * 32 + lane);
+            u[t] = idx_before(i, e) ? __ldg(col + i) : -1;
         }
 #pragma unroll
         for (int t = 0; t < 4; t++) l[t] = u[t] >= 0 ? __ldg(level + u[t]) : -2;
@@ -108,10 +109,10 @@ __global__ void k_parents_pull_light(const RT *__restrict__ row, const int *__re
             best = INT_MAX;  // stays so for offers, and in a long row: the heavy kernel's
             const RT b = row[v], e = row[v + 1];
             if (e - b <= HEAVY_DEGREE && !is_set(push, lv - 1)) {
-                for (RT i = b; i < e; i += 4) {
+                for (RT i = b; idx_before(i, e); i = idx_add(i, 4)) {
                     int u[4], l[4];
 #pragma unroll
-                    for (int t = 0; t < 4; t++) u[t] = __ldg(col + (i + t < e ? i + t : e - 1));
+                    for (int t = 0; t < 4; t++) u[t] = __ldg(col + idx_end(i, t, e - 1));
 #pragma unroll
                     for (int t = 0; t < 4; t++) l[t] = __ldg(level + u[t]);
 #pragma unroll
@@ -130,12 +131,12 @@ template <int ILP, typename RT>
 __device__ __forceinline__ void warp_offer_by(int u, int lu, const int *__restrict__ col, RT b, RT e,
                                               const int *__restrict__ level, int *parent, int lane)
 {
-    for (RT i0 = b; i0 < e; i0 += 32 * ILP) {
+    for (RT i0 = b; idx_before(i0, e); i0 = idx_add(i0, 32 * ILP)) {
         int v[ILP], l[ILP];
 #pragma unroll
         for (int t = 0; t < ILP; t++) {
-            const RT i = i0 + t * 32 + lane;
-            v[t] = i < e ? __ldg(col + i) : -1;
+            const RT i = idx_add(i0, t * 32 + lane);
+            v[t] = idx_before(i, e) ? __ldg(col + i) : -1;
         }
 #pragma unroll
         for (int t = 0; t < ILP; t++) l[t] = v[t] >= 0 ? __ldg(level + v[t]) : -2;
@@ -174,7 +175,7 @@ __global__ void k_parents_pull_heavy(const RT *__restrict__ row, const int *__re
         const int lv = __ldg(level + pc.x);
         if (lv < 1) continue;  // written by the light kernel, as is level 1
         const RT b = row[pc.x] + (RT)pc.y * MS_PIECE;
-        const RT e = min(row[pc.x + 1], b + MS_PIECE);
+        const RT e = idx_end(b, MS_PIECE, row[pc.x + 1]);
         if (is_set(push, lv)) warp_offer(pc.x, lv, col, b, e, level, parent, lane);
         if (lv == 1 || is_set(push, lv - 1)) continue;
         // an earlier piece of an ascending row has the answer (one read,
@@ -226,7 +227,7 @@ __global__ void k_parents_push(const RT *__restrict__ row, const int *__restrict
         const int lu = __ldg(level + pc.x);
         if (lu < 1) continue;  // unreached, or the source (its offers are in place)
         const RT b = row[pc.x] + (RT)pc.y * MS_PIECE;
-        warp_offer(pc.x, lu, col, b, min(row[pc.x + 1], b + MS_PIECE), level, parent, lane);
+        warp_offer(pc.x, lu, col, b, idx_end(b, MS_PIECE, row[pc.x + 1]), level, parent, lane);
     }
     for (long long u = gw; u < n; u += nw) {
         const int lu = __ldg(level + u);

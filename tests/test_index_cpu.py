@@ -6,6 +6,7 @@ signed overflow.
 """
 from __future__ import annotations
 
+import re
 import shutil
 import subprocess
 
@@ -33,3 +34,21 @@ def test_buckets_are_walked_by_the_checked_loop():
     body = text[text.index("k_bucket_rows(const BucketPlan"):text.index("struct BinLists")]
     assert body.count("walk_range<BK_BLOCK, BK_ILP>(s, e, t,") == 2
     assert "i0" not in body
+
+
+# kernels whose rows may end at 2^31 - 1, and forms of their index arithmetic that
+# leave the type there
+PLAIN = [r"\(lo \+ hi\) *>> *1", r"\+= *(128|32 \* ILP)\b", r"\b(b|rb) \+ (MS_PIECE(?! - 1)|j \* )", r"\bi0 \+ t \* 32"]
+
+
+@pytest.mark.parametrize("name", ["parents.cu", "msbfs.cu"])
+def test_rows_are_walked_by_checked_arithmetic(name):
+    text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+    for pattern in PLAIN:
+        assert not re.search(pattern, text), pattern
+
+
+def test_symmetry_check_halves_without_overflow():
+    text = (CSRC / "csr_build.cu").read_text()
+    body = text[text.index("k_check_sym(const RT"):text.index("k_check_sorted(const RT")]
+    assert "idx_mid(lo, hi)" in body and not re.search(PLAIN[0], body)
