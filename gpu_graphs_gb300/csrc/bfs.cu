@@ -43,6 +43,7 @@
 #include "bfs.cuh"
 #include "bfs_args.cuh"
 #include "blockq.cuh"
+#include "index.h"
 #include "pinned.cuh"
 
 namespace gbfs {
@@ -433,7 +434,7 @@ __device__ __forceinline__ void probe_rows(RT &ia, RT ea, bool &fa, RT &ib, RT e
                                            const unsigned *fc, unsigned lane)
 {
     for (;;) {
-        const bool aa = ia < ea && !fa, ab = ib < eb && !fb;
+        const bool aa = idx_before(ia, ea) && !fa, ab = idx_before(ib, eb) && !fb;
         const unsigned ma = __ballot_sync(FULL, aa), mb = __ballot_sync(FULL, ab);
         if (!(ma | mb)) return;
         if (__popc(ma) + __popc(mb) <= COOP_ROWS) {
@@ -449,10 +450,10 @@ __device__ __forceinline__ void probe_rows(RT &ia, RT ea, bool &fa, RT &ib, RT e
                     const RT ri = __shfl_sync(FULL, isb ? ib : ia, sl);
                     const RT re = __shfl_sync(FULL, isb ? eb : ea, sl);
                     bool found = false;
-                    for (RT i0 = ri; i0 < re && !found; i0 += 32) {
-                        const RT i = i0 + (RT)lane;
+                    for (RT i0 = ri; idx_before(i0, re) && !found; i0 = idx_add(i0, 32)) {
+                        const RT i = idx_add(i0, (int)lane);
                         unsigned hit = 0;
-                        if (i < re) {
+                        if (idx_before(i, re)) {
                             const int u = __ldg(bcol + i);
                             hit = (fc[u >> 5] >> (u & 31)) & 1u;
                         }
@@ -469,8 +470,8 @@ __device__ __forceinline__ void probe_rows(RT &ia, RT ea, bool &fa, RT &ib, RT e
         int ua[PROBE], ub[PROBE];
 #pragma unroll
         for (int t = 0; t < PROBE; t++) {
-            ua[t] = (aa && ia + t < ea) ? __ldg(bcol + ia + t) : -1;
-            ub[t] = (ab && ib + t < eb) ? __ldg(bcol + ib + t) : -1;
+            ua[t] = (aa && ea - ia > t) ? __ldg(bcol + ia + t) : -1;
+            ub[t] = (ab && eb - ib > t) ? __ldg(bcol + ib + t) : -1;
         }
         unsigned ga = 0, gb = 0;
 #pragma unroll
@@ -478,8 +479,8 @@ __device__ __forceinline__ void probe_rows(RT &ia, RT ea, bool &fa, RT &ib, RT e
             if (ua[t] >= 0) ga |= fc[ua[t] >> 5] >> (ua[t] & 31);
             if (ub[t] >= 0) gb |= fc[ub[t] >> 5] >> (ub[t] & 31);
         }
-        if (aa) { if (ga & 1u) fa = true; else ia += PROBE; }
-        if (ab) { if (gb & 1u) fb = true; else ib += PROBE; }
+        if (aa) { if (ga & 1u) fa = true; else ia = idx_add(ia, PROBE); }
+        if (ab) { if (gb & 1u) fb = true; else ib = idx_add(ib, PROBE); }
     }
 }
 
@@ -888,7 +889,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
                                 my_deg += (unsigned long long)(brow == row ? re[h] - rb[h]
                                                                            : __ldg(row + v + 1) - __ldg(row + v));
                             }
-                            const bool defer = v >= 0 && !f && rb[h] + skip < re[h];
+                            const bool defer = v >= 0 && !f && re[h] - rb[h] > skip;
                             const unsigned dm = __ballot_sync(FULL, defer);
                             if (defer) {
                                 const int slotd = dn + __popc(dm & lanemask_lt());
@@ -984,8 +985,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
                         if (pb >= 0) hb |= fc[pb >> 5] >> (pb & 31);
                         if (qb >= 0) hb |= fc[qb >> 5] >> (qb & 31);
                         bool fa = ha & 1u, fb = hb & 1u;
-                        ia += two ? 2 : 1;
-                        ib += two ? 2 : 1;
+                        ia = idx_add(ia, two ? 2 : 1);
+                        ib = idx_add(ib, two ? 2 : 1);
                         probe_rows(ia, ea, fa, ib, eb, fb, a.bcol, fc, lane);
                         // the next frontier's out-edges (for the direction rule): the
                         // probed in-degree when in-edges are the out-edges

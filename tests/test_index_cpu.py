@@ -48,6 +48,13 @@ def test_rows_are_walked_by_checked_arithmetic(name):
         assert not re.search(pattern, text), pattern
 
 
+def test_bottom_up_probes_stay_in_range():
+    text = re.sub(r"//[^\n]*", "", (CSRC / "bfs.cu").read_text())
+    body = text[text.index("void probe_rows("):text.index("k_bfs(BfsArgs a)")]
+    assert not re.search(r"\+= *(32|PROBE)\b|\bi[ab0]? *\+ *\(?(t|RT)\b[^;]*<|\bi0? < re\b", body)
+    assert "+ skip < re" not in text and "+= two" not in text
+
+
 def test_symmetry_check_halves_without_overflow():
     text = (CSRC / "csr_build.cu").read_text()
     body = text[text.index("k_check_sym(const RT"):text.index("k_check_sorted(const RT")]
