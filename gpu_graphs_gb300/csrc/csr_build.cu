@@ -1259,7 +1259,8 @@ __global__ void k_validate_csr(const RT *__restrict__ row, const int *__restrict
 
 // Calls f(e, u, in) for the m entries e of the rows, u the entry's row: a warp
 // takes EDGE_CHUNK consecutive entries at a time, 32 a step (in: the lane has
-// one), so the work does not follow the rows' lengths.  All lanes call f.
+// one), so the work does not follow the rows' lengths.  All lanes call f; a step
+// in which it returns true (to all of them) ends the warp's walk.
 constexpr int EDGE_CHUNK = 1024;
 
 template <typename RT, typename F>
@@ -1289,27 +1290,56 @@ __device__ __forceinline__ void for_edges(const RT *__restrict__ row, int n, int
                 if (mine < 0 && k < 32) mine = w + k;
                 if (!__any_sync(FULL, in && mine < 0)) break;
             }
-            f(e, mine, in);
+            if (f(e, mine, in)) return;
             u = __shfl_sync(FULL, mine, (int)(min(end, e0 + 32) - e0) - 1);
         }
     }
 }
 
-// Symmetry check on sorted rows: every (u,v) has (v,u).
+// Whether sorted row v has an entry u.
+template <typename RT>
+__device__ __forceinline__ bool row_has(const RT *__restrict__ row, const int *__restrict__ col, int v, int u)
+{
+    const RT last = row[v + 1];
+    RT lo = row[v], hi = last;
+    while (lo < hi) {
+        const RT mid = idx_mid(lo, hi);
+        if (col[mid] < u) lo = mid + 1; else hi = mid;
+    }
+    return lo < last && col[lo] == u;
+}
+
+// Symmetry check on sorted rows: every (u,v) has (v,u).  A warp stops at its first
+// entry without, which in a directed graph is soon enough (looking at the flag for
+// what others have found costs more, as all warps' looks queue up in L2).
 template <typename RT>
 __global__ void k_check_sym(const RT *__restrict__ row, const int *__restrict__ col, int n, int64_t m, int *flags)
 {
     for_edges(row, n, m, [&](int64_t e, int u, bool in) {
-        if (!in || ld_relaxed_i32(flags + 1)) return;
-        const int v = col[e];
-        const RT last = row[v + 1];
-        RT lo = row[v], hi = last;
-        while (lo < hi) {
-            const RT mid = idx_mid(lo, hi);
-            if (col[mid] < u) lo = mid + 1; else hi = mid;
-        }
-        if (lo >= last || col[lo] != u) flags[1] = 1;
+        const bool missing = in && !row_has(row, col, col[e], u);
+        if (missing) flags[1] = 1;
+        return __any_sync(FULL, missing) != 0;
     });
+}
+
+// The same with a thread per row (up to its first entry without), for graphs without rows of more than
+// HEAVY_DEGREE entries, where finding each entry's row costs more than uneven
+// rows: uniform random, 4 M vertices, 64 M entries: 1.76 ms against 2.33 by
+// entries, a grid of 3000 x 3000 0.10 against 0.30; with a hub among the rows it
+// would be the longest row's time (RMAT-20: 100 ms against 1.1).
+template <typename RT>
+__global__ void k_check_sym_rows(const RT *__restrict__ row, const int *__restrict__ col, int n, int *flags)
+{
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += stride) {
+        const RT b = row[u], e = row[u + 1];
+        bool missing = false;
+        for (RT i = b; i < e && !missing; i++) missing = !row_has(row, col, col[i], (int)u);
+        if (missing) {
+            flags[1] = 1;
+            return;
+        }
+    }
 }
 
 // Rows ascend where every descent of the column array is at a row's start:
@@ -1857,7 +1887,11 @@ int csr_check_symmetric(DeviceCsr &c, cudaStream_t st, bool &sym, std::string &e
             if (rc) goto done;
             col = copy;
         }
-        if (c.wide) k_check_sym<<<grid, 256, 0, st>>>((const long long *)c.row64, col, c.n, c.m, flags);
+        const int rows = grid_for(c.n, 256, 152 * 8);
+        const bool by_rows = c.nheavy == 0;
+        if (c.wide && by_rows) k_check_sym_rows<<<rows, 256, 0, st>>>((const long long *)c.row64, col, c.n, flags);
+        else if (c.wide) k_check_sym<<<grid, 256, 0, st>>>((const long long *)c.row64, col, c.n, c.m, flags);
+        else if (by_rows) k_check_sym_rows<<<rows, 256, 0, st>>>((const int *)c.row, col, c.n, flags);
         else k_check_sym<<<grid, 256, 0, st>>>((const int *)c.row, col, c.n, c.m, flags);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(h, flags, 8, cudaMemcpyDeviceToHost, st));
@@ -1910,6 +1944,7 @@ __global__ void k_in_scatter(const int *__restrict__ row, const int *__restrict_
 {
     for_edges(row, n, m, [&](int64_t e, int u, bool in) {
         if (in) tcol[atomicAdd(&cursor[col[e]], 1)] = u;
+        return false;
     });
 }
 
