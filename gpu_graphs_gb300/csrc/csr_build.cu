@@ -1257,6 +1257,29 @@ __global__ void k_validate_csr(const RT *__restrict__ row, const int *__restrict
     }
 }
 
+// The first of 32 rows among which entry e's is, for a w with row[w] <= e: rows
+// w + 1 to the one sought are empty or end before e.  Strides of 32, 32^2, ...
+// rows as far as that is too few, then back down, 32 looks at once: a gap of g
+// rows takes about 2 log32(g / 32) + 1 round trips (32 rows at a time, a gap of 5 M
+// empty rows held one warp for 156,000).  The whole warp calls it.
+template <typename RT>
+__device__ __forceinline__ int skip_empty_rows(const RT *__restrict__ row, int n, int w, int64_t e)
+{
+    int64_t at = w, stride = 32;
+    for (;; stride *= 32) {
+        const int64_t x = at + (lane_id() + 1) * stride;
+        const int k = __popc(__ballot_sync(FULL, x <= n && (int64_t)row[x <= n ? x : 0] <= e));
+        at += k * stride;
+        if (k < 32) break;
+    }
+    while (stride > 32) {
+        stride /= 32;
+        const int64_t x = at + (lane_id() + 1) * stride;
+        at += stride * __popc(__ballot_sync(FULL, x <= n && (int64_t)row[x <= n ? x : 0] <= e));
+    }
+    return (int)at;
+}
+
 // Calls f(e, u, in) for the m entries e of the rows, u the entry's row: a warp
 // takes EDGE_CHUNK consecutive entries at a time, 32 a step (in: the lane has
 // one), so the work does not follow the rows' lengths.  All lanes call f; a step
@@ -1280,15 +1303,19 @@ __device__ __forceinline__ void for_edges(const RT *__restrict__ row, int n, int
             const int64_t e = e0 + lane;
             const bool in = e < end;
             int mine = -1;
-            for (int w = u;; w += 32) {  // 32 rows' ends at a time
+            for (int w = u;;) {  // 32 rows' ends at a time
                 const int64_t at = (int64_t)w + 1 + lane, r = at <= n ? (int64_t)row[at] : INT64_MAX;
                 int k = 0;  // of them at or before e
 #pragma unroll
                 for (int s = 16; s > 0; s >>= 1)
                     if (__shfl_sync(FULL, r, k + s - 1) <= e) k += s;
                 if (__shfl_sync(FULL, r, k) <= e) ++k;
-                if (mine < 0 && k < 32) mine = w + k;
-                if (!__any_sync(FULL, in && mine < 0)) break;
+                const bool hit = mine < 0 && k < 32;
+                if (hit) mine = w + k;
+                const unsigned left = __ballot_sync(FULL, in && mine < 0);
+                if (!left) break;
+                w += 32;
+                if (!__any_sync(FULL, in && hit)) w = skip_empty_rows(row, n, w, e0 + __ffs(left) - 1);
             }
             if (f(e, mine, in)) return;
             u = __shfl_sync(FULL, mine, (int)(min(end, e0 + 32) - e0) - 1);
