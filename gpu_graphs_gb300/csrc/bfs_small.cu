@@ -35,10 +35,8 @@ namespace gbfs {
 
 namespace {
 
-constexpr int SM_CTAS = 16;      // CTAs of the largest cluster
-// vertices per CTA: 2^10 up to 2^SM_MAX_LOGS
-constexpr int SM_MAX_LOGS = 13;
-constexpr int SM_LONG = 512;     // rows the whole CTA walks
+constexpr int SM_CTAS = SMALL_CTAS;  // CTAs of the largest cluster
+constexpr int SM_LONG = SMALL_LONG;  // rows the whole CTA walks
 constexpr int SM_TRACE = 64;     // trace rows held in shared memory
 
 // The longest row is more than 16 times the mean one.
@@ -299,10 +297,12 @@ cudaError_t small_launch(const BfsArgs &args, cudaStream_t st)
 template <typename RT>
 cudaError_t small_launch_n(const BfsArgs &a, cudaStream_t st)
 {
-    if (a.n <= SM_CTAS << 10) return small_launch<10, 1024, RT>(a, st);
-    if (a.n <= SM_CTAS << 11) return small_launch<11, 1024, RT>(a, st);
-    if (a.n <= SM_CTAS << 12) return small_launch<12, 1024, RT>(a, st);
-    return small_launch<13, 1024, RT>(a, st);
+    switch (small_part_log(a.n)) {
+    case 10: return small_launch<10, 1024, RT>(a, st);
+    case 11: return small_launch<11, 1024, RT>(a, st);
+    case 12: return small_launch<12, 1024, RT>(a, st);
+    default: return small_launch<SMALL_MAX_LOG, 1024, RT>(a, st);
+    }
 }
 
 }  // namespace
@@ -317,10 +317,22 @@ cudaError_t small_launch_n(const BfsArgs &a, cudaStream_t st)
 //   edges a vertex 45 and 75, 16: 46 and 67, 32: 56 and 50; 131,072, 15 a
 //   vertex: 72 and 101; RMAT: 16,384 vertices, 426 K edges: 34 and 42; 32,768,
 //   530 K: 41 and 49; 65,536: 381 K 46 and 48, 740 K 52 and 50.
+// Nor a graph of which one CTA would walk too much, as every level is the time of
+// its slowest CTA and the grid kernel deals rows to all SMs: the costliest part of
+// small_row_cost, and the longest row.  (us here and in the grid kernel) top-down:
+// uniform random, 16,000 vertices, 261 K entries in a part: 53 and 84, 517 K with
+// rows of 512 among them: 174 and 127; 2,000, 820 K: 348 and 87; a clique of 1,000
+// of 131,000 vertices: 408 and 96; a star of 20,000: 24 and 24, of 131,000: 90 and
+// 27.  Direction-optimising: uniform random, 16,000 vertices, 66 K in a part: 31 and
+// 37, 131 K 39 and 37; 131,072, 66 K: 66 and 70, 132 K 74 and 58; RMAT, 16,384
+// vertices, a cost of some 73 K: 33 and 39, 117 K 43 and 38; 131,072, 80 K: 61 and
+// 55; a star of 5,000: 14 and 19, of 20,000: 25 and 20.
 bool bfs_small(const DeviceCsr &g, const gbfs_params &p)
 {
     if (p.per_level_launch || p.direction == GBFS_DIR_BOTTOMUP || bfs_relax_tail(g, p)) return false;
-    if (g.n > SM_CTAS << SM_MAX_LOGS || g.m > 4 << 20) return false;
+    if (g.n > SMALL_MAX_N || g.m > 4 << 20 || g.max_degree > 1 << 14) return false;
+    const int64_t most = p.direction == GBFS_DIR_TOPDOWN ? 250000 : g.n <= SMALL_MAX_N / 2 ? 100000 : 70000;
+    if (g.part_cost > most) return false;
     if (p.direction == GBFS_DIR_TOPDOWN) return true;
     return small_skewed(g.max_degree, g.n, g.m) ? g.m <= 1 << 19 : g.m <= 20 * (int64_t)g.n;
 }

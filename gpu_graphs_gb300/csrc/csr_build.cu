@@ -1190,13 +1190,13 @@ __global__ void k_compact(const RT *__restrict__ row, const RT *__restrict__ row
 
 template <typename RT>
 __global__ void k_finalize(const RT *__restrict__ row, int n, unsigned *zmask, int *maxdeg,
-                           unsigned long long *nonisolated, unsigned *nover4)
+                           unsigned long long *nonisolated, unsigned *nover4, unsigned long long *part, int part_log)
 {
     __shared__ unsigned long long s_red[32];
     __shared__ int s_max[32];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     // non-isolated rows, and rows of more than four entries in the high half
-    unsigned long long mine = 0;
+    unsigned long long mine = 0, cost = 0;
     int mx = 0;
     const int W = (n + 31) >> 5;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < (int64_t)W * 32;
@@ -1206,7 +1206,12 @@ __global__ void k_finalize(const RT *__restrict__ row, int n, unsigned *zmask, i
         unsigned z = __ballot_sync(FULL, d == 0);  // out-of-range bits count as zero-degree
         if (lane_id() == 0) zmask[v >> 5] = z;
         mine += (d > 0 ? 1ull : 0ull) + (d > 4 ? 1ull << 32 : 0ull);
+        cost += (unsigned long long)small_row_cost(d);
         mx = max(mx, d);
+    }
+    if (part_log > 0) {  // (the grid covers so small a graph in one go: a CTA's vertices are of one part)
+        cost = block_sum(cost, s_red);
+        if (threadIdx.x == 0 && cost) atomicAdd(part + ((blockIdx.x * blockDim.x) >> part_log), cost);
     }
     unsigned long long t = block_sum(mine, s_red);
     if (threadIdx.x == 0 && t) {
@@ -1598,15 +1603,22 @@ template <typename RT>
 int finalize_t(DeviceCsr &out, const RT *row, cudaStream_t st, std::string &err)
 {
     int rc = GBFS_OK;
-    struct Res { unsigned long long nonisolated; int maxdeg; unsigned nheavy, nover4, pad; };
+    struct Res {
+        unsigned long long nonisolated;
+        int maxdeg;
+        unsigned nheavy, nover4, pad;
+        unsigned long long part[SMALL_CTAS];
+    };
     Pinned<Res> h;
     NEED_PINNED(h);
     Res *d_res = nullptr;
     const int W = (out.n + 31) / 32;
     CK(cudaMalloc(&d_res, sizeof(Res)));
     CK(cudaMemsetAsync(d_res, 0, sizeof(Res), st));
+    static_assert(SMALL_MAX_N <= 256 * 152 * 16, "one pass of k_finalize's grid covers a small graph");
     k_finalize<<<grid_for((int64_t)W * 32, 256), 256, 0, st>>>(row, out.n, out.zmask, &d_res->maxdeg,
-                                                                &d_res->nonisolated, &d_res->nover4);
+                                                                &d_res->nonisolated, &d_res->nover4, d_res->part,
+                                                                out.n <= SMALL_MAX_N ? small_part_log(out.n) : 0);
     CK(cudaGetLastError());
     k_heavy_list<<<grid_for(out.n, 1024, 152 * 4), 1024, 0, st>>>(row, out.n, out.heavy, &d_res->nheavy);
     CK(cudaGetLastError());
@@ -1616,6 +1628,7 @@ int finalize_t(DeviceCsr &out, const RT *row, cudaStream_t st, std::string &err)
     out.nonisolated = (int64_t)h->nonisolated;
     out.nover4 = (int32_t)h->nover4;
     out.nheavy = (int32_t)h->nheavy;
+    out.part_cost = (int64_t)*std::max_element(h->part, h->part + SMALL_CTAS);
 done:
     if (d_res) cudaFree(d_res);
     return rc;

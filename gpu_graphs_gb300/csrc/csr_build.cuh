@@ -24,6 +24,7 @@ struct DeviceCsr {
     unsigned *zmask = nullptr; // (n+31)/32
     int32_t max_degree = 0;
     int64_t nonisolated = 0;
+    int64_t part_cost = 0;     // graphs of up to SMALL_MAX_N vertices: largest sum of small_row_cost in a part
     int *heavy = nullptr;      // vertices of out-degree > HEAVY_DEGREE (any order)
     int32_t nheavy = 0;
     // each row's first and second entries, -1 where the row is shorter (with
@@ -59,6 +60,29 @@ struct DeviceCsr {
     int32_t ntpieces = 0;
     bool tpieces_built = false;
 };
+
+// Graphs that one thread-block cluster may search (bfs_small.cu): the cluster's
+// CTAs own aligned parts of 2^small_part_log vertices each.
+constexpr int SMALL_CTAS = 16;
+constexpr int SMALL_MAX_LOG = 13;
+constexpr int SMALL_MAX_N = SMALL_CTAS << SMALL_MAX_LOG;
+constexpr int SMALL_LONG = 512;  // rows that the whole CTA walks, one after another
+
+inline int small_part_log(int32_t n)
+{
+    int l = 10;
+    while (SMALL_CTAS << l < n) l++;
+    return l;
+}
+
+// What walking a row of d entries costs a CTA there, in entries of short rows
+// (about 0.1 ns): a long row is a step of its own (0.35 us), and has more
+// neighbours per word to mark.
+__host__ __device__ inline long long small_row_cost(int d)
+{
+    if (d < SMALL_LONG) return d;
+    return 3ll * d > 3500 ? 3ll * d : 3500;
+}
 
 // Rows longer than this are walked by a whole warp in multi-source passes.
 constexpr int HEAVY_DEGREE = 64;
