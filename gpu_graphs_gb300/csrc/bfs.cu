@@ -66,8 +66,11 @@ constexpr int BU_DEF = QCAP;
 // now: uniform random of 1 M vertices 156 -> 106 us, 200,000 vertices 103 -> 81,
 // 3 M vertices 228 -> 194, RMAT 50 -> 50 and 66 -> 63.  Above the line the queue
 // may hold hubs, whose rows would be put off to a pass of their own (RMAT-22
-// with rows always: 95 -> 118 us).
+// with rows always: 95 -> 118 us).  Edges are balanced too where rows of more than
+// BALANCE_ROW entries would not be put off: big_degree set to 2^20, a queue of
+// 2,000 rows, one of them of 60,000 entries: 1,279 us in one warp, 66 balanced.
 constexpr unsigned long long BALANCE_DEGREE = 64;
+constexpr int BALANCE_ROW = 1024;
 constexpr unsigned long long BMTD_EDGES = 65536;  // top-down from the bitmap up to this many frontier edges
 // Long searches on graphs whose largest out-degree is at most
 // RELAX_MAX_DEGREE (meshes, grids, road networks: thousands of levels of
@@ -711,7 +714,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_bfs(BfsArgs a)
             const float growth = fmaxf(1.f, (float)mf / (float)(prev_mf ? prev_mf : 1ull));
             const bool likely_bu = (float)mf * growth * (float)a.alpha > (float)m_u;
             unsigned *fnw = a.direction == GBFS_DIR_OPTIMIZING && brow && likely_bu ? fn : nullptr;
-            const bool balance = nf <= (unsigned long long)SEG && mf > BALANCE_DEGREE * nf;
+            const bool balance = nf <= (unsigned long long)SEG && mf > a.balance_degree * nf;
             if (from_bitmap) {
                 bitmap_expand(fc, W, (long long)nf, a, nl, q, cnt_next, qn, qbn, my_deg, &ctrl->big[L % 3], gwarp, nwarps,
                               lane, fnw);
@@ -1276,6 +1279,7 @@ BfsArgs make_args(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const in
     a.direction = p.direction;
     a.has_big = g.max_degree >= a.big_degree ? 1 : 0;
     a.max_degree = std::max(1, (int)g.max_degree);
+    a.balance_degree = std::min(a.max_degree, a.big_degree) > BALANCE_ROW ? 0 : BALANCE_DEGREE;
     a.may_yield = 0;
     a.yield_level = RELAX_YIELD_LEVEL;
     a.yield_max_f = RELAX_ENTER_F;

@@ -40,6 +40,7 @@ struct BfsArgs {
     int alpha, beta, big_degree, direction;
     int has_big;             // some row has big_degree entries or more (else none is ever deferred)
     int max_degree;          // largest out-degree
+    unsigned long long balance_degree;  // small queues whose rows average more entries are balanced edge by edge
     // the grid kernel may park its level loop for the label-correcting
     // kernel launched right after it: from level yield_level on, at a
     // top-down frontier of at most yield_max_f vertices
