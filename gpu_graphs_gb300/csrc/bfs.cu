@@ -1377,12 +1377,20 @@ bool bfs_relax_tail(const DeviceCsr &g, const gbfs_params &p)
 
 bool bfs_wants_quads(const DeviceCsr &g, const gbfs_params &p)
 {
-    // Up to one row in 16 longer than four (grids, road networks).  A linked
-    // row costs its hop another round trip.  2000 x 2000 grid with a growing
-    // share of such rows, quads against the CSR kernel: 0.1 % 3.95 and 7.99 ms,
-    // 4 % 4.62 and 5.60, 7.6 % 5.43 and 5.34, 12 % 6.27 and 5.12, all (a
-    // triangular mesh) 16.0 and 4.65.
-    return bfs_relax_tail(g, p) && g.max_degree <= QUAD_MAX_DEGREE && (int64_t)g.nover4 * 16 <= g.n;
+    // Up to one row in 32 longer than four (grids, road networks), in 64 on
+    // graphs of more than 2^20 vertices.  A linked row costs its hop another round
+    // trip, and the wider the frontier, the more hops have one.  Grids with a
+    // growing share of such rows, quads against the CSR kernel, ms: 1000 x 1000:
+    // 0.25 % 1.75 and 3.39, 1 % 1.88 and 2.99, 2 % 2.04 and 2.73, 3 % 2.22 and
+    // 2.56, 5 % 2.45 and 2.34; 6000 x 6000: 0.25 % 14.6 and 25.2, 1 % 17.0 and
+    // 22.4, 2 % 19.1 and 20.5, 3 % 20.9 and 19.3.
+    // And hardly any vertex without edges: where many have none, the graph is
+    // a sparse random one, whose frontiers fill the GPU, and a slot per
+    // neighbour that is not there costs more than the round trip it saves
+    // (uniform random, 4 M vertices of mean degree 1.6: 0.81 ms with quads, 0.50
+    // without; 2: 1.26 and 0.72).
+    return bfs_relax_tail(g, p) && g.max_degree <= QUAD_MAX_DEGREE &&
+           (int64_t)g.nover4 * (g.n <= 1 << 20 ? 32 : 64) <= g.n && g.nonisolated * 20 >= (int64_t)g.n * 19;
 }
 
 int bfs_launches_per_search(const DeviceCsr &g, const gbfs_params &p) { return bfs_relax_tail(g, p) ? 2 : 1; }
