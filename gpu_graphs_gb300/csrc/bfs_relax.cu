@@ -435,6 +435,12 @@ __global__ void __launch_bounds__(RX_BLOCK, 2) k_bfs_relax(BfsArgs a)
 // warps slow its barrier (7000 x 7000 grid: 14.1 ms with 512 threads, 13.9 with
 // 256; 1000 x 1000: 1.51 and 1.35; 128 threads are too few on the large grid)
 constexpr int RXQ_BLOCK = 256;
+// Vertices per lane in rounds whose pieces do not fit a local frontier.  Such a
+// round is all throughput: staged in shared memory and dealt by slots, with half
+// the threads of the CSR kernel, it was slower than that one (ring of 4 M vertices
+// with 0.8 M shortcuts: 0.64 ms there, 0.82 staged, 0.54 straight from queue to
+// queue; random 4-regular graph of 4 M vertices 1.09, 0.95 and 0.49).
+constexpr int RXQ_WIDE = 2;
 constexpr size_t RXQ_SMEM = 2 * RX_CAP * (sizeof(int4) + sizeof(unsigned) + sizeof(int));
 
 __global__ void __launch_bounds__(RXQ_BLOCK, 2) k_bfs_relax_quads(BfsArgs a)
@@ -550,6 +556,22 @@ __global__ void __launch_bounds__(RXQ_BLOCK, 2) k_bfs_relax_quads(BfsArgs a)
             }
         };
 
+        // linked rows (link < -1, lf: the vertex's level and first flag as in
+        // s_l): the warp takes the node's entries, one per lane
+        auto linked_rows = [&](int link, unsigned lf, bool last, int nb, unsigned *cnt_nb) {
+            unsigned links = __ballot_sync(FULL, link < -1);
+            while (links) {
+                const int src = __ffs(links) - 1;
+                links &= links - 1u;
+                const int k = -2 - __shfl_sync(FULL, link, src);
+                const unsigned llf = __shfl_sync(FULL, lf, src);
+                const int lw = lane < 15 ? __ldg(over + 16 * (size_t)k + lane) : -1;
+                const unsigned lnd = (llf >> 1) + 1u;
+                edges += (llf & 1u) & (unsigned)(lw >= 0);
+                relax(std::integral_constant<int, 1>{}, &lw, &lnd, last, nb, cnt_nb);
+            }
+        };
+
         // expand local frontier `cur` (nc entries) one level, Q edges per
         // thread in flight
         auto expand = [&](auto ilp, int cur, int nc, bool last, unsigned *cnt_nb) {
@@ -580,27 +602,78 @@ __global__ void __launch_bounds__(RXQ_BLOCK, 2) k_bfs_relax_quads(BfsArgs a)
                 }
                 relax(ilp, w, nd, last, cur ^ 1, cnt_nb);
                 if (!__any_sync(FULL, linked)) continue;
-                // linked rows: the warp takes the node's entries, one per lane
 #pragma unroll
-                for (int q = 0; q < Q; q++) {
-                    unsigned links = __ballot_sync(FULL, w[q] < -1);
-                    while (links) {
-                        const int src = __ffs(links) - 1;
-                        links &= links - 1u;
-                        const int k = -2 - __shfl_sync(FULL, w[q], src);
-                        const unsigned llf = __shfl_sync(FULL, lf[q], src);
-                        const int lw = lane < 15 ? __ldg(over + 16 * (size_t)k + lane) : -1;
-                        const unsigned lnd = (llf >> 1) + 1u;
-                        edges += (llf & 1u) & (unsigned)(lw >= 0);
-                        relax(std::integral_constant<int, 1>{}, &lw, &lnd, last, cur ^ 1, cnt_nb);
+                for (int q = 0; q < Q; q++) linked_rows(w[q], lf[q], last, cur ^ 1, cnt_nb);
+            }
+        };
+
+        // a piece too large to hop, straight from the global queue to the next
+        // one: RXQ_WIDE vertices per lane, all their edges in flight, and one
+        // place in the queue taken per warp and step
+        auto sweep = [&](unsigned long long lo, unsigned long long hi) {
+            constexpr int E = 4 * RXQ_WIDE;
+            for (unsigned long long b = lo + warp * 32 * RXQ_WIDE; b < hi; b += RXQ_BLOCK * RXQ_WIDE) {
+                int w[E];
+                unsigned nd[RXQ_WIDE];
+#pragma unroll
+                for (int x = 0; x < RXQ_WIDE; x++) {
+                    const unsigned long long i = b + 32 * x + lane;
+                    int4 vq = make_int4(-1, -1, -1, -1);
+                    nd[x] = 0;
+                    if (i < hi) {
+                        const int v = __ldcg(qin + i);
+                        nd[x] = __ldcg(lvl + v) + 1u;
+                        vq = __ldg(quad + v);
                     }
+                    w[4 * x] = vq.x;
+                    w[4 * x + 1] = vq.y;
+                    w[4 * x + 2] = vq.z;
+                    w[4 * x + 3] = vq.w;
+                }
+                unsigned old[E];
+                int deg[E];
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    old[e] = 0;
+                    deg[e] = 0;
+                    if (w[e] >= 0) {
+                        old[e] = atomicMin(lvl + w[e], nd[e / 4]);
+                        deg[e] = a.wide ? (int)(__ldg(a.row64 + w[e] + 1) - __ldg(a.row64 + w[e]))
+                                        : __ldg(a.row + w[e] + 1) - __ldg(a.row + w[e]);
+                    }
+                }
+                unsigned go = 0;
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    if (nd[e / 4] >= old[e]) continue;  // (no edge: old is 0)
+                    if (old[e] == 0xffffffffu) {
+                        ++reached;
+                        edges += (unsigned)deg[e];
+                    }
+                    if (atomicMax(stamp + w[e], mark) < mark) go |= 1u << e;
+                }
+                const int incl = warp_incl_scan(__popc(go));
+                const int all = __shfl_sync(FULL, incl, 31);
+                if (all) {
+                    unsigned long long at = 0;
+                    if (lane == 0) at = cd_count(atomicAdd(cnt_out, (unsigned long long)all));
+                    at = __shfl_sync(FULL, at, 0) + (unsigned)(incl - __popc(go));
+#pragma unroll
+                    for (int e = 0; e < E; e++)
+                        if (go >> e & 1u) qout[at++] = w[e];
+                }
+#pragma unroll
+                for (int x = 0; x < RXQ_WIDE; x++) {
+                    const unsigned lf = 2 * (nd[x] - 1u);  // counted when it was queued
+                    linked_rows(w[4 * x + 3], lf, true, 0, s_cnt);
                 }
             }
         };
 
         const unsigned long long lo = F * blockIdx.x / gridDim.x, hi = F * (blockIdx.x + 1) / gridDim.x;
         const bool hops = hi - lo <= (unsigned long long)RX_CAP;
-        for (unsigned long long s0 = lo; s0 < hi; s0 += RX_CAP) {
+        if (!hops) sweep(lo, hi);
+        for (unsigned long long s0 = lo; hops && s0 < hi; s0 += RX_CAP) {
             const int ns = (int)min((unsigned long long)RX_CAP, hi - s0);
             for (int i = (int)t; i < ns; i += RXQ_BLOCK) {
                 const int v = __ldcg(qin + s0 + i);
@@ -620,7 +693,7 @@ __global__ void __launch_bounds__(RXQ_BLOCK, 2) k_bfs_relax_quads(BfsArgs a)
             __syncthreads();
             int nc = ns;
             for (int h = 0;; ++h) {
-                const bool last = !hops || h == RX_HOPS - 1;
+                const bool last = h == RX_HOPS - 1;
                 if (t == 0 && h > 0) s_cnt[(h + 2) % 3] = 0;
                 unsigned *cnt_nb = &s_cnt[(h + 1) % 3];
                 if (4 * nc <= RXQ_BLOCK) expand(std::integral_constant<int, 1>{}, h & 1, nc, last, cnt_nb);
