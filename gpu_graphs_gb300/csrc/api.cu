@@ -371,9 +371,14 @@ static gbfs_params effective_params(gbfs_graph *g)
     if (!g->symmetric && !g->csr.trow) p.direction = GBFS_DIR_TOPDOWN;
     // the label-correcting kernel's adjacency (it walks the rows themselves
     // where that does not fit in memory)
-    if (!g->csr.quad && bfs_wants_quads(g->csr, p)) {
+    if (!g->csr.quad && bfs_wants_quads(g->csr, p) && g->quad_retry.due()) {
         std::string err;
-        if (csr_build_quads(g->csr, g->stream, err) != GBFS_OK) cudaGetLastError();
+        if (csr_build_quads(g->csr, g->stream, err) == GBFS_OK) {
+            g->quad_retry.succeeded();
+        } else {
+            g->quad_retry.failed();
+            cudaGetLastError();
+        }
     }
     return p;
 }
@@ -435,7 +440,14 @@ extern "C" int gbfs_bfs_parents(gbfs_graph *g, int32_t source, int32_t *levels_o
     rc = bfs_run(g->csr, p, w, nullptr, 1, source, d_level, g->stream, res, err, g->symmetric);
     if (rc) return fail(rc, err);
     // long rows in pieces; a graph without room for those is walked by whole rows
-    if (ms_prepare(g->csr, g->stream, err) != GBFS_OK) cudaGetLastError();
+    if (g->piece_retry.due()) {
+        if (ms_prepare(g->csr, g->stream, err) == GBFS_OK) {
+            g->piece_retry.succeeded();
+        } else {
+            g->piece_retry.failed();
+            cudaGetLastError();
+        }
+    }
     cudaError_t e = parents_enqueue(g->csr, g->symmetric, source, d_level, w.ctrl, d_parent, g->stream);
     if (e == cudaSuccess && !dev_par)
         e = cudaMemcpyAsync(parents_out, d_parent, sizeof(int) * n, cudaMemcpyDeviceToHost, g->stream);

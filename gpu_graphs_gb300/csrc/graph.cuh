@@ -12,6 +12,7 @@
 #include "bfs.cuh"
 #include "csr_build.cuh"
 #include "msbfs.cuh"
+#include "retry.h"
 
 struct gbfs_graphset;
 
@@ -26,6 +27,7 @@ struct gbfs_graph {
     bool symmetric = false;      // in-edges == out-edges (bottom-up allowed)
     bool last_multi = false;     // the last traversal was multi-source (trace source)
     std::mutex mu;
+    gbfs::Retry quad_retry, piece_retry;  // under mu
     // graph set cached by gbfs_bfs_batch_graphs (keyed by the handle list)
     std::vector<const gbfs_graph *> batch_key;
     gbfs_graphset *batch_set = nullptr;
