@@ -2109,34 +2109,45 @@ __global__ void k_quads(const RT *__restrict__ row, const int *__restrict__ col,
 
 }  // namespace
 
-int64_t csr_quad_bytes(const DeviceCsr &c)
-{
-    return (int64_t)sizeof(int4) * c.n + 16 * (int64_t)sizeof(int) * c.nover4;
-}
+namespace {
+
+// quad, over and the count of rows in over, in one allocation.
+struct QuadLayout {
+    Carve cv;
+    size_t quad, over, cnt;
+    explicit QuadLayout(const DeviceCsr &c)
+    {
+        quad = cv.add(sizeof(int4) * (size_t)std::max(1, c.n));
+        over = cv.add(16 * sizeof(int) * (size_t)c.nover4);
+        cnt = cv.add(sizeof(unsigned));
+    }
+};
+
+}  // namespace
+
+int64_t csr_quad_bytes(const DeviceCsr &c) { return (int64_t)QuadLayout(c).cv.size; }
 
 int csr_build_quads(DeviceCsr &c, cudaStream_t st, std::string &err)
 {
     if (c.quad) return GBFS_OK;
     int rc = GBFS_OK;
-    int4 *quad = nullptr;
-    int *over = nullptr;
-    unsigned *cnt = nullptr;
-    CK(cudaMalloc(&quad, sizeof(int4) * (size_t)std::max(1, c.n)));
-    CK(cudaMalloc(&over, 16 * sizeof(int) * (size_t)std::max(1, c.nover4)));
-    CK(cudaMalloc(&cnt, sizeof(unsigned)));
-    CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned), st));
-    if (c.wide) k_quads<<<grid_for(c.n, 256), 256, 0, st>>>((const long long *)c.row64, c.col, c.n, quad, over, cnt);
-    else k_quads<<<grid_for(c.n, 256), 256, 0, st>>>((const int *)c.row, c.col, c.n, quad, over, cnt);
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(st));
-    c.quad = quad;
-    c.over = over;
-    quad = nullptr;
-    over = nullptr;
+    char *mem = nullptr;
+    const QuadLayout at(c);
+    CK(cudaMalloc(&mem, at.cv.size));
+    CK(cudaMemsetAsync(mem + at.cnt, 0, sizeof(unsigned), st));
+    {
+        int4 *const quad = (int4 *)(mem + at.quad);
+        int *const over = (int *)(mem + at.over);
+        unsigned *const cnt = (unsigned *)(mem + at.cnt);
+        if (c.wide) k_quads<<<grid_for(c.n, 256), 256, 0, st>>>((const long long *)c.row64, c.col, c.n, quad, over, cnt);
+        else k_quads<<<grid_for(c.n, 256), 256, 0, st>>>((const int *)c.row, c.col, c.n, quad, over, cnt);
+        CK(cudaGetLastError());
+        c.quad = quad;
+        c.over = over;
+    }
+    mem = nullptr;
 done:
-    if (quad) cudaFree(quad);
-    if (over) cudaFree(over);
-    if (cnt) cudaFree(cnt);
+    if (mem) cudaFree(mem);
     return rc;
 }
 
@@ -2161,7 +2172,6 @@ void csr_free(DeviceCsr &c)
     if (c.tfirst) cudaFree(c.tfirst);
     if (c.tpieces) cudaFree(c.tpieces);
     if (c.quad) cudaFree(c.quad);
-    if (c.over) cudaFree(c.over);
     if (c.pieces) cudaFree(c.pieces);
     if (c.own_row && c.row) cudaFree(c.row);
     if (c.own_row && c.row64) cudaFree(c.row64);

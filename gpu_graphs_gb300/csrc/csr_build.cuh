@@ -40,7 +40,7 @@ struct DeviceCsr {
     // there and a link -2 - k in the fourth place to its node, over[16 k ..]:
     // the entries from the fourth on (-1 past the end) and, last, its degree
     int32_t nover4 = 0;        // rows of more than four entries
-    int4 *quad = nullptr;      // n
+    int4 *quad = nullptr;      // n; the allocation of both
     int *over = nullptr;       // 16 per row of more than four entries
     // multi-source pull pieces (built on demand by ms_prepare): every row of
     // degree > 2 * MS_PIECE contributes {vertex, j} for its j-th MS_PIECE edges
@@ -118,7 +118,8 @@ int csr_build_transpose(DeviceCsr &c, cudaStream_t st, std::string &err);
 int csr_build_first(DeviceCsr &c, cudaStream_t st, std::string &err);
 
 // Build c.quad / c.over; a no-op once built.  Only for graphs of out-degree at
-// most QUAD_MAX_DEGREE.  Synchronises st.
+// most QUAD_MAX_DEGREE.  Enqueued on st; no sync (work on other streams has to
+// wait for it).
 constexpr int QUAD_MAX_DEGREE = 16;
 int csr_build_quads(DeviceCsr &c, cudaStream_t st, std::string &err);
 // Bytes csr_build_quads allocates.

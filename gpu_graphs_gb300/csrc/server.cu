@@ -581,7 +581,9 @@ extern "C" int gbfs_server_add_graph(gbfs_server *s, gbfs_graph *g, int32_t *gra
         int rc = want_t ? csr_build_transpose(g->csr, g->stream, err) : GBFS_OK;
         if (!rc) rc = ms_prepare(g->csr, g->stream, err);
         if (rc) return fail(rc, err);
-        if (want_q && csr_build_quads(g->csr, g->stream, err) != GBFS_OK) cudaGetLastError();
+        if (want_q && (csr_build_quads(g->csr, g->stream, err) != GBFS_OK ||
+                       cudaStreamSynchronize(g->stream) != cudaSuccess))
+            cudaGetLastError();
         csr_snapshot = g->csr;
         if (!want_q) {
             csr_snapshot.quad = nullptr;
