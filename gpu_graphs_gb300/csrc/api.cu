@@ -383,19 +383,27 @@ static gbfs_params effective_params(gbfs_graph *g)
     return p;
 }
 
+// effective_params into p, and the workspace that searches with them need.
+// Caller holds g->mu.
+static int search_setup(gbfs_graph *g, gbfs_params &p)
+{
+    p = effective_params(g);
+    std::string err;
+    const int rc = bfs_work_alloc(g->work, g->csr.n, err, g->csr.wide, bfs_small(g->csr, p));
+    return rc ? fail(rc, err) : GBFS_OK;
+}
+
 // Runs a BFS into the graph's workspace or the caller's device buffer, then
-// copies to the caller's host buffer if needed.  Caller holds g->mu.
-static int run_bfs_locked(gbfs_graph *g, const int *d_roots, int k, int single_root, int32_t *levels_out,
-                          BfsResult &res)
+// copies to the caller's host buffer if needed.  Caller holds g->mu and has
+// called search_setup.
+static int run_bfs_locked(gbfs_graph *g, const gbfs_params &p, const int *d_roots, int k, int single_root,
+                          int32_t *levels_out, BfsResult &res)
 {
     std::string err;
-    int rc = bfs_work_alloc(g->work, g->csr.n, err, g->csr.wide);
-    if (rc) return fail(rc, err);
     const bool dev_out = is_device_ptr(levels_out);
     int *d_level = dev_out ? levels_out : g->work.level;
-    gbfs_params p = effective_params(g);
     g->last_multi = false;
-    rc = bfs_run(g->csr, p, g->work, d_roots, k, single_root, d_level, g->stream, res, err, g->symmetric);
+    int rc = bfs_run(g->csr, p, g->work, d_roots, k, single_root, d_level, g->stream, res, err, g->symmetric);
     if (rc) return fail(rc, err);
     if (!dev_out) {
         cudaError_t e = cudaMemcpyAsync(levels_out, d_level, sizeof(int) * (size_t)g->csr.n,
@@ -412,7 +420,9 @@ extern "C" int gbfs_bfs(gbfs_graph *g, int32_t source, int32_t *levels_out, gbfs
     if (source < 0 || source >= g->csr.n) return fail(GBFS_ERR_INVALID_ARG, "source outside [0, n)");
     std::lock_guard<std::mutex> lk(g->mu);
     BfsResult res;
-    int rc = run_bfs_locked(g, nullptr, 1, source, levels_out, res);
+    gbfs_params p;
+    int rc = search_setup(g, p);
+    if (!rc) rc = run_bfs_locked(g, p, nullptr, 1, source, levels_out, res);
     if (rc) return rc;
     fill_stats(stats, res, 1);
     return GBFS_OK;
@@ -425,16 +435,15 @@ extern "C" int gbfs_bfs_parents(gbfs_graph *g, int32_t source, int32_t *levels_o
     if (source < 0 || source >= g->csr.n) return fail(GBFS_ERR_INVALID_ARG, "source outside [0, n)");
     std::lock_guard<std::mutex> lk(g->mu);
     std::string err;
-    int rc = bfs_work_alloc(g->work, g->csr.n, err, g->csr.wide);
-    if (rc) return fail(rc, err);
+    gbfs_params p;
+    int rc = search_setup(g, p);
+    if (rc) return rc;
     BfsWork &w = g->work;
     const size_t n = (size_t)g->csr.n;
     const bool dev_lv = levels_out && is_device_ptr(levels_out);
     const bool dev_par = is_device_ptr(parents_out);
     int *d_level = dev_lv ? levels_out : w.level;
-    // the traversal's queues are free once it has finished
-    int *d_parent = dev_par ? parents_out : w.q0;
-    gbfs_params p = effective_params(g);
+    int *d_parent = dev_par ? parents_out : w.roots;  // (one source: no roots are staged)
     g->last_multi = false;
     BfsResult res;
     rc = bfs_run(g->csr, p, w, nullptr, 1, source, d_level, g->stream, res, err, g->symmetric);
@@ -474,13 +483,14 @@ extern "C" int gbfs_bfs_many(gbfs_graph *g, const int32_t *sources, int32_t k, i
         if (hsrc[i] < 0 || hsrc[i] >= g->csr.n) return fail(GBFS_ERR_INVALID_ARG, "source outside [0, n)");
     std::lock_guard<std::mutex> lk(g->mu);
     std::string err;
-    int rc = bfs_work_alloc(g->work, g->csr.n, err, g->csr.wide);
-    if (!rc) rc = bfs_work_reserve_many(g->work, k, err);
+    gbfs_params p;
+    int rc = search_setup(g, p);
+    if (rc) return rc;
+    rc = bfs_work_reserve_many(g->work, k, err);
     if (rc) return fail(rc, err);
     BfsWork &w = g->work;
     const size_t n = (size_t)g->csr.n;
     const bool dev_out = levels_out && is_device_ptr(levels_out);
-    const gbfs_params p = effective_params(g);
     if (p.per_level_launch) {  // host loop per level: one source at a time
         for (int32_t i = 0; i < k; i++) {
             BfsResult r;
@@ -629,14 +639,14 @@ extern "C" int gbfs_bfs_multiroot(gbfs_graph *g, const int32_t *sources, int32_t
         for (int32_t i = 0; i < k; i++)
             if (sources[i] < 0 || sources[i] >= g->csr.n) return fail(GBFS_ERR_INVALID_ARG, "root outside [0, n)");
     std::lock_guard<std::mutex> lk(g->mu);
-    std::string err;
-    int rc = bfs_work_alloc(g->work, g->csr.n, err, g->csr.wide);
-    if (rc) return fail(rc, err);
+    gbfs_params p;
+    int rc = search_setup(g, p);
+    if (rc) return rc;
     cudaError_t e = cudaMemcpyAsync(g->work.roots, sources, sizeof(int) * (size_t)k,
                                     dev_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, g->stream);
     if (e != cudaSuccess) return cuda_fail(e, "roots upload");
     BfsResult res;
-    rc = run_bfs_locked(g, g->work.roots, k, -1, levels_out, res);
+    rc = run_bfs_locked(g, p, g->work.roots, k, -1, levels_out, res);
     if (rc) return rc;
     fill_stats(stats, res, res.roots);
     return GBFS_OK;

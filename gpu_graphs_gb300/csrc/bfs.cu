@@ -1133,16 +1133,68 @@ int bfs_max_ctas(const gbfs_params &p)
     }
 }
 
-int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide)
+namespace {
+
+// The arrays that a small workspace has not, at `at` in an allocation.
+struct QueueLayout {
+    size_t at, visited, fb0, fb1, fb2, q0, q1, qb0, qb1, big;
+    QueueLayout(Carve &c, int32_t n, bool wide) : at(c.size)
+    {
+        const size_t n4 = sizeof(int) * (size_t)n, w4 = sizeof(unsigned) * (((size_t)n + 31) / 32);
+        const size_t qb = (wide ? sizeof(longlong2) : sizeof(int2)) * (size_t)n;
+        visited = c.add(w4);
+        fb0 = c.add(w4);
+        fb1 = c.add(w4);
+        fb2 = c.add(w4);
+        q0 = c.add(n4);
+        q1 = c.add(n4);
+        qb0 = c.add(qb);
+        qb1 = c.add(qb);
+        big = c.add(n4);
+    }
+    void place(BfsWork &w, char *p) const
+    {
+        w.visited = (unsigned *)(p + visited);
+        w.fb0 = (unsigned *)(p + fb0);
+        w.fb1 = (unsigned *)(p + fb1);
+        w.fb2 = (unsigned *)(p + fb2);
+        w.q0 = (int *)(p + q0);
+        w.q1 = (int *)(p + q1);
+        w.qb0 = (int2 *)(p + qb0);
+        w.qb1 = (int2 *)(p + qb1);
+        w.big = (int *)(p + big);
+    }
+};
+
+}  // namespace
+
+int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide, bool small)
 {
-    if (w.ctrl && w.n == n && w.wide == wide) return GBFS_OK;
+    const bool have = w.ctrl && w.n == n && w.wide == wide;
+    if (have && (small || w.q0)) return GBFS_OK;
+    if (have) {  // small until now
+        Carve c;
+        const QueueLayout q(c, n, wide);
+        const cudaError_t e = cudaMalloc(&w.queues, c.size);
+        if (e != cudaSuccess) {
+            w.queues = nullptr;
+            err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+            return GBFS_ERR_OOM;
+        }
+        q.place(w, (char *)w.queues);
+        w.bytes += (int64_t)c.size;
+        return GBFS_OK;
+    }
     bfs_work_free(w);
-    const size_t n4 = sizeof(int) * (size_t)n, w4 = sizeof(unsigned) * (((size_t)n + 31) / 32);
-    const size_t qb = (wide ? sizeof(longlong2) : sizeof(int2)) * (size_t)n;
+    // (a small workspace fits what is left of the 2 MB that the driver maps at a
+    // time: the first search of 30,000 vertices took 165 us with queues beside it,
+    // 80 to 100 of them for a mapping of their own)
+    const size_t n4 = sizeof(int) * (size_t)n;
     Carve c;
-    const size_t level = c.add(n4), visited = c.add(w4), fb0 = c.add(w4), fb1 = c.add(w4), fb2 = c.add(w4),
-                 q0 = c.add(n4), q1 = c.add(n4), qb0 = c.add(qb), qb1 = c.add(qb), big = c.add(n4), roots = c.add(n4),
-                 ctrl = c.add(sizeof(BfsCtrl));
+    const size_t level = c.add(n4), roots = c.add(n4), ctrl = c.add(sizeof(BfsCtrl));
+    Carve with = c;
+    const QueueLayout q(with, n, wide);
+    if (!small) c = with;
     const cudaError_t e = cudaMalloc(&w.block, c.size);
     if (e != cudaSuccess) {
         w.block = nullptr;
@@ -1152,17 +1204,9 @@ int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide)
     }
     char *p = (char *)w.block;
     w.level = (int *)(p + level);
-    w.visited = (unsigned *)(p + visited);
-    w.fb0 = (unsigned *)(p + fb0);
-    w.fb1 = (unsigned *)(p + fb1);
-    w.fb2 = (unsigned *)(p + fb2);
-    w.q0 = (int *)(p + q0);
-    w.q1 = (int *)(p + q1);
-    w.qb0 = (int2 *)(p + qb0);
-    w.qb1 = (int2 *)(p + qb1);
-    w.big = (int *)(p + big);
     w.roots = (int *)(p + roots);
     w.ctrl = (BfsCtrl *)(p + ctrl);
+    if (!small) q.place(w, p);
     w.bytes = (int64_t)c.size;
     static_assert(offsetof(BfsCtrl, t_entry) <= PINNED_SLOT, "the results fit a pinned slot");
     w.h_ctrl = (BfsCtrl *)pinned_slot_take();
@@ -1180,6 +1224,7 @@ int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide)
 void bfs_work_free(BfsWork &w)
 {
     if (w.block) cudaFree(w.block);
+    if (w.queues) cudaFree(w.queues);
     if (w.d_outs) cudaFree(w.d_outs);
     if (w.h_outs) cudaFreeHost(w.h_outs);
     if (w.evs) {
@@ -1401,9 +1446,9 @@ cudaError_t bfs_enqueue(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, co
 {
     BfsArgs a = make_args(g, p, w, d_roots, k, single_root, d_level, slot, symmetric, resume, max_steps);
     if (!resume && !max_steps && !max_ctas && bfs_small(g, p)) {
-        const cudaError_t es = bfs_small_launch(a, st);
-        if (es != cudaErrorInvalidConfiguration) return es;  // no room for such a cluster on this device
+        return bfs_small_launch(a, st);
     }
+    if (!w.q0) return cudaErrorInvalidValue;  // a small workspace
     if (resume || max_steps || !bfs_relax_tail(g, p))
         return bfs_launch_any(a, p.threads_per_block, p.blocks_per_sm, st, max_ctas);
     // a graph of small degree: a search still running at level

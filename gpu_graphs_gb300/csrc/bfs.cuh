@@ -83,7 +83,8 @@ struct BfsCtrl {
 // Per-graph traversal workspace (allocated on first use, reused).
 struct BfsWork {
     int32_t n = 0;
-    void *block = nullptr;       // the device arrays from here to ctrl
+    void *block = nullptr;       // level, roots and ctrl, and the other device arrays with them or
+    void *queues = nullptr;      // in an allocation of their own (null, and those arrays, in a small workspace)
     int *level = nullptr;        // n (used when the caller's buffer is on the host)
     unsigned *visited = nullptr; // W
     unsigned *fb0 = nullptr;     // W frontier bitmaps (three, rotating)
@@ -95,7 +96,7 @@ struct BfsWork {
     int2 *qb1 = nullptr;         // (16-byte longlong2 entries when `wide`)
     bool wide = false;           // sized for a graph with 64-bit row offsets
     int *big = nullptr;          // n deferred rows
-    int *roots = nullptr;        // root staging (n)
+    int *roots = nullptr;        // root staging (n), or scratch between searches
     BfsCtrl *ctrl = nullptr;
     BfsCtrl *h_ctrl = nullptr;   // pinned: the part of a control block before t_entry; searches
                                  // write their results there (h_ctrl->out) themselves
@@ -125,7 +126,9 @@ void bfs_graph_free(BfsWork &w);
 // Allocate the second level buffer, the copy stream and its events.
 int bfs_work_reserve_overlap(BfsWork &w, std::string &err);
 
-int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide = false);
+// small: for searches that run on one cluster (bfs_small), without queues and
+// bitmaps; a later call for others adds them.
+int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide = false, bool small = false);
 void bfs_work_free(BfsWork &w);
 
 struct BfsResult {
@@ -153,7 +156,7 @@ int bfs_run(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const int *d_r
 // label-correcting kernel, and the kernel launches one search enqueues
 // (2 then, else 1).
 bool bfs_relax_tail(const DeviceCsr &g, const gbfs_params &p);
-// Whether such a search runs on one cluster (bfs_small.cu).
+// Whether such a search of the current device runs on one cluster (bfs_small.cu).
 bool bfs_small(const DeviceCsr &g, const gbfs_params &p);
 // Whether that kernel runs on the graph's fixed-width adjacency
 // (csr_build_quads) when it has been built.

@@ -258,12 +258,13 @@ __global__ void __launch_bounds__(BLOCK, 1) k_bfs_small(BfsArgs a)
     }
 }
 
+// args null: whether the device holds the largest such cluster at all
+// (cudaErrorInvalidConfiguration: no).
 template <int LOGS, int BLOCK, typename RT>
-cudaError_t small_launch(const BfsArgs &args, cudaStream_t st)
+cudaError_t small_launch(const BfsArgs *args, cudaStream_t st)
 {
     static LaunchSetup setup;  // per template instance
     const size_t smem = sizeof(SmallShared<LOGS>);
-    const int ctas = (args.n + (1 << LOGS) - 1) >> LOGS;
     int unused = 0, fits = 0;
     auto config = [&](int c, cudaLaunchAttribute *at) {
         cudaLaunchConfig_t cfg = {};
@@ -289,20 +290,29 @@ cudaError_t small_launch(const BfsArgs &args, cudaStream_t st)
     });
     if (e != cudaSuccess) return e;
     if (fits < 1) return cudaErrorInvalidConfiguration;
+    if (!args) return cudaSuccess;
     cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = config(ctas, &at);
-    return cudaLaunchKernelEx(&cfg, k_bfs_small<LOGS, BLOCK, RT>, args);
+    const cudaLaunchConfig_t cfg = config((args->n + (1 << LOGS) - 1) >> LOGS, &at);
+    return cudaLaunchKernelEx(&cfg, k_bfs_small<LOGS, BLOCK, RT>, *args);
 }
 
 template <typename RT>
-cudaError_t small_launch_n(const BfsArgs &a, cudaStream_t st)
+cudaError_t small_launch_n(int n, const BfsArgs *a, cudaStream_t st)
 {
-    switch (small_part_log(a.n)) {
+    switch (small_part_log(n)) {
     case 10: return small_launch<10, 1024, RT>(a, st);
     case 11: return small_launch<11, 1024, RT>(a, st);
     case 12: return small_launch<12, 1024, RT>(a, st);
     default: return small_launch<SMALL_MAX_LOG, 1024, RT>(a, st);
     }
+}
+
+// (a device that has no room for the cluster, or whose set-up fails: the grid kernel)
+bool small_fits(const DeviceCsr &g)
+{
+    const cudaError_t e = g.wide ? small_launch_n<long long>(g.n, nullptr, nullptr) : small_launch_n<int>(g.n, nullptr, nullptr);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e == cudaSuccess;
 }
 
 }  // namespace
@@ -333,13 +343,15 @@ bool bfs_small(const DeviceCsr &g, const gbfs_params &p)
     if (g.n > SMALL_MAX_N || g.m > 4 << 20 || g.max_degree > 1 << 14) return false;
     const int64_t most = p.direction == GBFS_DIR_TOPDOWN ? 250000 : g.n <= SMALL_MAX_N / 2 ? 100000 : 70000;
     if (g.part_cost > most) return false;
-    if (p.direction == GBFS_DIR_TOPDOWN) return true;
-    return small_skewed(g.max_degree, g.n, g.m) ? g.m <= 1 << 19 : g.m <= 20 * (int64_t)g.n;
+    if (p.direction != GBFS_DIR_TOPDOWN &&
+        g.m > (small_skewed(g.max_degree, g.n, g.m) ? (int64_t)1 << 19 : 20 * (int64_t)g.n))
+        return false;
+    return small_fits(g);
 }
 
 cudaError_t bfs_small_launch(const BfsArgs &a, cudaStream_t st)
 {
-    return a.wide ? small_launch_n<long long>(a, st) : small_launch_n<int>(a, st);
+    return a.wide ? small_launch_n<long long>(a.n, &a, st) : small_launch_n<int>(a.n, &a, st);
 }
 
 }  // namespace gbfs
