@@ -2177,6 +2177,7 @@ void csr_free(DeviceCsr &c)
     if (c.own_row && c.row64) cudaFree(c.row64);
     if (c.col) cudaFree(c.col);
     if (c.block) cudaFree(c.block);
+    if (c.keep) cudaFree(c.keep);
     c = DeviceCsr{};
 }
 
@@ -2373,6 +2374,7 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
                                                 : BuildScratch<int>(n, most, flags & GBFS_DEDUP).size;
     const bool together = later <= (size_t)64 << 20;
     const size_t at_later = together ? cv.add(later) : 0;
+    CK(cudaMalloc(&out.keep, 256));
     CK(cudaMalloc(&mem, cv.size));
     CK(cudaMemsetAsync(mem, 0, zeroed, st));
     scan_scratch_carve(mem + at_scan, tiles, ss);
@@ -2451,6 +2453,7 @@ int csr_adopt_t(int32_t n, int64_t m, RT *d_row, int *d_col, cudaStream_t st, De
     int *status = nullptr;
     RT h[2] = {0, 0};
     int h_status = 0;
+    CK(cudaMalloc(&out.keep, 256));
     CK(cudaMalloc(&status, sizeof(int)));
     CK(cudaMemsetAsync(status, 0, sizeof(int), st));
     k_validate_csr<RT><<<grid_for(std::max<int64_t>(m, n), 256), 256, 0, st>>>(d_row, d_col, n, m, status);

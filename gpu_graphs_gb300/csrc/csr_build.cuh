@@ -15,6 +15,11 @@ struct DeviceCsr {
     // second, and the row offsets of a graph built here (a given CSR's are its own)
     void *block = nullptr;
     bool own_row = false;      // row / row64 is an allocation of its own
+    // a few bytes: the driver maps memory for small allocations 2 MB at a time and
+    // unmaps it with the last of them, some 100 us each way, which calls that only
+    // use a little scratch would pay again and again (another graph taken over
+    // beside this one: 380 us without it, 270 so)
+    void *keep = nullptr;
     int32_t n = 0;
     int64_t m = 0;
     int *row = nullptr;        // n+1 (null when wide)
