@@ -50,7 +50,11 @@ bool is_device_ptr(const void *p)
 
 int graph_wrap(DeviceCsr &csr, bool symmetric_known, bool symmetric, cudaStream_t st, gbfs_graph **out)
 {
-    gbfs_graph *g = new (std::nothrow) gbfs_graph();
+    gbfs_graph *g = nullptr;
+    try {
+        g = new gbfs_graph();
+    } catch (const std::bad_alloc &) {
+    }
     if (!g) {
         csr_free(csr);
         if (st) cudaStreamDestroy(st);
@@ -370,8 +374,9 @@ static gbfs_params effective_params(gbfs_graph *g)
     }
     if (!g->symmetric && !g->csr.trow) p.direction = GBFS_DIR_TOPDOWN;
     // the label-correcting kernel's adjacency (it walks the rows themselves
-    // where that does not fit in memory)
-    if (!g->csr.quad && bfs_wants_quads(g->csr, p) && g->quad_retry.due()) {
+    // where that does not fit in memory, or in the budget of a server that the
+    // graph is admitted to)
+    if (!g->csr.quad && bfs_wants_quads(g->csr, p) && g->quads->barred == 0 && g->quad_retry.due()) {
         std::string err;
         if (csr_build_quads(g->csr, g->stream, err) == GBFS_OK) {
             g->quad_retry.succeeded();

@@ -2151,6 +2151,13 @@ done:
     return rc;
 }
 
+void csr_drop_quads(DeviceCsr &c)
+{
+    if (c.quad) cudaFree(c.quad);
+    c.quad = nullptr;
+    c.over = nullptr;
+}
+
 int64_t csr_device_bytes(const DeviceCsr &c)
 {
     const int64_t n = c.n, m = c.m;
@@ -2171,7 +2178,7 @@ void csr_free(DeviceCsr &c)
     if (c.theavy) cudaFree(c.theavy);
     if (c.tfirst) cudaFree(c.tfirst);
     if (c.tpieces) cudaFree(c.tpieces);
-    if (c.quad) cudaFree(c.quad);
+    csr_drop_quads(c);
     if (c.pieces) cudaFree(c.pieces);
     if (c.own_row && c.row) cudaFree(c.row);
     if (c.own_row && c.row64) cudaFree(c.row64);

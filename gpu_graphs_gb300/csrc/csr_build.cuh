@@ -129,6 +129,7 @@ constexpr int QUAD_MAX_DEGREE = 16;
 int csr_build_quads(DeviceCsr &c, cudaStream_t st, std::string &err);
 // Bytes csr_build_quads allocates.
 int64_t csr_quad_bytes(const DeviceCsr &c);
+void csr_drop_quads(DeviceCsr &c);
 
 // Device bytes held by the CSR and everything built on it.
 int64_t csr_device_bytes(const DeviceCsr &c);

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <memory>
 #include <mutex>
@@ -16,8 +17,20 @@
 
 struct gbfs_graphset;
 
+namespace gbfs {
+
+// Servers and a graph's fixed-width adjacency (csr.quad).  Counts go up under the
+// graph's mutex, and the adjacency is freed under it, only while users is 0.
+struct QuadHold {
+    std::atomic<int> users{0};   // servers that serve the graph from it, in their budgets
+    std::atomic<int> barred{0};  // servers whose budget has no room for it: it is not built
+};
+
+}  // namespace gbfs
+
 struct gbfs_graph {
     gbfs::DeviceCsr csr;
+    std::shared_ptr<gbfs::QuadHold> quads = std::make_shared<gbfs::QuadHold>();
     gbfs_params params{};        // read and written only under pmu (graph_params / set)
     mutable std::mutex pmu;
     gbfs::BfsWork work;

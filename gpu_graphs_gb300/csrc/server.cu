@@ -81,6 +81,19 @@ struct SrvGraph {
     double est_us = 0;     // recent launch time (moving average), 0 before the first
     bool singles = false;  // small degree: served as single-source searches
     int drainer = -1;      // the slot that stops filling units for this graph's next batch
+    // its fixed-width adjacency: held where csr.quad is set (counted in bytes), else
+    // barred where the graph could have one
+    std::shared_ptr<QuadHold> quads;
+    bool barred = false;
+
+    // the graph is no longer served here (g itself may be gone)
+    void release_quads()
+    {
+        if (!quads) return;
+        if (csr.quad) --quads->users;
+        if (barred) --quads->barred;
+        quads.reset();
+    }
 };
 
 // Units (concurrent single-source searches) per slot.  A 4000 x 4000 grid
@@ -212,6 +225,7 @@ struct gbfs_server {
     void plan(int idx, std::vector<int> &units, Clock::time_point &next_ready);
     void take(Slot &sl, int j, int32_t gid, SrvGraph &c, int k, int cap, int lanes, std::vector<int> &units);
     void launch(Slot &sl, int j);
+    void reclaim_quads(std::unique_lock<std::mutex> &lk, int64_t bytes);
     void advance(Slot &sl, int j);
     void finish(Slot &sl, int j, int status);
 };
@@ -420,6 +434,32 @@ void gbfs_server::worker(int idx)
     }
 }
 
+// Under mu and admit_mu: gives up fixed-width adjacencies until `bytes` fit the
+// budget beside what is resident, or none is left; the graphs are served from their
+// rows then.  One that another server uses is in that one's budget and stays; others
+// are freed.  Waits for the launches in flight.
+void gbfs_server::reclaim_quads(std::unique_lock<std::mutex> &lk, int64_t bytes)
+{
+    resizing = true;
+    cv_done.wait(lk, [&] { return busy_jobs == 0; });
+    for (auto &kv : graphs) {
+        SrvGraph &c = kv.second;
+        if (resident + bytes <= cfg.mem_budget_bytes) break;
+        if (!c.csr.quad) continue;
+        std::lock_guard<std::mutex> glk(c.g->mu);
+        const int64_t b = csr_quad_bytes(c.csr);
+        c.csr.quad = nullptr;
+        c.csr.over = nullptr;
+        ++c.quads->barred;
+        if (--c.quads->users == 0) csr_drop_quads(c.g->csr);
+        c.barred = true;
+        c.bytes -= b;
+        resident -= b;
+    }
+    resizing = false;
+    wake_all();
+}
+
 extern "C" int gbfs_server_create(const gbfs_server_config *cfg, gbfs_server **out)
 {
     if (!cfg || !out) return fail(GBFS_ERR_INVALID_ARG, "NULL argument");
@@ -502,6 +542,7 @@ extern "C" void gbfs_server_destroy(gbfs_server *s)
         for (auto st : sl->st)
             if (st) cudaStreamDestroy(st);
     }
+    for (auto &kv : s->graphs) kv.second.release_quads();
     delete s;
 }
 
@@ -517,17 +558,28 @@ extern "C" int gbfs_server_add_graph(gbfs_server *s, gbfs_graph *g, int32_t *gra
     const bool has_t = want_t || g->csr.trow != nullptr;
     const int64_t tbytes =  // trow, tcol, theavy, tfirst still to build
         want_t && !g->csr.trow ? (int64_t)sizeof(int) * (3 * (int64_t)g->csr.n + 1 + g->csr.m) : 0;
+    // the label-correcting kernel's adjacency, built or not yet, where the budget
+    // has room for it (else searches of the graph walk its rows while it is
+    // admitted, and one that is built is given back; for graphs that fit the budget
+    // no other way, adjacencies of those admitted before are)
     const int64_t qbytes = csr_quad_bytes(g->csr);
-    int64_t gbytes = csr_device_bytes(g->csr) - (g->csr.quad ? qbytes : 0) + tbytes + ms_prepare_bytes(g->csr, has_t);
+    const bool have_q = g->csr.quad != nullptr;
+    const bool could_q = have_q || bfs_wants_quads(g->csr, graph_params(g));
+    int64_t gbytes = csr_device_bytes(g->csr) - (have_q ? qbytes : 0) + tbytes + ms_prepare_bytes(g->csr, has_t);
     const int64_t new_cap = std::max<int64_t>(s->n_cap, g->csr.n);
     int64_t need = s->resident + gbytes + s->slots_total(new_cap);
-    // the label-correcting kernel's adjacency, where the budget has room for
-    // it (else this server's searches of the graph walk its rows)
-    const bool want_q =
-        bfs_wants_quads(g->csr, graph_params(g)) && need + qbytes <= s->cfg.mem_budget_bytes;
-    if (want_q) {
+    bool use_q = could_q && need + qbytes <= s->cfg.mem_budget_bytes;
+    if (use_q) {
         gbytes += qbytes;
         need += qbytes;
+    } else if (need > s->cfg.mem_budget_bytes) {
+        int64_t held = 0;
+        for (auto &kv : s->graphs)
+            if (kv.second.csr.quad) held += csr_quad_bytes(kv.second.csr);
+        if (need - held <= s->cfg.mem_budget_bytes) {
+            s->reclaim_quads(lk, need - s->resident);
+            need = s->resident + gbytes + s->slots_total(new_cap);
+        }
     }
     if (need > s->cfg.mem_budget_bytes) {
         ++s->rejected;
@@ -581,20 +633,28 @@ extern "C" int gbfs_server_add_graph(gbfs_server *s, gbfs_graph *g, int32_t *gra
         int rc = want_t ? csr_build_transpose(g->csr, g->stream, err) : GBFS_OK;
         if (!rc) rc = ms_prepare(g->csr, g->stream, err);
         if (rc) return fail(rc, err);
-        if (want_q && (csr_build_quads(g->csr, g->stream, err) != GBFS_OK ||
-                       cudaStreamSynchronize(g->stream) != cudaSuccess))
+        if (use_q && (csr_build_quads(g->csr, g->stream, err) != GBFS_OK ||
+                      cudaStreamSynchronize(g->stream) != cudaSuccess)) {
             cudaGetLastError();
+            use_q = false;
+            gbytes -= qbytes;
+        }
+        if (!use_q && g->quads->users == 0) csr_drop_quads(g->csr);
         csr_snapshot = g->csr;
-        if (!want_q) {
+        if (!use_q) {
             csr_snapshot.quad = nullptr;
             csr_snapshot.over = nullptr;
         }
+        if (use_q) ++g->quads->users;
+        else if (could_q) ++g->quads->barred;
     }
     const int32_t gid = s->next_gid++;
     SrvGraph sg;
     sg.g = g;
     sg.csr = csr_snapshot;
     sg.bytes = gbytes;
+    sg.quads = g->quads;
+    sg.barred = could_q && !use_q;
     sg.singles = bfs_relax_tail(csr_snapshot, graph_params(g));
     s->graphs.emplace(gid, std::move(sg));
     s->resident += gbytes;
@@ -613,6 +673,16 @@ extern "C" int gbfs_server_remove_graph(gbfs_server *s, int32_t graph_id)
     if (!it->second.pending.empty() || it->second.inflight > 0)
         return fail(GBFS_ERR_INVALID_ARG, "graph has queries pending or in flight");
     s->resident -= it->second.bytes;
+    {
+        // (the last server with room for its adjacency, and some without)
+        const std::shared_ptr<QuadHold> quads = it->second.quads;
+        gbfs_graph *g = it->second.g;
+        it->second.release_quads();
+        if (quads->users == 0 && quads->barred > 0) {
+            std::lock_guard<std::mutex> glk(g->mu);
+            if (quads->users == 0) csr_drop_quads(g->csr);
+        }
+    }
     s->graphs.erase(it);
     return GBFS_OK;
 }

@@ -441,8 +441,12 @@ void gbfs_server_destroy(gbfs_server *s);
 /* Admit a resident graph (borrowed; must outlive the server or be removed).
  * A directed graph whose direction is not GBFS_DIR_TOPDOWN gets its
  * transpose (in-edge rows, for bottom-up and pull steps) built here and
- * counted in the budget.  GBFS_ERR_BUDGET if its CSR plus one slot's
- * workspace does not fit.  Concurrent calls are serialised (each sees the
+ * counted in the budget.  A small-degree graph's fixed-width adjacency is
+ * built and counted where the budget has room; where it has not, one that
+ * searches have built is given back and none is built while the graph is
+ * admitted, and a graph that would not fit otherwise takes the room of those
+ * admitted before.  GBFS_ERR_BUDGET if the graph's CSR plus one
+ * slot's workspace does not fit.  Concurrent calls are serialised (each sees the
  * bytes the others admitted). */
 int gbfs_server_add_graph(gbfs_server *s, gbfs_graph *g, int32_t *graph_id);
 int gbfs_server_remove_graph(gbfs_server *s, int32_t graph_id);
