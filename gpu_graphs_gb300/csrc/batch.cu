@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "graph.cuh"
+#include "level_route.h"
 
 using namespace gbfs;
 
@@ -48,6 +49,16 @@ __global__ void k_slices_out(const int *__restrict__ level, long long n, const g
         int *dst = slices[lo].dst;
         if (dst) dst[v - slices[lo].offset] = level[v];
     }
+}
+
+LevelRoute output_route(const void *p, int device)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return LevelRoute::HOST;
+    }
+    return level_route((int)at.type, at.device, device);
 }
 
 int make_set(gbfs_graph *g, int32_t count, const std::vector<int64_t> &offsets, gbfs_graphset **out)
@@ -198,7 +209,16 @@ extern "C" int gbfs_bfs_batch(gbfs_graphset *s, const int32_t *sources, int32_t 
 {
     if (!s || !sources || !levels_out) return fail(GBFS_ERR_INVALID_ARG, "NULL argument");
     const int32_t count = (int32_t)s->sizes.size();
-    std::vector<int32_t> roots(count);
+    std::vector<int32_t> roots;
+    std::vector<gbfs_graphset::Slice> slices;
+    std::vector<LevelRoute> routes;
+    try {
+        roots.resize(count);
+        slices.resize(count);
+        routes.resize(count);
+    } catch (const std::bad_alloc &) {
+        return fail(GBFS_ERR_OOM, "host allocation failed for the batch");
+    }
     for (int32_t i = 0; i < count; i++) {
         if (!levels_out[i]) return fail(GBFS_ERR_INVALID_ARG, "NULL level buffer");
         if (sources[i] < 0 || sources[i] >= s->sizes[i]) return fail(GBFS_ERR_INVALID_ARG, "source outside its graph");
@@ -216,20 +236,26 @@ extern "C" int gbfs_bfs_batch(gbfs_graphset *s, const int32_t *sources, int32_t 
     int rc = gbfs_bfs_multiroot(g, roots.data(), count, g->work.level, &st);
     if (rc) return rc;
     std::lock_guard<std::mutex> lk(g->mu);
-    std::vector<gbfs_graphset::Slice> slices(count);
-    bool any_host = false, any_dev = false;
+    bool any_host = false, any_kernel = false;
     for (int32_t i = 0; i < count; i++) {
-        const bool dev = is_device_ptr(levels_out[i]);
-        slices[i] = {dev ? levels_out[i] : nullptr, (long long)s->offsets[i]};
-        any_host = any_host || !dev;
-        any_dev = any_dev || dev;
+        routes[i] = output_route(levels_out[i], g->device);
+        slices[i] = {routes[i] == LevelRoute::KERNEL ? levels_out[i] : nullptr, (long long)s->offsets[i]};
+        any_host = any_host || routes[i] == LevelRoute::HOST;
+        any_kernel = any_kernel || routes[i] == LevelRoute::KERNEL;
+    }
+    if (any_kernel && !s->d_slices &&
+        cudaMalloc(&s->d_slices, sizeof(gbfs_graphset::Slice) * (size_t)count) != cudaSuccess) {
+        // no room for the table: a copy per member
+        cudaGetLastError();
+        s->d_slices = nullptr;
+        any_kernel = false;
+        for (auto &r : routes)
+            if (r == LevelRoute::KERNEL) r = LevelRoute::COPY;
     }
     cudaError_t e = cudaSuccess;
-    if (any_dev) {
-        if (!s->d_slices) e = cudaMalloc(&s->d_slices, sizeof(gbfs_graphset::Slice) * (size_t)count);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(s->d_slices, slices.data(), sizeof(gbfs_graphset::Slice) * (size_t)count,
-                                cudaMemcpyHostToDevice, g->stream);
+    if (any_kernel) {
+        e = cudaMemcpyAsync(s->d_slices, slices.data(), sizeof(gbfs_graphset::Slice) * (size_t)count,
+                            cudaMemcpyHostToDevice, g->stream);
         if (e == cudaSuccess) {
             const long long n = g->csr.n, per = SLICE_BLOCK * SLICE_PER;
             k_slices_out<<<(unsigned)((n + per - 1) / per), SLICE_BLOCK, 0, g->stream>>>(g->work.level, n, s->d_slices,
@@ -250,10 +276,14 @@ extern "C" int gbfs_bfs_batch(gbfs_graphset *s, const int32_t *sources, int32_t 
         if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
         if (e == cudaSuccess)
             for (int32_t i = 0; i < count; i++)
-                if (!slices[i].dst)
+                if (routes[i] == LevelRoute::HOST)
                     memcpy(levels_out[i], stage + s->offsets[i], sizeof(int32_t) * (size_t)s->sizes[i]);
         cudaFreeHost(stage);
     }
+    for (int32_t i = 0; i < count && e == cudaSuccess; i++)
+        if (routes[i] == LevelRoute::COPY)
+            e = cudaMemcpyAsync(levels_out[i], g->work.level + s->offsets[i], sizeof(int32_t) * (size_t)s->sizes[i],
+                                cudaMemcpyDeviceToDevice, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     if (e != cudaSuccess) return cuda_fail(e, "batch levels copy-out");
     if (stats) *stats = st;
