@@ -26,12 +26,15 @@ void set_error(const std::string &msg) { tl_error = msg; }
 
 int fail(int code, const std::string &msg)
 {
+    // a refused allocation is reported here, and not by the next call's launches
+    if (code == GBFS_ERR_OOM || code == GBFS_ERR_CUDA) cudaGetLastError();
     tl_error = msg;
     return code;
 }
 
 int cuda_fail(cudaError_t e, const char *what)
 {
+    cudaGetLastError();
     tl_error = std::string(what) + ": " + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? GBFS_ERR_OOM : GBFS_ERR_CUDA;
 }

@@ -61,6 +61,7 @@ enum BinClass : int { BIN_W4, BIN_W16, BIN_1K, BIN_2K, BIN_4K, BIN_LONG, BIN_CLA
     do {                                                                         \
         cudaError_t e_ = (call);                                                 \
         if (e_ != cudaSuccess) {                                                 \
+            cudaGetLastError(); /* or the next call's launches report it */      \
             err = std::string(#call) + ": " + cudaGetErrorString(e_);            \
             rc = (e_ == cudaErrorMemoryAllocation) ? GBFS_ERR_OOM : GBFS_ERR_CUDA; \
             goto done;                                                           \
