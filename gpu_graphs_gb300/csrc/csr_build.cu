@@ -1631,6 +1631,7 @@ int finalize_t(DeviceCsr &out, const RT *row, cudaStream_t st, std::string &err)
     out.nheavy = (int32_t)h->nheavy;
     out.part_cost = (int64_t)*std::max_element(h->part, h->part + SMALL_CTAS);
 done:
+    if (rc) cudaStreamSynchronize(st);  // before h's slot is another's
     if (d_res) cudaFree(d_res);
     return rc;
 }
@@ -1838,6 +1839,7 @@ int sort_rows_inplace(const RT *row, int *col, int32_t n, int64_t m, cudaStream_
     CK(sorter.sort(row, n, col, 0, (int *)(mem + ucnt), nullptr, 0, st));
     CK(cudaStreamSynchronize(st));
 done:
+    if (rc) cudaStreamSynchronize(st);  // before the sorter's slot is another's
     if (mem) cudaFree(mem);
     return rc;
 }
@@ -1893,6 +1895,7 @@ int hub_first_rows(const RT *row, int n, int64_t m, int *col, cudaStream_t st, s
     }
     CK(cudaStreamSynchronize(st));
 done:
+    if (rc) cudaStreamSynchronize(st);  // before h's slot is another's
     if (mem) cudaFree(mem);
     if (best) cudaFree(best);
     return rc;
@@ -2339,6 +2342,7 @@ int build_rows(int32_t n, int64_t m, int64_t md, const int *d_src, const int *d_
     col_out = col;
     col = nullptr;
 done:
+    if (rc) cudaStreamSynchronize(st);  // before the slots of h_m2 and the sorter are another's
     if (mem) cudaFree(mem);
     if (col) cudaFree(col);
     if (tmp) cudaFree(tmp);
@@ -2447,6 +2451,7 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
     rc = finalize(out, st, err);
 
 done:
+    if (rc) cudaStreamSynchronize(st);  // before h's slot is another's
     if (mem) cudaFree(mem);
     if (rc != GBFS_OK) csr_free(out);
     return rc;

@@ -55,3 +55,14 @@ def test_small_search_reads_a_word_of_new_vertices_before_it_is_cleared():
     read = body.index("= sh.fresh[v >> 5]")
     clear = body.index("sh.fresh[v >> 5] = 0")
     assert read < clear and "__syncwarp()" in body[read:clear]
+
+
+def test_builds_that_fail_wait_for_their_copies():
+    """A pinned slot goes back to all users of the pool at the end of its scope: a
+    function that copies into one synchronises before it returns an error."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "csr_build.cu").read_text())
+    functions = re.split(r"\n(?=(?:template [^\n]*\n)?(?:int|struct|cudaError_t|void) \w)", text)
+    holders = [f for f in functions if re.search(r"\bPinned<\w+> \w+;|\bRowSorter<RT> \w+;", f) and "done:" in f]
+    assert len(holders) == 5
+    for f in holders:
+        assert "if (rc) cudaStreamSynchronize(st);" in f[f.rindex("done:"):], f[:200]
