@@ -574,7 +574,8 @@ extern "C" int gbfs_last_trace(gbfs_graph *g, gbfs_level_trace *rows, int32_t ca
     int trace_len;
     const LevelTrace *trace;
     cudaError_t e;
-    // the control blocks' parts from t_entry on
+    // the control blocks' parts from t_entry on, copied on the graph's stream (the
+    // default stream's work, and captures in other threads, are not this call's)
     std::unique_ptr<BfsCtrl> hb;
     std::unique_ptr<MsCtrl> hm;
     if (g->last_multi) {
@@ -582,11 +583,12 @@ extern "C" int gbfs_last_trace(gbfs_graph *g, gbfs_level_trace *rows, int32_t ca
         hm.reset(new (std::nothrow) MsCtrl);
         MsCtrl *h = hm.get();
         if (!h) return fail(GBFS_ERR_OOM, "host allocation failed for the trace");
-        e = cudaStreamSynchronize(g->stream);
+        e = cudaMemcpyAsync(&h->t_entry, &g->ms.ctrl->t_entry, sizeof(MsCtrl) - offsetof(MsCtrl, t_entry),
+                            cudaMemcpyDeviceToHost, g->stream);
         if (e == cudaSuccess)
-            e = cudaMemcpy(&h->t_entry, &g->ms.ctrl->t_entry, sizeof(MsCtrl) - offsetof(MsCtrl, t_entry),
-                           cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(&h->trace_len, &g->ms.ctrl->trace_len, sizeof(int), cudaMemcpyDeviceToHost);
+            e = cudaMemcpyAsync(&h->trace_len, &g->ms.ctrl->trace_len, sizeof(int), cudaMemcpyDeviceToHost, g->stream);
+        const cudaError_t done = cudaStreamSynchronize(g->stream);
+        if (e == cudaSuccess) e = done;
         if (e != cudaSuccess) return cuda_fail(e, "trace D2H");
         t_entry = h->t_entry; t_start = h->t_start; t_end = h->t_end; t_exit = h->t_exit;
         trace_len = h->trace_len; trace = h->trace;
@@ -595,10 +597,10 @@ extern "C" int gbfs_last_trace(gbfs_graph *g, gbfs_level_trace *rows, int32_t ca
         hb.reset(new (std::nothrow) BfsCtrl);
         BfsCtrl *h = hb.get();
         if (!h) return fail(GBFS_ERR_OOM, "host allocation failed for the trace");
-        e = cudaStreamSynchronize(g->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(&h->t_entry, &g->work.ctrl->t_entry, sizeof(BfsCtrl) - offsetof(BfsCtrl, t_entry),
-                           cudaMemcpyDeviceToHost);
+        e = cudaMemcpyAsync(&h->t_entry, &g->work.ctrl->t_entry, sizeof(BfsCtrl) - offsetof(BfsCtrl, t_entry),
+                            cudaMemcpyDeviceToHost, g->stream);
+        const cudaError_t done = cudaStreamSynchronize(g->stream);
+        if (e == cudaSuccess) e = done;
         if (e != cudaSuccess) return cuda_fail(e, "trace D2H");
         t_entry = h->t_entry; t_start = h->t_start; t_end = h->t_end; t_exit = h->t_exit;
         trace_len = h->trace_len; trace = h->trace;

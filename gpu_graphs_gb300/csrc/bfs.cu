@@ -1591,8 +1591,10 @@ int bfs_run(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const int *d_r
     }
     if (e == cudaSuccess) e = cudaEventRecord(w.ev1, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess && w.h_ctrl->out.levels < 0)
-        e = cudaMemcpy(&w.h_ctrl->status, &w.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && w.h_ctrl->out.levels < 0) {
+        e = cudaMemcpyAsync(&w.h_ctrl->status, &w.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    }
     if (e != cudaSuccess) {
         err = std::string("BFS launch: ") + cudaGetErrorString(e);
         return GBFS_ERR_CUDA;
