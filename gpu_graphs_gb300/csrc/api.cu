@@ -397,7 +397,7 @@ static int search_setup(gbfs_graph *g, gbfs_params &p)
 {
     p = effective_params(g);
     std::string err;
-    const int rc = bfs_work_alloc(g->work, g->csr.n, err, g->csr.wide, bfs_small(g->csr, p));
+    const int rc = bfs_work_alloc(g->work, g->csr.n, err, g->stream, g->csr.wide, bfs_small(g->csr, p));
     return rc ? fail(rc, err) : GBFS_OK;
 }
 
@@ -680,7 +680,7 @@ extern "C" int gbfs_bfs_multi(gbfs_graph *g, const int32_t *sources, int32_t k, 
     if (g->csr.wide) return fail(GBFS_ERR_TOO_LARGE, "multi-source search needs 32-bit row offsets");
     std::lock_guard<std::mutex> lk(g->mu);
     std::string err;
-    int rc = ms_work_alloc(g->ms, g->csr.n, err);
+    int rc = ms_work_alloc(g->ms, g->csr.n, err, g->stream);
     if (rc) return fail(rc, err);
     const gbfs_params p = effective_params(g);  // builds the transpose a directed graph's pull steps need
     rc = ms_prepare(g->csr, g->stream, err);
@@ -756,14 +756,13 @@ extern "C" int gbfs_exclusive_scan_i32(const int32_t *d_in, int64_t *d_out, int6
             cudaDeviceSynchronize();
             cudaFree(pool.mem);
             pool.mem = nullptr;
+            pool.tiles = 0;
         }
         const int64_t want = std::max<int64_t>(tiles, 1024);
         e = cudaMalloc(&pool.mem, scan_scratch_bytes(want));
-        if (e != cudaSuccess) {
-            pool.tiles = 0;
-            return cuda_fail(e, "scan scratch");
-        }
-        e = cudaMemset(pool.mem, 0, scan_scratch_bytes(want));
+        if (e != cudaSuccess) return cuda_fail(e, "scan scratch");
+        // (on the scan's stream; the next scan, on whichever, comes after this one)
+        e = cudaMemsetAsync(pool.mem, 0, scan_scratch_bytes(want), st);
         if (e != cudaSuccess) return cuda_fail(e, "scan scratch");
         scan_scratch_carve(pool.mem, want, pool.s);
         pool.tiles = want;

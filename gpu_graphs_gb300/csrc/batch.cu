@@ -230,7 +230,7 @@ extern "C" int gbfs_bfs_batch(gbfs_graphset *s, const int32_t *sources, int32_t 
     {
         std::string err;
         std::lock_guard<std::mutex> lk(g->mu);
-        int rc = bfs_work_alloc(g->work, g->csr.n, err, g->csr.wide, bfs_small(g->csr, graph_params(g)));
+        int rc = bfs_work_alloc(g->work, g->csr.n, err, g->stream, g->csr.wide, bfs_small(g->csr, graph_params(g)));
         if (rc) return fail(rc, err);
     }
     int rc = gbfs_bfs_multiroot(g, roots.data(), count, g->work.level, &st);

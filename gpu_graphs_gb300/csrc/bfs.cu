@@ -1168,7 +1168,7 @@ struct QueueLayout {
 
 }  // namespace
 
-int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide, bool small)
+int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, cudaStream_t st, bool wide, bool small)
 {
     const bool have = w.ctrl && w.n == n && w.wide == wide;
     if (have && (small || w.q0)) return GBFS_OK;
@@ -1210,7 +1210,7 @@ int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide, bool smal
     w.bytes = (int64_t)c.size;
     static_assert(offsetof(BfsCtrl, t_entry) <= PINNED_SLOT, "the results fit a pinned slot");
     w.h_ctrl = (BfsCtrl *)pinned_slot_take();
-    if (!w.h_ctrl || cudaMemset(w.ctrl, 0, sizeof(BfsCtrl)) != cudaSuccess ||
+    if (!w.h_ctrl || cudaMemsetAsync(w.ctrl, 0, sizeof(BfsCtrl), st) != cudaSuccess ||
         cudaEventCreate(&w.ev0) != cudaSuccess || cudaEventCreate(&w.ev1) != cudaSuccess) {
         err = "workspace setup failed";
         bfs_work_free(w);
@@ -1585,7 +1585,8 @@ int bfs_run(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const int *d_r
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) break;
             int status = 0;
-            e = cudaMemcpy(&status, &w.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost);
+            e = cudaMemcpyAsync(&status, &w.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess || status != DEV_OK || w.h_ctrl->rs.done) break;
         }
     }

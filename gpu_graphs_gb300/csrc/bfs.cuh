@@ -127,8 +127,9 @@ void bfs_graph_free(BfsWork &w);
 int bfs_work_reserve_overlap(BfsWork &w, std::string &err);
 
 // small: for searches that run on one cluster (bfs_small), without queues and
-// bitmaps; a later call for others adds them.
-int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, bool wide = false, bool small = false);
+// bitmaps; a later call for others adds them.  The control block is zeroed on st,
+// which the searches have to be on (or after).
+int bfs_work_alloc(BfsWork &w, int32_t n, std::string &err, cudaStream_t st, bool wide = false, bool small = false);
 void bfs_work_free(BfsWork &w);
 
 struct BfsResult {

@@ -2043,7 +2043,8 @@ int csr_build_transpose(DeviceCsr &c, cudaStream_t st, std::string &err)
     CK(cudaStreamSynchronize(st));
     {
         unsigned h_scan_status[3] = {0, 0, 0};
-        CK(cudaMemcpy(h_scan_status, ss.ctl, 12, cudaMemcpyDeviceToHost));
+        CK(cudaMemcpyAsync(h_scan_status, ss.ctl, 12, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
         if (h_scan_status[2] != 0) {
             err = "scan look-back timed out";
             rc = GBFS_ERR_TIMEOUT;

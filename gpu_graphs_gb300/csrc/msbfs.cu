@@ -781,7 +781,7 @@ int ms_prepare(DeviceCsr &g, cudaStream_t st, std::string &err)
     return GBFS_OK;
 }
 
-int ms_work_alloc(MsWork &w, int32_t n, std::string &err)
+int ms_work_alloc(MsWork &w, int32_t n, std::string &err, cudaStream_t st)
 {
     if (w.ctrl && w.n == n) return GBFS_OK;
     ms_work_free(w);
@@ -814,7 +814,7 @@ int ms_work_alloc(MsWork &w, int32_t n, std::string &err)
     w.bytes = (int64_t)c.size;
     static_assert(offsetof(MsCtrl, t_entry) <= PINNED_SLOT, "the results fit a pinned slot");
     w.h_ctrl = (MsCtrl *)pinned_slot_take();
-    if (!w.h_ctrl || cudaMemset(w.ctrl, 0, sizeof(MsCtrl)) != cudaSuccess ||
+    if (!w.h_ctrl || cudaMemsetAsync(w.ctrl, 0, sizeof(MsCtrl), st) != cudaSuccess ||
         cudaEventCreate(&w.ev0) != cudaSuccess || cudaEventCreate(&w.ev1) != cudaSuccess) {
         err = "multi-source workspace setup failed";
         ms_work_free(w);

@@ -58,7 +58,8 @@ int64_t ms_prepare_bytes(const DeviceCsr &g, bool transpose);
 // Device bytes ms_work_alloc takes for n vertices.
 int64_t ms_work_bytes(int64_t n);
 
-int ms_work_alloc(MsWork &w, int32_t n, std::string &err);
+// The control block is zeroed on st, which the searches have to be on (or after).
+int ms_work_alloc(MsWork &w, int32_t n, std::string &err, cudaStream_t st);
 void ms_work_free(MsWork &w);
 
 struct MsResult {

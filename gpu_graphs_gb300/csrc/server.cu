@@ -599,9 +599,10 @@ extern "C" int gbfs_server_add_graph(gbfs_server *s, gbfs_graph *g, int32_t *gra
             sl.cap = 0;
         };
         auto slot_alloc = [](gbfs_server::Slot &sl, int64_t cap, std::string &e) {
-            int r = ms_work_alloc(sl.w, (int32_t)cap, e);
+            int r = ms_work_alloc(sl.w, (int32_t)cap, e, sl.st[0]);
             for (auto &bw : sl.bw)
-                if (!r) r = bfs_work_alloc(bw, (int32_t)cap, e);
+                if (!r) r = bfs_work_alloc(bw, (int32_t)cap, e, sl.st[0]);
+            cudaStreamSynchronize(sl.st[0]);  // (the units' searches are on streams of their own)
             if (!r) sl.cap = cap;
             return r;
         };
