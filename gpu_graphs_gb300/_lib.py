@@ -173,6 +173,7 @@ SIGNATURES = {
     "gbfs_gen_grid_capacity": (I64, [I32, C.c_double]),
     "gbfs_selftest_wait_timeout": (C.c_int, [I32]),
     "gbfs_selftest_mark_timeout": (C.c_int, [C.c_void_p]),
+    "gbfs_selftest_build_route": (C.c_int, []),
     "gbfs_server_create": (C.c_int, [C.POINTER(ServerConfig), C.POINTER(P)]),
     "gbfs_server_destroy": (None, [P]),
     "gbfs_server_add_graph": (C.c_int, [P, P, PI32]),

@@ -34,6 +34,10 @@
 
 namespace gbfs {
 
+static thread_local int tl_route = 0;
+
+int csr_build_route() { return tl_route; }
+
 namespace {
 
 constexpr int W4_MAX = 128;       // rows up to this length: warp sort, 4 values per lane
@@ -1762,6 +1766,7 @@ struct RowSorter {
         if (nch && dedup) {
             e = sort_long(BIN_LONG, row, n, tmp, ucnt, st, bitmaps);
             if (e != cudaSuccess) return e;
+            if (bitmaps) tl_route |= BUILD_LONG_BITS;
         }
         if (nch && !bitmaps) {
             const size_t cb = sizeof(Chunk) * (size_t)nch;
@@ -1789,6 +1794,7 @@ struct RowSorter {
         if (h->rows[BIN_4K] && dedup && BitmapShape(n).ctas <= BMR_CTAS_4K)
             e = sort_long(BIN_4K, row, n, tmp, ucnt, st, done4k);
         if (e != cudaSuccess) return e;
+        if (done4k) tl_route |= BUILD_4K_BITS;
         if (h->rows[BIN_4K] && !done4k)
             k_sort_block<512, RT><<<ctas(h->rows[BIN_4K], 152 * 16), 512, 0, st>>>(row, lists.list[BIN_4K],
                                                                                  rows + BIN_4K, tmp, dedup, ucnt);
@@ -2373,6 +2379,7 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
     const int thr = 256;
     out = DeviceCsr{};
     out.n = n;
+    tl_route = 0;
 
     // Degrees, scratch for both scans (n+1 elements at most), and the counters.
     const int64_t tiles = scan_tiles((int64_t)n + 1);
@@ -2406,6 +2413,7 @@ int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_ds
         if (h->bucket_largest <= BK_MAX_BUCKET && h->bucket_total > 0 && h->bucket_near <= h->bucket_seen / 2 &&
             bk.take((int64_t)h->bucket_total, h->bucket_over))
             CK(cudaMemcpyAsync(total, &bk.plan->total, 8, cudaMemcpyDeviceToDevice, st));
+        if (bk.packed) tl_route |= BUILD_BUCKETS;
     }
     if (m > 0 && !bk.packed) {
         k_count<<<grid_for(m, thr, EDGE_CTAS), thr, 0, st>>>(d_src, d_dst, m, n, flags, deg, total, status);

@@ -99,6 +99,14 @@ constexpr int HEAVY_DEGREE = 64;
 int csr_build_from_edges(int32_t n, int64_t m, const int *d_src, const int *d_dst,
                          unsigned flags, cudaStream_t st, DeviceCsr &out, std::string &err);
 
+// The ways this thread's last csr_build_from_edges took (for tests).
+enum BuildRoute : int {
+    BUILD_BUCKETS = 1,    // entries by buckets of rows
+    BUILD_LONG_BITS = 2,  // rows of more than 4,096 entries through bitmaps
+    BUILD_4K_BITS = 4,    // rows of 2,049 to 4,096 entries too
+};
+int csr_build_route();
+
 // Take an existing device CSR (row n+1, col m; ownership moves to `out`),
 // validate it and compute zmask / max_degree / nonisolated.
 int csr_adopt(int32_t n, int64_t m, int *d_row, int *d_col, cudaStream_t st, DeviceCsr &out,

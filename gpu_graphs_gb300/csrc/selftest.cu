@@ -6,7 +6,8 @@
 // return, leaving the CUDA context usable.  Nothing faults, traps or hangs.
 //
 // And a mark on a graph's control block, as left by a search in which some
-// CTA's wait ran out: the next search has to report and clear it.
+// CTA's wait ran out: the next search has to report and clear it.  And which ways
+// the last build from edges took.
 #include "graph.cuh"
 
 using namespace gbfs;
@@ -46,6 +47,8 @@ extern "C" int gbfs_selftest_wait_timeout(int32_t timeout_ms)
     if (h.status == DEV_TIMEOUT && h.passed == 0) return fail(GBFS_ERR_TIMEOUT, "bounded wait ran out as expected");
     return fail(GBFS_ERR_CUDA, "bounded wait did not report a timeout");
 }
+
+extern "C" int gbfs_selftest_build_route(void) { return csr_build_route(); }
 
 extern "C" int gbfs_selftest_mark_timeout(gbfs_graph *g)
 {

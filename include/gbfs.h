@@ -344,6 +344,13 @@ int gbfs_selftest_wait_timeout(int32_t timeout_ms);
  * GBFS_ERR_TIMEOUT, and the one after that to succeed.
  */
 int gbfs_selftest_mark_timeout(gbfs_graph *g);
+/*
+ * How this thread's last gbfs_graph_from_edges sorted its entries: bit 0 by
+ * buckets of rows, bit 1 rows of more than 4,096 entries through bitmaps of
+ * the vertices, bit 2 rows of 2,049 to 4,096 too; 0: straight to the rows,
+ * sorted there.
+ */
+int gbfs_selftest_build_route(void);
 
 /* ---- file format and workload generators ------------------------------ */
 /*

@@ -57,5 +57,5 @@ def test_bottom_up_probes_stay_in_range():
 
 def test_symmetry_check_halves_without_overflow():
     text = (CSRC / "csr_build.cu").read_text()
-    body = text[text.index("k_check_sym(const RT"):text.index("k_check_sorted(const RT")]
+    body = text[text.index("bool row_has(const RT"):text.index("k_check_sorted(const RT")]
     assert "idx_mid(lo, hi)" in body and not re.search(PLAIN[0], body)
