@@ -1582,12 +1582,10 @@ int bfs_run(const DeviceCsr &g, const gbfs_params &p, BfsWork &w, const int *d_r
             e = bfs_enqueue(g, p, w, d_roots, k, single_root, d_level, &w.h_ctrl->out, st, symmetric, resume, 1);
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(&w.h_ctrl->rs, &w.ctrl->rs, sizeof(BfsResume), cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(&w.h_ctrl->status, &w.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess) break;
-            int status = 0;
-            e = cudaMemcpyAsync(&status, &w.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess || status != DEV_OK || w.h_ctrl->rs.done) break;
+            if (e != cudaSuccess || w.h_ctrl->status != DEV_OK || w.h_ctrl->rs.done) break;
         }
     }
     if (e == cudaSuccess) e = cudaEventRecord(w.ev1, st);
