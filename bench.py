@@ -220,7 +220,7 @@ def log(msg: str) -> None:
     print(f"[bench] {msg}", file=sys.stderr, flush=True)
 
 
-KERNEL_SOURCES = ("bfs.cu", "bfs.cuh", "bfs_args.cuh", "common.cuh", "blockq.cuh")
+KERNEL_SOURCES = ("bfs.cu", "bfs.cuh", "bfs_args.cuh", "common.cuh", "blockq.cuh", "index.h")
 
 
 def kernel_source_hash() -> str:

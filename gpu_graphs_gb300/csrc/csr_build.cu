@@ -201,12 +201,12 @@ __global__ void k_scatter(const int *__restrict__ src, const int *__restrict__ d
 // in shared memory; then one CTA per bucket counts its rows in shared memory,
 // writes their offsets and places the columns, all within a range that L2 holds.
 // For inputs of BK_MIN_M entries (below, the direct scatter's range fits L2: whole
-// builds, buckets and direct, RMAT of 8 M entries 1.26 and 1.29 ms, 25 M 2.04 and
-// 2.20, 34 M 2.34 and 2.63, 134 M 7.1 and 8.9; uniform random of 12 M entries 1.19
-// and 1.16, 67 M 2.8 and 4.6) on up to BK_MAX_N vertices (a word holds 10 + 22
-// bits), unless one bucket holds more than BK_MAX_BUCKET entries, which would be
-// one CTA's tail, or edges beside each other mostly have both ends in the same
-// buckets (a grid's in order, 17 M entries: 1.44 and 1.20 ms).
+// builds, buckets and direct, RMAT of 8 M entries 0.99 and 0.87 ms, 25 M 1.50 and
+// 1.59, 34 M 1.73 and 1.88, 67 M 2.88 and 3.29, 134 M 4.8 and 6.4; uniform random
+// of 12 M entries 0.97 and 0.86, 67 M 2.5 and 3.7) on up to BK_MAX_N vertices (a
+// word holds 10 + 22 bits), unless one bucket holds more than BK_MAX_BUCKET
+// entries, which would be one CTA's tail, or edges beside each other mostly have
+// both ends in the same buckets (a grid's in order, 16 M entries: 1.21 and 0.88 ms).
 constexpr int BK_LOG = 10;
 constexpr int BK_MAX_N = 1 << 22;
 constexpr int BK_BUCKETS = BK_MAX_N >> BK_LOG;

@@ -22,9 +22,9 @@
 // symmetric graphs with rows in other than ascending order, levels whose
 // vertices have far more edges than the level before are pushed to as well.
 //
-// The longest rows bounded this: RMAT-20 with its search took 1,033 us with a
+// The longest rows bounded this: RMAT-20 with its search took 1,060 us with a
 // warp to each row, walked to its end (900 of them in the heavy rows' kernel),
-// and takes 161 us now; the level gathers hit L2.
+// and takes 145 to 155 us now; the level gathers hit L2.
 #include <algorithm>
 #include <climits>
 

@@ -146,7 +146,11 @@ typedef struct gbfs_params {
                                    level replayed by a CUDA graph with a
                                    device-side while loop (no host round
                                    trip between levels)                     */
-    int32_t timeout_ms;         /* bound on every device-side wait          */
+    int32_t timeout_ms;         /* bound on every grid-wide wait of a search
+                                   (one-cluster searches of small graphs, and
+                                   the build's long rows, meet in hardware
+                                   cluster barriers, which have none: every
+                                   CTA of the cluster reaches them)          */
 } gbfs_params;
 
 /* Built-in defaults (before any autotuning). */
