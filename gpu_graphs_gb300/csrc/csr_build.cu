@@ -1193,7 +1193,8 @@ __global__ void k_compact(const RT *__restrict__ row, const RT *__restrict__ row
     }
 }
 
-template <typename RT>
+// SMALL: with the costs of the parts that the one-cluster search deals in.
+template <bool SMALL, typename RT>
 __global__ void k_finalize(const RT *__restrict__ row, int n, unsigned *zmask, int *maxdeg,
                            unsigned long long *nonisolated, unsigned *nover4, unsigned long long *part, int part_log)
 {
@@ -1211,10 +1212,10 @@ __global__ void k_finalize(const RT *__restrict__ row, int n, unsigned *zmask, i
         unsigned z = __ballot_sync(FULL, d == 0);  // out-of-range bits count as zero-degree
         if (lane_id() == 0) zmask[v >> 5] = z;
         mine += (d > 0 ? 1ull : 0ull) + (d > 4 ? 1ull << 32 : 0ull);
-        cost += (unsigned long long)small_row_cost(d);
+        if (SMALL) cost += (unsigned long long)small_row_cost(d);
         mx = max(mx, d);
     }
-    if (part_log > 0) {  // (the grid covers so small a graph in one go: a CTA's vertices are of one part)
+    if (SMALL) {  // (the grid covers so small a graph in one go: a CTA's vertices are of one part)
         cost = block_sum(cost, s_red);
         if (threadIdx.x == 0 && cost) atomicAdd(part + ((blockIdx.x * blockDim.x) >> part_log), cost);
     }
@@ -1621,9 +1622,12 @@ int finalize_t(DeviceCsr &out, const RT *row, cudaStream_t st, std::string &err)
     CK(cudaMalloc(&d_res, sizeof(Res)));
     CK(cudaMemsetAsync(d_res, 0, sizeof(Res), st));
     static_assert(SMALL_MAX_N <= 256 * 152 * 16, "one pass of k_finalize's grid covers a small graph");
-    k_finalize<<<grid_for((int64_t)W * 32, 256), 256, 0, st>>>(row, out.n, out.zmask, &d_res->maxdeg,
-                                                                &d_res->nonisolated, &d_res->nover4, d_res->part,
-                                                                out.n <= SMALL_MAX_N ? small_part_log(out.n) : 0);
+    if (out.n <= SMALL_MAX_N)
+        k_finalize<true><<<grid_for((int64_t)W * 32, 256), 256, 0, st>>>(
+            row, out.n, out.zmask, &d_res->maxdeg, &d_res->nonisolated, &d_res->nover4, d_res->part, small_part_log(out.n));
+    else
+        k_finalize<false><<<grid_for((int64_t)W * 32, 256), 256, 0, st>>>(
+            row, out.n, out.zmask, &d_res->maxdeg, &d_res->nonisolated, &d_res->nover4, d_res->part, 0);
     CK(cudaGetLastError());
     k_heavy_list<<<grid_for(out.n, 1024, 152 * 4), 1024, 0, st>>>(row, out.n, out.heavy, &d_res->nheavy);
     CK(cudaGetLastError());
