@@ -58,7 +58,7 @@ LevelRoute output_route(const void *p, int device)
         cudaGetLastError();
         return LevelRoute::HOST;
     }
-    return level_route((int)at.type, at.device, device);
+    return level_route(p, (int)at.type, at.device, device);
 }
 
 int make_set(gbfs_graph *g, int32_t count, const std::vector<int64_t> &offsets, gbfs_graphset **out)
