@@ -243,11 +243,22 @@ extern "C" int gbfs_bfs_batch(gbfs_graphset *s, const int32_t *sources, int32_t 
         any_host = any_host || routes[i] == LevelRoute::HOST;
         any_kernel = any_kernel || routes[i] == LevelRoute::KERNEL;
     }
-    if (any_kernel && !s->d_slices &&
+    bool copies = false;
+    if (any_kernel) {
+        try {
+            std::vector<std::pair<uintptr_t, uintptr_t>> scratch;
+            copies = outputs_overlap(levels_out, s->sizes.data(), routes.data(), (size_t)count, scratch);
+        } catch (const std::bad_alloc &) {
+            copies = true;
+        }
+    }
+    if (any_kernel && !copies && !s->d_slices &&
         cudaMalloc(&s->d_slices, sizeof(gbfs_graphset::Slice) * (size_t)count) != cudaSuccess) {
-        // no room for the table: a copy per member
-        cudaGetLastError();
+        cudaGetLastError();  // no room for the table
         s->d_slices = nullptr;
+        copies = true;
+    }
+    if (copies) {  // one per member
         any_kernel = false;
         for (auto &r : routes)
             if (r == LevelRoute::KERNEL) r = LevelRoute::COPY;
