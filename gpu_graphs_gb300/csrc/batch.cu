@@ -31,7 +31,7 @@ constexpr int SLICE_BLOCK = 256, SLICE_PER = 16;  // threads, vertices per threa
 
 // The union's levels to the members' own arrays (dst null: none) in one launch:
 // 512 members of 5.7 M vertices together took 2.5 ms a call with a copy per
-// member, 2 of them the host's, and take 0.36 ms so.  A CTA takes SLICE_BLOCK *
+// member, 2 of them the host's, and take 0.37 ms so.  A CTA takes SLICE_BLOCK *
 // SLICE_PER consecutive vertices and finds the member of its first by bisection.
 __global__ void k_slices_out(const int *__restrict__ level, long long n, const gbfs_graphset::Slice *__restrict__ slices,
                              int count)

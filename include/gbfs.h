@@ -288,7 +288,8 @@ int gbfs_graphset_vertex_offsets(const gbfs_graphset *s, int64_t *offsets);
 
 /*
  * One BFS per graph (sources[i] local to graph i), all in one persistent
- * launch.  levels_out[i]: n[i] int32 (host or device).
+ * launch.  levels_out[i]: n[i] int32 (host or device); where two overlap, the
+ * later member's levels stand.
  */
 int gbfs_bfs_batch(gbfs_graphset *s, const int32_t *sources,
                    int32_t *const *levels_out, gbfs_stats *stats);
